@@ -188,17 +188,14 @@ int shape_engine_stage_times(shape_engine *e, int form, double *ms, int max);
 
 /* Facet-bin capacity per 16x16 POS tile. 0 (default) lets finalize size it
  * from a dry-run binning of the model (next power of two above 1.25x the
- * fullest tile); tiles whose bin overflows are rasterized by an ordered scan
- * of all facets, which is exact but slow. Takes effect at the next finalize. */
+ * fullest tile); tiles whose bin overflows are rasterized by scans of all
+ * facets, which are exact but slow. Takes effect at the next finalize. */
 int shape_engine_set_bin_capacity(shape_engine *e, int cap);
-/* Batched FP32 form, radar views: 1 (default) redoes every pixel whose
- * coverage or depth-order decision lies within FP32 error by the FP64
- * form's rules, so facet maps are the FP64 form's (kept POS maps also get
- * the FP64 form's depths); 0 takes the FP32 decisions as they are (a pixel
- * within FP32 error of a facet edge or of a depth tie may take another
- * facet than the FP64 form: a faster raster, and a small frame's
- * chi-square may move by ~1e-4 when that happens). Lightcurve views are
- * always exact. Takes effect at the next evaluation. */
+/* Batched FP32 form, radar views. Coverage and depth are evaluated in FP64 in
+ * every form, so the FP32 form's facet and depth maps are the FP64 form's with
+ * either value; the switch is kept for callers that set it (it used to admit
+ * decisions in FP32, which were faster then). Takes effect at the next
+ * evaluation. */
 int shape_engine_set_fp32_exact(shape_engine *e, int exact);
 /* vary_params (src/shape/vary_params.c:84-327): the four means the
  * reference computes for its joint adjustments of the 0th delay-correction
@@ -223,17 +220,15 @@ int shape_engine_vary_params(shape_engine *e, const shape_vary_options *opt, dou
 
 /* Raster kernel of the batched forms./* Raster kernel of the batched forms. mode -1 (default): the first batched
  * evaluation of each form times four candidates on this engine's datasets
- * (the tile-per-CTA kernel and the warp-independent kernel, each with one
- * CTA per non-empty tile or a persistent grid of resident CTAs on every
- * SM striding over the tiles) and keeps the fastest; the choice is
- * remembered for engines of the same size class in the process. mode 0 /
- * 1: that kernel, one CTA per tile, no timing. Every candidate computes the
- * same images. Lightcurve views always use the tile-per-CTA kernel (in the
- * FP32 form their own launch; in the FP64 form an engine with lightcurve
- * points tunes the grid only). */
+ * (256 or 128 threads per tile, each with one CTA per non-empty tile or a
+ * persistent grid of resident CTAs on every SM striding over the tiles)
+ * and keeps the fastest; the choice is remembered for engines of the same
+ * size class in the process. mode 0 / 1: 256 / 128 threads, one CTA per
+ * tile, no timing. Every candidate computes the same images. Radar views
+ * and lightcurve / sky views are two launches of the same choice. */
 int shape_engine_set_raster_tuning(shape_engine *e, int mode);
-/* The raster choice of a form: *variant (0 tile-per-CTA, 1 warp-
- * independent), *persistent, and ms[4] (may be NULL) the measured raster
+/* The raster choice of a form: *variant (0: 256 threads per tile, 1: 128),
+ * *persistent, and ms[4] (may be NULL) the measured raster
  * times of the candidates variant*2 + persistent (0 where not measured).
  * Returns 1 once the form is tuned, 0 before its first evaluation. */
 int shape_engine_get_raster_tuning(shape_engine *e, int form, int *variant, int *persistent, double *ms);

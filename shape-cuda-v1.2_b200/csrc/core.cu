@@ -110,7 +110,8 @@ __global__ void k_realize_vf(int nv, int nf, const double *__restrict__ a, const
 // vertex normal = normalized sum of attached facet normals, in af order
 // (src/shape/realize_mod.c:550-563)
 __global__ void k_realize_vnormals(int nv, const int *__restrict__ af_ptr, const int *__restrict__ af_idx,
-                                   const double4 *__restrict__ fn, double4 *__restrict__ vn)
+                                   const double4 *__restrict__ fn, double4 *__restrict__ vn,
+                                   float4 *__restrict__ vnf)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nv) return;
@@ -128,6 +129,7 @@ __global__ void k_realize_vnormals(int nv, const int *__restrict__ af_ptr, const
         n0 /= norm; n1 /= norm; n2 /= norm;
     }
     vn[i] = make_double4(n0, n1, n2, 0.0);
+    if (vnf) vnf[i] = make_float4((float)n0, (float)n1, (float)n2, 0.0f);
 }
 
 // ------------------------------------------------------------- transforms
@@ -1249,7 +1251,8 @@ void launch_realize_vf(const ModelDev &m, cudaStream_t s)
 void launch_realize_vn(const ModelDev &m, cudaStream_t s)
 {
     const int B = 256;
-    k_realize_vnormals<<<(m.nv + B - 1) / B, B, 0, s>>>(m.nv, m.af_ptr, m.af_idx, m.fn, m.vn);
+    k_realize_vnormals<<<(m.nv + B - 1) / B, B, 0, s>>>(m.nv, m.af_ptr, m.af_idx, m.fn, m.vn,
+                                                          m.vnf);
 }
 
 void launch_realize(const ModelDev &m, cudaStream_t s)

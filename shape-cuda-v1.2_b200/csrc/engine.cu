@@ -116,6 +116,7 @@ int EngineImpl::finalize()
         for (int t = 0; t < g.tiles_x * g.tiles_x; t++) work.push_back(make_int2((int)geoms.size(), t));
         tile_base += g.tiles_x * g.tiles_x;
         pos_base += (long long)g.side * g.side;
+        if (g.kind == VIEW_RADAR) radar_lean_consts(g, laws[g.law]);
         view_float_consts(g);
         geoms.push_back(g);
     };
@@ -326,7 +327,7 @@ int EngineImpl::finalize()
     d_scale = d_r + nv;
     AL(d_fv, (size_t)3 * nf); AL(d_afp, (size_t)nv + 1); AL(d_afi, af_idx.size());
     AL(md.vx, (size_t)nv); AL(md.vn, (size_t)nv); AL(md.fn, (size_t)nf); AL(md.area, (size_t)nf);
-    AL(md.fvi, (size_t)nf);
+    AL(md.fvi, (size_t)nf); AL(md.vnf, (size_t)nv);
     AL(d_geoms, (size_t)nviews); AL(d_states, (size_t)nviews); AL(d_laws, laws.size());
     AL(d_work, work.size());
     AL(d_vt64, (size_t)nviews * nv);
@@ -1108,6 +1109,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     ra.vt = d_vt64;         // both forms stage from the FP64 view-frame vertices
     ra.fvi = md.fvi;
     ra.vn = md.vn;
+    ra.vnf = md.vnf;
     ra.fn = md.fn;
     ra.nf = nf;
     ra.bin_count = d_bin_count;
@@ -1153,6 +1155,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
             RasterArgs rv = ra;
             rv.work = d_work + view_work0[v];
             rv.nwork = view_nwork[v];
+            rv.maps = geoms[v].kind != VIEW_RADAR;
             launch_raster_f64(rv, s);
             const FrameGeom &g = geoms[v];
             if (g.kind == VIEW_RADAR && fh[g.frame_index].view == v) {
@@ -1195,29 +1198,26 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         // one CTA per tile that was non-empty when the bins were tuned (they
         // lead each part of the sorted list); the grid-stride loop visits the
         // tiles after them, empty then, so those cost no CTA launches of
-        // their own. The FP32 form rasters lightcurve views with its exact
-        // variant, in a second launch.
+        // their own. Radar tiles and lightcurve / sky tiles are two launches:
+        // the first shades and synthesizes in the form's arithmetic, the
+        // second shades and writes maps in FP64 in both forms.
         ra.work = d_work_sorted;
         ra.pdl = pdl ? 1 : 0;
         ra.variant = raster_variant[form];
+        RasterArgs rr = ra, rl = ra;
+        rr.nwork = work_radar;
+        rr.grid = raster_grid(form, nonempty_radar, rr, f32);
+        rl.work = d_work_sorted + work_radar;
+        rl.nwork = (int)work.size() - work_radar;
+        rl.maps = 1;
+        rl.grid = raster_grid(form, nonempty_lc, rl, false);
         if (f32) {
-            RasterArgs rr = ra, rl = ra;
-            rr.nwork = work_radar;
-            rr.exact = fp32_exact;
-            rr.grid = raster_grid(form, nonempty_radar, rr, true);
-            rl.work = d_work_sorted + work_radar;
-            rl.nwork = (int)work.size() - work_radar;
-            rl.exact = 1;
-            rl.variant = 0;       // lightcurve views: the tile-per-CTA kernel
-            rl.lc_views = 1;
-            rl.grid = raster_grid(form, nonempty_lc, rl, true);
             launch_raster_f32(rr, s);
-            launch_raster_f32(rl, s);
+            launch_raster_f64(rl, s);
             launch_dop_fit_f32(d_dop_frames, (int)dop_frames.size(), d_fh, d_geoms, d_fit64, d_fit32, s);
         } else {
-            ra.nwork = (int)work.size();
-            ra.grid = raster_grid(form, tuned_nonempty, ra, false);
-            launch_raster_f64(ra, s);
+            launch_raster_f64(rr, s);
+            launch_raster_f64(rl, s);
         }
         mark(4);
         if (int rc_ = launched("raster")) return rc_;
@@ -1307,8 +1307,8 @@ int EngineImpl::kernels_per_eval(int form) const
                               geoms[v].kind == VIEW_LC_SUN ? 1 : 0);
     } else {
         n += 3;                          // transform, bin, raster
-        if (form == SHAPE_FORM_BATCHED_FP32 && work_radar > 0 && work_radar < (int)work.size())
-            n += 1;                      // FP32: radar and lightcurve views in two launches
+        if (work_radar > 0 && work_radar < (int)work.size())
+            n += 1;                      // radar and lightcurve / sky views in two launches
         if (form == SHAPE_FORM_BATCHED_FP32 && !dop_frames.empty())
             n += 1;                      // FP32: Doppler spectra rounded from their FP64 sums
         n += (chi2_items.empty() || fused_chi2) ? 0 : 1;   // fused: counted with the summary
@@ -1362,7 +1362,7 @@ int EngineImpl::launch(int form)
                     int rc = autotune(form);
                     if (rc) return rc;
                 } else {
-                    raster_variant[form] = (form == SHAPE_FORM_BATCHED_FP64 && !lcpts.empty()) ? 0 : tune_mode;
+                    raster_variant[form] = tune_mode;
                     raster_persistent[form] = 0;
                     tuned[form] = 1;
                 }
@@ -1515,11 +1515,7 @@ int EngineImpl::autotune(int form)
     for (auto &x : ev) CK(cudaEventCreate(&x));
     int best = 0, rc = SHAPE_OK;
     double best_ms = 1e300;
-    // the warp-independent kernel is a candidate for radar views only: a
-    // batched FP64 launch that also holds lightcurve views keeps the
-    // tile-per-CTA kernel
-    const int ncand = (form == SHAPE_FORM_BATCHED_FP64 && !lcpts.empty()) ? 2 : 4;
-    for (int c = 0; c < ncand && rc == SHAPE_OK; c++) {
+    for (int c = 0; c < 4 && rc == SHAPE_OK; c++) {
         raster_variant[form] = c >> 1;
         raster_persistent[form] = c & 1;
         double m = 1e300;

@@ -310,7 +310,7 @@ struct EngineImpl {
     // (nonempty_lc non-empty at tuning)
     int work_radar = 0, nonempty_radar = 0, nonempty_lc = 0;
     int fixed_cap = 0;            // > 0: bin capacity set by the caller, no autotuning
-    int fp32_exact = 1;           // batched FP32: radar views by the exact raster variant too
+    int fp32_exact = 1;           // shape_engine_set_fp32_exact (part of the tuning key only)
     // Raster kernel per form (RasterArgs::variant) and grid (0: one CTA per
     // tile that was non-empty at bin tuning; 1: persistent, resident CTAs x
     // SMs striding over the tiles). tune_mode -1: the first batched

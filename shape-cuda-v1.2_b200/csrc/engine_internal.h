@@ -61,6 +61,13 @@ struct FrameGeom {
     // response is exactly 1; pixels whose footprint leaves the spectrum go to
     // an overflow spectrum of DOP_MAXOVERFLOW bins (src/shape/pos2doppler.c)
     int dop1d;           // 1: Doppler spectrum
+    // synthesis shortcuts (radar_lean_consts): lean: the delay response is
+    // tri2 of the offset over lean_sos and there is one sinc^2 point per
+    // pixel; linlaw: the law is amp cos(e) / kmpp^2 (amp, famp with the pixel's
+    // area); half_w = sinc2width / 2; fscale = wscale
+    int lean, lean_sos, linlaw;
+    double half_w, amp;
+    float famp, fscale;
     int idop0;           // overflow bin of spectrum bin 0: MAXOVERFLOW/2 - floor(dopshift + 0.5)
     long long ovf_base;  // first element of this frame's overflow spectrum
     // the synthesis constants rounded to float on the host for the FP32

@@ -49,6 +49,7 @@ struct ModelDev {
     const int *fv;                     // [nf*3]
     const int *af_ptr, *af_idx;
     double4 *vx, *vn, *fn;             // realized
+    float4 *vnf;                       // vertex normals rounded to float (FP32 form; may be null)
     double *area;
     int4 *fvi;                         // corner indices, padded
 };
@@ -58,11 +59,11 @@ struct RasterArgs {
     const int2 *work;          // (view, tile) items
     int nwork;                 // items
     int grid;                  // CTAs (0: one per item); fewer CTAs stride over the rest
-    int exact;                 // FP32 form: the exact variant (lightcurve views)
     int pdl;                   // programmatic dependent launch (launch_k)
     const void *vt;            // double4 view-frame vertices (both forms)
     const int4 *fvi;
     const double4 *vn;
+    const float4 *vnf;
     const double4 *fn;
     int nf;
     const int *bin_count;
@@ -79,21 +80,16 @@ struct RasterArgs {
     int mark_seen;
     int keep_pos;
     double *ovf;               // Doppler overflow spectra (DOP_MAXOVERFLOW per Doppler frame)
-    size_t smem_bytes;         // dynamic shared memory of the raster CTA (set by the launcher)
     // FP64 raster of a single view into images that already hold earlier
     // calls' results (posvis accumulating over model components): each pixel
     // starts from its z / facet / cos(e) / cos(i), and won[p] is set to 1
     // where this launch assigned pixel p. 0 for the engine's evaluations.
     int accumulate;
     unsigned char *won;
-    // 0: the tile-per-CTA kernel (k_raster: the CTA's warps share one
-    // sorted facet list and meet at block barriers); 1: the warp-independent
-    // kernel (k_raster_w: each warp sorts and replays its own block's list)
-    int variant;
-    // FP32 form: the launch holds only lightcurve views, whose cosines the
-    // exact variant recomputes in FP64 (a separate instantiation, so radar
-    // launches carry none of it)
-    int lc_views;
+    int variant;               // 0: 256 threads per tile, 1: 128
+    // 1: lightcurve, sky and single POS views (shading and maps, FP64 in
+    // both forms); 0: radar views (shading and delay-Doppler synthesis)
+    int maps;
 };
 
 // core.cu (FP64, no FMA contraction)

@@ -262,6 +262,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     ra.pos_f = static_cast<int *>(c->f.p);
     ra.keep_pos = 1;
     ra.accumulate = 1;
+    ra.maps = 1;
     ra.won = static_cast<unsigned char *>(c->won.p);
     launch_raster_f64(ra, s);
     PV_CK(cudaGetLastError());
@@ -322,7 +323,7 @@ __global__ void k_pos2deldop(P2dArgs a)
     const FrameGeom &g = *a.g;
     const DDC<double> kc = load_ddc<double>(g);
     PixPos pp;
-    PixDD<double> d = pixel_dd_setup<double>(g, kc, xi, yj, z, pp);
+    PixDD<double> d = pixel_dd_setup(g, xi, yj, z, pp);
     if (a.xoff != 0.0 || a.yoff != 0.0) {
         // Doppler position with the binary-orbit offsets (x - xoff, y - yoff)
         d.dopPOS = kc.ax * ((double)xi - a.xoff) + kc.ay * ((double)yj - a.yoff) + kc.dopshift;
@@ -344,7 +345,7 @@ __global__ void k_pos2deldop(P2dArgs a)
     atomicMin(&S.doplim[0], dkey(pp.dop));
     atomicMax(&S.doplim[1], dkey(pp.dop));
     S.any_lit = 1;
-    if (d.ok) pixel_dd_scatter<double>(a.ra, g, kc, cose, d, a.fit, 1, 1, g.ndop);
+    if (d.ok) pixel_dd_scatter<double, double>(a.ra, g, cose, d, a.fit);
 }
 
 static int pos2deldop_impl(int device, const shape_pos_view *view, const shape_pos_images *img,

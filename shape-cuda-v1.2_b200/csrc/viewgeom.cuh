@@ -95,6 +95,19 @@ __host__ __device__ inline void lc_view_geom(FrameGeom &go, FrameGeom &gs, LcPoi
     mul_bt(pd.so, P.se, P.oe);
 }
 
+// The synthesis shortcuts of a radar view (law: its scattering law); the
+// view's kmpp, code and sampling constants and wscale must be set.
+__host__ __device__ inline void radar_lean_consts(FrameGeom &g, const RadarLawDev &law)
+{
+    g.lean = g.nsinc2 == 1 && (g.codemethod == SHAPE_CODE_LONG_ORIG || g.spb == 1);
+    g.lean_sos = g.codemethod == SHAPE_CODE_LONG_ORIG ? g.spb_over_stride : 1;
+    g.linlaw = law.type == SHAPE_RADLAW_COSINE_DIFF && law.diff_linear;
+    g.amp = law.diff_R * (law.diff_C + 1) * g.kmpp * g.kmpp;
+    g.famp = (float)g.amp;
+    g.half_w = g.sinc2width / 2.0;
+    g.fscale = (float)g.wscale;
+}
+
 // The float copies of a view's constants that the FP32 raster reads.
 __host__ __device__ inline void view_float_consts(FrameGeom &g)
 {

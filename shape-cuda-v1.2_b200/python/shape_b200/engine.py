@@ -334,9 +334,8 @@ class Engine:
         _chk(self.L.shape_engine_set_bin_capacity(self.h, int(cap)))
 
     def set_fp32_exact(self, exact=True):
-        """Batched FP32 form, radar views: True (the default) redoes pixels
-        whose decisions lie within FP32 error by the FP64 rules; False keeps
-        the FP32 decisions (faster raster)."""
+        """Kept for callers that set it: coverage and depth are FP64 in every
+        form, so both values give the FP64 form's facet and depth maps."""
         _chk(self.L.shape_engine_set_fp32_exact(self.h, 1 if exact else 0))
 
     def set_spin_device(self, on=True):
@@ -368,8 +367,8 @@ class Engine:
 
     def set_raster_tuning(self, mode=-1):
         """-1: time the raster candidates at each batched form's first
-        evaluation and keep the fastest; 0 / 1: the tile-per-CTA / warp-
-        independent kernel, one CTA per tile."""
+        evaluation and keep the fastest; 0 / 1: 256 / 128 threads per tile,
+        one CTA per tile."""
         _chk(self.L.shape_engine_set_raster_tuning(self.h, int(mode)))
 
     def raster_tuning(self, form):
