@@ -34,16 +34,22 @@ __device__ inline int clamp_hi(double v) { return (v > (double)INT_MAX) ? INT_MA
 // its rotation offsets are not all zero) and translation (when its offsets
 // are not all zero), as realize_mod does (src/shape/realize_mod.c:474-512).
 // cxf holds per component m (9, row-major), off (3) and the two flags.
-__device__ inline double4 realize_vertex(int i, const double *__restrict__ a, const double *__restrict__ u,
-                                         const double *__restrict__ r, const double *__restrict__ scale,
+// P: where the deviations and scale factors are read (r(i), scale(k)).
+struct ArrayParams {
+    const double *__restrict__ rv;
+    const double *__restrict__ sv;
+    __device__ double r(int i) const { return rv[i]; }
+    __device__ double scale(int k) const { return sv[k]; }
+};
+template <typename P>
+__device__ inline double4 realize_vertex(int i, const double *__restrict__ a, const double *__restrict__ u, const P &par,
                                          const int *__restrict__ vcomp, const double *__restrict__ cxf)
 {
     const int c = vcomp ? vcomp[i] : 0;
-    const double *sc = scale + 3 * c;
-    double ri = r[i];
-    double x0 = sc[0] * (u[3 * i + 0] * ri + a[3 * i + 0]);
-    double x1 = sc[1] * (u[3 * i + 1] * ri + a[3 * i + 1]);
-    double x2 = sc[2] * (u[3 * i + 2] * ri + a[3 * i + 2]);
+    double ri = par.r(i);
+    double x0 = par.scale(3 * c + 0) * (u[3 * i + 0] * ri + a[3 * i + 0]);
+    double x1 = par.scale(3 * c + 1) * (u[3 * i + 1] * ri + a[3 * i + 1]);
+    double x2 = par.scale(3 * c + 2) * (u[3 * i + 2] * ri + a[3 * i + 2]);
     if (cxf) {
         const double *T = cxf + CXF_N * c;
         if (T[12] != 0.0) {
@@ -89,32 +95,37 @@ __device__ inline void realize_facet(int f, const int *__restrict__ fv, double4 
 // its three corners, which they compute themselves with the vertex formula
 // (same operations, so the same bits as the vertex threads), and threads
 // [nf, nf + nv) realize the vertices for the later stages.
+template <typename P>
+__device__ inline void realize_vf(int k, int nv, int nf, const double *__restrict__ a, const double *__restrict__ u,
+                                  const P &par, const int *__restrict__ vcomp, const double *__restrict__ cxf,
+                                  const int *__restrict__ fv, double4 *__restrict__ vx, double4 *__restrict__ fn,
+                                  double *__restrict__ area, int4 *__restrict__ fvi)
+{
+    if (k < nf) {
+        int i0 = fv[3 * k + 0], i1 = fv[3 * k + 1], i2 = fv[3 * k + 2];
+        fvi[k] = make_int4(i0, i1, i2, 0);
+        realize_facet(k, fv, realize_vertex(i0, a, u, par, vcomp, cxf), realize_vertex(i1, a, u, par, vcomp, cxf),
+                      realize_vertex(i2, a, u, par, vcomp, cxf), fn, area);
+    } else if (k < nf + nv) {
+        vx[k - nf] = realize_vertex(k - nf, a, u, par, vcomp, cxf);
+    }
+}
 __global__ void k_realize_vf(int nv, int nf, const double *__restrict__ a, const double *__restrict__ u,
                              const double *__restrict__ r, const double *__restrict__ scale,
                              const int *__restrict__ vcomp, const double *__restrict__ cxf,
                              const int *__restrict__ fv, double4 *__restrict__ vx, double4 *__restrict__ fn,
                              double *__restrict__ area, int4 *__restrict__ fvi)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nf) {
-        int i0 = fv[3 * k + 0], i1 = fv[3 * k + 1], i2 = fv[3 * k + 2];
-        fvi[k] = make_int4(i0, i1, i2, 0);
-        realize_facet(k, fv, realize_vertex(i0, a, u, r, scale, vcomp, cxf),
-                      realize_vertex(i1, a, u, r, scale, vcomp, cxf), realize_vertex(i2, a, u, r, scale, vcomp, cxf),
-                      fn, area);
-    } else if (k < nf + nv) {
-        vx[k - nf] = realize_vertex(k - nf, a, u, r, scale, vcomp, cxf);
-    }
+    realize_vf(blockIdx.x * blockDim.x + threadIdx.x, nv, nf, a, u, ArrayParams{r, scale}, vcomp, cxf, fv, vx, fn, area,
+               fvi);
 }
 
 // vertex normal = normalized sum of attached facet normals, in af order
 // (src/shape/realize_mod.c:550-563)
-__global__ void k_realize_vnormals(int nv, const int *__restrict__ af_ptr, const int *__restrict__ af_idx,
-                                   const double4 *__restrict__ fn, double4 *__restrict__ vn,
-                                   float4 *__restrict__ vnf)
+__device__ inline void realize_vnormal(int i, const int *__restrict__ af_ptr, const int *__restrict__ af_idx,
+                                       const double4 *__restrict__ fn, double4 *__restrict__ vn,
+                                       float4 *__restrict__ vnf)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
     double n0 = 0.0, n1 = 0.0, n2 = 0.0;
     for (int j = af_ptr[i]; j < af_ptr[i + 1]; j++) {
         double4 fnj = fn[af_idx[j]];
@@ -130,6 +141,13 @@ __global__ void k_realize_vnormals(int nv, const int *__restrict__ af_ptr, const
     }
     vn[i] = make_double4(n0, n1, n2, 0.0);
     if (vnf) vnf[i] = make_float4((float)n0, (float)n1, (float)n2, 0.0f);
+}
+__global__ void k_realize_vnormals(int nv, const int *__restrict__ af_ptr, const int *__restrict__ af_idx,
+                                   const double4 *__restrict__ fn, double4 *__restrict__ vn,
+                                   float4 *__restrict__ vnf)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nv) realize_vnormal(i, af_ptr, af_idx, fn, vn, vnf);
 }
 
 // ------------------------------------------------------------- transforms
@@ -162,32 +180,6 @@ __global__ void k_xform(const FrameGeom *__restrict__ geoms, const double4 *__re
     store_vt(vt, g.vt_base + i, t[0], t[1], t[2]);
 }
 
-// The same transform of vertices realized on the fly (realize_vertex, the
-// operations k_realize_vf uses), so the batched graph can run it beside
-// k_realize_vf instead of after it: the view-frame vertices are identical.
-template <typename T4>
-__global__ void k_xform_realize(const FrameGeom *__restrict__ geoms, const double *__restrict__ a,
-                                const double *__restrict__ u, const double *__restrict__ r,
-                                const double *__restrict__ scale, const int *__restrict__ vcomp,
-                                const double *__restrict__ cxf, int nv, T4 *__restrict__ vt)
-{
-    grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
-    const FrameGeom &g = geoms[blockIdx.y];
-    double4 x = realize_vertex(i, a, u, r, scale, vcomp, cxf);
-    double t[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        t[k] = 0.0;
-        t[k] += g.oa[3 * k + 0] * x.x;
-        t[k] += g.oa[3 * k + 1] * x.y;
-        t[k] += g.oa[3 * k + 2] * x.z;
-        t[k] += g.off[k];
-    }
-    store_vt(vt, g.vt_base + i, t[0], t[1], t[2]);
-}
-
 // -------------------------------------------------------------- binning
 
 // Resident 256-thread blocks per SM the binning kernel's registers must
@@ -204,10 +196,18 @@ template <typename T4>
 __global__ void __launch_bounds__(256, BIN_MIN_BLOCKS) k_bin(const FrameGeom *__restrict__ geoms, int view0, int nf,
                       const int4 *__restrict__ fvi, const double4 *__restrict__ fn,
                       const T4 *__restrict__ vt, FrameState *__restrict__ states,
-                      int *__restrict__ bin_count, int2 *__restrict__ bin_ids, int cap)
+                      int *__restrict__ bin_count, int2 *__restrict__ bin_ids, int cap, VnormalArgs vna)
 {
+    grid_dep_trigger();
     grid_dep_wait();
     int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (vna.nv > 0 && blockIdx.y == gridDim.y - 1) {
+        // the batched graph's last row of blocks: the vertex normals, which
+        // like the binning wait for the facet normals only
+        for (int i = f; i < vna.nv; i += gridDim.x * blockDim.x)
+            realize_vnormal(i, vna.af_ptr, vna.af_idx, fn, vna.vn, vna.vnf);
+        return;
+    }
     if (f >= nf) return;
     int v = view0 + blockIdx.y;
     const FrameGeom &g = geoms[v];
@@ -292,29 +292,96 @@ __global__ void __launch_bounds__(256, BIN_MIN_BLOCKS) k_bin(const FrameGeom *__
         }
 }
 
+__device__ inline FrameState blank_state()
+{
+    FrameState s;
+    s.outbnd = 0;
+    s.bin_overflow = 0;
+    s.cov_i[0] = s.cov_j[0] = INT_MAX;
+    s.cov_i[1] = s.cov_j[1] = INT_MIN;
+    s.ofr_i[0] = s.ofr_j[0] = INT_MAX;
+    s.ofr_i[1] = s.ofr_j[1] = INT_MIN;
+    s.ofr_ov[0] = s.ofr_ov[2] = dkey(HUGENUMBER);
+    s.ofr_ov[1] = s.ofr_ov[3] = dkey(-HUGENUMBER);
+    s.idellim[0] = s.idoplim[0] = INT_MAX;
+    s.idellim[1] = s.idoplim[1] = INT_MIN;
+    s.dellim[0] = s.doplim[0] = dkey(HUGENUMBER);
+    s.dellim[1] = s.doplim[1] = dkey(-HUGENUMBER);
+    s.any_lit = 0;
+    s.any_overflow = 0;
+    return s;
+}
 __global__ void k_reset_state(FrameState *st, int nviews, int *bin_count, int ntiles)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nviews) {
-        FrameState s;
-        s.outbnd = 0;
-        s.bin_overflow = 0;
-        s.cov_i[0] = s.cov_j[0] = INT_MAX;
-        s.cov_i[1] = s.cov_j[1] = INT_MIN;
-        s.ofr_i[0] = s.ofr_j[0] = INT_MAX;
-        s.ofr_i[1] = s.ofr_j[1] = INT_MIN;
-        s.ofr_ov[0] = s.ofr_ov[2] = dkey(HUGENUMBER);
-        s.ofr_ov[1] = s.ofr_ov[3] = dkey(-HUGENUMBER);
-        s.idellim[0] = s.idoplim[0] = INT_MAX;
-        s.idellim[1] = s.idoplim[1] = INT_MIN;
-        s.dellim[0] = s.doplim[0] = dkey(HUGENUMBER);
-        s.dellim[1] = s.doplim[1] = dkey(-HUGENUMBER);
-        s.any_lit = 0;
-        s.any_overflow = 0;
-        st[i] = s;
-    }
+    if (i < nviews) st[i] = blank_state();
     for (int t = i; t < ntiles; t += gridDim.x * blockDim.x)
         bin_count[t] = 0;
+}
+
+// The first launch of a batched evaluation: everything that depends only on the
+// parameters or on nothing, by ranges of blocks. The views' vertices
+// (each realized on the fly with k_realize_vf's operations, then k_xform's),
+// the facets' normals and areas, the vertices, the views' blank states and bin
+// counts, and the cleared images. As separate launches on side branches (a
+// reset kernel and three or four clears after one another) the clears ended
+// 9.8 us after the parameters had arrived and binning started then; as one
+// launch it starts after 2.8 (one frame).
+struct FrontParams {
+    const FrontArgs &a;
+    __device__ double r(int i) const
+    {
+        double v = a.m.r[i];
+        for (int k = 0; k < a.nchange; k++)
+            if (a.change_at[k] == i) v = a.change_to[k];
+        return v;
+    }
+    __device__ double scale(int k) const { return a.nscale ? a.scale[k] : a.m.scale[k]; }
+};
+__global__ void __launch_bounds__(256) k_front(const __grid_constant__ FrontArgs a)
+{
+    grid_dep_trigger();
+    const ModelDev &m = a.m;
+    const FrontParams par{a};
+    int b = blockIdx.x;
+    if (b < a.nb_xform) {
+        const int bpv = (m.nv + 255) / 256, v = b / bpv;
+        const int i = (b - v * bpv) * 256 + threadIdx.x;
+        if (i >= m.nv) return;
+        const FrameGeom &g = a.geoms[v];
+        const double4 x = realize_vertex(i, m.a, m.u, par, m.vcomp, m.cxf);
+        double t[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            t[k] = 0.0;
+            t[k] += g.oa[3 * k + 0] * x.x;
+            t[k] += g.oa[3 * k + 1] * x.y;
+            t[k] += g.oa[3 * k + 2] * x.z;
+            t[k] += g.off[k];
+        }
+        store_vt(a.vt, g.vt_base + i, t[0], t[1], t[2]);
+        return;
+    }
+    b -= a.nb_xform;
+    if (b < a.nb_model) {
+        realize_vf(b * 256 + threadIdx.x, m.nv, m.nf, m.a, m.u, par, m.vcomp, m.cxf, m.fv, m.vx, m.fn, m.area, m.fvi);
+        return;
+    }
+    b -= a.nb_model;
+    const int nb = gridDim.x - a.nb_xform - a.nb_model;
+    const long long t0 = (long long)b * 256 + threadIdx.x, step = (long long)nb * 256;
+    for (long long i = t0; i < a.nviews; i += step) a.states[i] = blank_state();
+    if (b == 0) {
+        if (threadIdx.x < a.nscale) a.scale_out[threadIdx.x] = a.scale[threadIdx.x];
+        if (threadIdx.x < a.nchange) a.r_out[a.change_at[threadIdx.x]] = a.change_to[threadIdx.x];
+    }
+    for (int k = 0; k < FrontArgs::CLEARS; k++) {
+        // 16-byte stores, then the last bytes
+        const size_t n16 = a.clear_bytes[k] / 16;
+        int4 *p = reinterpret_cast<int4 *>(a.clear[k]);
+        for (size_t i = (size_t)t0; i < n16; i += (size_t)step) p[i] = make_int4(0, 0, 0, 0);
+        if (t0 < (long long)(a.clear_bytes[k] % 16)) a.clear[k][16 * n16 + t0] = 0;
+    }
 }
 
 // ----------------------------------------------------------------- chi2
@@ -517,6 +584,8 @@ __device__ shape_deldop_result finalize_frame(const FinalizeArgs &a, int fr, con
 // its mean bin) and flags a model wider than the overflow spectrum.
 __global__ void k_doppler_overflow(DopOvfArgs a)
 {
+    grid_dep_trigger();
+    grid_dep_wait();
     __shared__ double red[4][32];
     const int k = blockIdx.x;
     const int fr = a.frames[k];
@@ -579,6 +648,8 @@ __global__ void k_doppler_overflow(DopOvfArgs a)
 template <typename T>
 __global__ void k_lc_photo(LcArgs a)
 {
+    grid_dep_trigger();
+    grid_dep_wait();
     __shared__ double red[32];
     for (int it = blockIdx.x; it < a.nitems; it += gridDim.x) {
         int2 item = a.items[it];
@@ -749,6 +820,8 @@ __device__ double poset_sample(const double *B, int n, int side, int mode, doubl
 // calibration (src/shape/chi2.c) and the views' posbnd terms.
 __global__ void k_poset_frames(PosetArgs a)
 {
+    grid_dep_trigger();
+    grid_dep_wait();
     __shared__ double red[5][32];
     __shared__ int redi[32];
     const PosetFrameDev F = a.frames[blockIdx.x];
@@ -909,6 +982,8 @@ __device__ double splint_dev(const double *x, const double *y, const double *y2,
 // instead of one global round trip per step.
 __global__ void k_lc_finalize(LcFinalizeArgs a)
 {
+    grid_dep_trigger();
+    grid_dep_wait();
     extern __shared__ double lsm[];
     const LcSetDev &S = a.sets[blockIdx.x];
     const int np = S.npts, n = S.n;
@@ -1002,6 +1077,7 @@ __device__ void summary_totals(const SummaryArgs &a, Term term);
 
 __global__ void k_summary(FinalizeArgs fa, SummaryArgs a)
 {
+    grid_dep_wait();
     extern __shared__ double ssm[];
     const bool use_sm = a.smem_frames;
     double *s_chi2 = ssm, *s_plog = ssm + fa.nframes, *s_blog = ssm + 2 * (size_t)fa.nframes;
@@ -1123,11 +1199,19 @@ template <typename T>
 __device__ void chi2_item_warp(const Chi2Args &a, int it, const Chi2Item &item, double *part)
 {
     const int lane = threadIdx.x & 31;
-    const FrameGeom &g = a.geoms[a.frame_view[item.frame]];
-    const long long base = g.fit_base + item.start;
+    const long long base = item.base;
     const T *fit = static_cast<const T *>(a.fit) + base;
     const double *obs = a.obs + base, *oov = a.oov + base;
     const bool pre = a.o2pre != nullptr;
+    if (pre && item.view >= 0) {
+        // no footprint reaches the item's rows: its fit is zero
+        const FrameState &st = a.states[item.view];
+        if (item.row1 < st.idellim[0] || item.row0 > st.idellim[1]) {
+            if (lane < 2) part[lane] = a.o2pre[2 * (size_t)it + lane];
+            else if (lane < 6) part[lane] = 0.0;
+            return;
+        }
+    }
     T ft[CHI2_LANE];
 #pragma unroll
     for (int j = 0; j < CHI2_LANE; j++) {
@@ -1173,8 +1257,8 @@ __device__ void chi2_item_warp(const Chi2Args &a, int it, const Chi2Item &item, 
 // grid-stride order. A frame's counter takes one count per item; the warp
 // that makes the frame's last count merges the frame's item partials
 // (frame_sums_warp, the order k_summary's frame_sums_serial reproduces) and
-// writes the frame's results (limits, flags, log-factors and chi-square
-// terms), and the warp that completes the last frame computes the totals in
+// writes the frame's chi-square terms (the warp of its first item has written
+// the limits, flags and log-factors), and the warp that completes the last frame computes the totals in
 // dataset order, as k_chi2_partials + k_summary do. Values another warp
 // wrote in this launch are read through L2 (__ldcg) after a fence.
 // counters: [nframes] per frame, then the finished frames; zero before the
@@ -1184,15 +1268,18 @@ __global__ void __launch_bounds__(CHI2_THREADS, CHI2_MIN_BLOCKS) k_chi2_summary(
                                                                int *counters)
 {
     extern __shared__ __align__(16) unsigned char stage[];   // chi2_summary_smem bytes (the totals)
-    grid_dep_wait();
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (int it = blockIdx.x * wpb + (threadIdx.x >> 5); it < ca.nitems; it += gridDim.x * wpb) {
-        const Chi2Item item = ca.items[it];
+    int it = blockIdx.x * wpb + (threadIdx.x >> 5);
+    Chi2Item item = ca.items[min(it, ca.nitems - 1)];         // constant data: read before the wait
+    grid_dep_wait();
+    for (; it < ca.nitems; it += gridDim.x * wpb, item = ca.items[min(it, ca.nitems - 1)]) {
         chi2_item_warp<T>(ca, it, item, ca.partials + (size_t)it * 6);
         const int fr = item.frame;
         const FrameHost &h = fa.fh[fr];
+        if (it == h.item0 && lane == 0) finalize_frame_geom(fa, fr, fa.results[fr]);
         int last = 0;
+        __syncwarp();                                         // a skipped item's lanes wrote its partials
         if (lane == 0) {
             __threadfence();                                  // the partials before the count
             last = (atomicAdd(&counters[fr], 1) == h.nitems - 1);
@@ -1206,10 +1293,7 @@ __global__ void __launch_bounds__(CHI2_THREADS, CHI2_MIN_BLOCKS) k_chi2_summary(
         frame_sums_warp(ca.partials + (size_t)h.item0 * 6, h.nitems, start, q, true);
         int lastf = 0;
         if (lane == 0) {
-            shape_deldop_result r;
-            finalize_frame_geom(fa, fr, r);
-            frame_chi2_from_sums(h, q, r);
-            fa.results[fr] = r;
+            frame_chi2_from_sums(h, q, fa.results[fr]);
             __threadfence();                                  // the results before the count
             lastf = (atomicAdd(&counters[fa.nframes], 1) == fa.nframes - 1);
         }
@@ -1270,10 +1354,17 @@ void launch_reset_state(FrameState *st, int nviews, int *bin_count, int ntiles, 
     k_reset_state<<<blocks, 256, 0, s>>>(st, nviews, bin_count, ntiles);
 }
 
-void launch_xform_realize_f64(const FrameGeom *g, int nviews, const ModelDev &m, double4 *vt, cudaStream_t s)
+void launch_front(const FrontArgs &a0, cudaStream_t s)
 {
-    dim3 grid((m.nv + 255) / 256, nviews);
-    k_xform_realize<double4><<<grid, 256, 0, s>>>(g, m.a, m.u, m.r, m.scale, m.vcomp, m.cxf, m.nv, vt);
+    FrontArgs a = a0;
+    a.nb_xform = a.nviews * ((a.m.nv + 255) / 256);
+    a.nb_model = (a.m.nf + a.m.nv + 255) / 256;
+    size_t words = (size_t)a.nviews;
+    for (size_t n : a.clear_bytes) words = n / 16 > words ? n / 16 : words;
+    // four 16-byte stores a thread, at most four blocks per SM
+    size_t nb = (words + 1023) / 1024;
+    nb = nb < 1 ? 1 : nb > 4 * 148 ? 4 * 148 : nb;
+    k_front<<<a.nb_xform + a.nb_model + (int)nb, 256, 0, s>>>(a);
 }
 
 void launch_xform_f64(const FrameGeom *g, int nviews, const double4 *vx, int nv, double4 *vt, cudaStream_t s,
@@ -1285,11 +1376,12 @@ void launch_xform_f64(const FrameGeom *g, int nviews, const double4 *vx, int nv,
 
 
 void launch_bin_f64(const FrameGeom *g, int view0, int nviews, const ModelDev &m, const double4 *vt,
-                    FrameState *st, int *bin_count, int2 *bin_ids, int cap, cudaStream_t s, bool pdl)
+                    FrameState *st, int *bin_count, int2 *bin_ids, int cap, cudaStream_t s, bool pdl, bool vnormals)
 {
-    dim3 grid((m.nf + 255) / 256, nviews);
+    dim3 grid((m.nf + 255) / 256, nviews + (vnormals ? 1 : 0));
+    const VnormalArgs vna = {vnormals ? m.nv : 0, m.af_ptr, m.af_idx, m.vn, m.vnf};
     launch_k(k_bin<double4>, grid, dim3(256), 0, s, pdl, g, view0, m.nf, (const int4 *)m.fvi, (const double4 *)m.fn,
-             vt, st, bin_count, bin_ids, cap);
+             vt, st, bin_count, bin_ids, cap, vna);
 }
 
 
@@ -1308,37 +1400,38 @@ void launch_chi2_partials(const Chi2Args &a, int fp32, cudaStream_t s)
 __global__ void k_dop_fit_f32(const int *dop_frames, const FrameHost *fh, const FrameGeom *geoms,
                               const double *fit64, float *fit32)
 {
+    grid_dep_trigger();
+    grid_dep_wait();
     const FrameGeom &g = geoms[fh[dop_frames[blockIdx.x]].view];
     const long long n = (long long)g.ndel * g.ndop;
     for (long long j = threadIdx.x; j < n; j += blockDim.x) fit32[g.fit_base + j] = (float)fit64[g.fit_base + j];
 }
 
 void launch_dop_fit_f32(const int *dop_frames, int n, const FrameHost *fh, const FrameGeom *geoms,
-                        const double *fit64, float *fit32, cudaStream_t s)
+                        const double *fit64, float *fit32, cudaStream_t s, bool pdl)
 {
     if (n <= 0) return;
-    k_dop_fit_f32<<<n, 256, 0, s>>>(dop_frames, fh, geoms, fit64, fit32);
+    launch_k(k_dop_fit_f32, dim3(n), dim3(256), 0, s, pdl, dop_frames, fh, geoms, fit64, fit32);
 }
 
-void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s)
+void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s, bool pdl)
 {
     if (a.n <= 0) return;
-    k_doppler_overflow<<<a.n, 256, 0, s>>>(a);
+    launch_k(k_doppler_overflow, dim3(a.n), dim3(256), 0, s, pdl, a);
 }
 
 
-void launch_poset_frames(const PosetArgs &a, cudaStream_t s)
+void launch_poset_frames(const PosetArgs &a, cudaStream_t s, bool pdl)
 {
     if (a.nframes <= 0) return;
-    k_poset_frames<<<a.nframes, 256, 0, s>>>(a);
+    launch_k(k_poset_frames, dim3(a.nframes), dim3(256), 0, s, pdl, a);
 }
 
-void launch_lc_photo(const LcArgs &a, int fp32, cudaStream_t s)
+void launch_lc_photo(const LcArgs &a, cudaStream_t s, bool pdl)
 {
     int blocks = a.nitems < 8 * 148 ? a.nitems : 8 * 148;
     if (blocks <= 0) return;
-    if (fp32) k_lc_photo<float><<<blocks, 256, 0, s>>>(a);
-    else k_lc_photo<double><<<blocks, 256, 0, s>>>(a);
+    launch_k(k_lc_photo<double>, dim3(blocks), dim3(256), 0, s, pdl, a);
 }
 
 // Shared memory one set needs (0 when it exceeds the block's budget: the
@@ -1355,10 +1448,10 @@ cudaError_t configure_lc_finalize()
                                 (int)LC_FINALIZE_SMEM_MAX);
 }
 
-void launch_lc_finalize(const LcFinalizeArgs &a, cudaStream_t s)
+void launch_lc_finalize(const LcFinalizeArgs &a, cudaStream_t s, bool pdl)
 {
     if (a.nsets <= 0) return;
-    k_lc_finalize<<<a.nsets, 256, a.smem_per_set, s>>>(a);
+    launch_k(k_lc_finalize, dim3(a.nsets), dim3(256), a.smem_per_set, s, pdl, a);
 }
 
 // Shared memory of the summary: per-frame terms, then (when they fit) the
@@ -1399,14 +1492,14 @@ void launch_chi2_summary(const Chi2Args &ca, const FinalizeArgs &fa, const Summa
     else launch_k(k_chi2_summary<double>, dim3(blocks), dim3(CHI2_THREADS), smem, s, pdl, ca, fa, sa, counters);
 }
 
-void launch_summary(const FinalizeArgs &fa, const SummaryArgs &a, cudaStream_t s)
+void launch_summary(const FinalizeArgs &fa, const SummaryArgs &a, cudaStream_t s, bool pdl)
 {
     SummaryArgs b = a;
     int wp = 0;
     const size_t sm = summary_smem(fa.nframes, a.nitems, &wp);
     b.smem_frames = (sm > 0 && fa.nframes > 0) ? 1 : 0;
     b.smem_partials = b.smem_frames && wp;
-    k_summary<<<1, 256, b.smem_frames ? sm : 0, s>>>(fa, b);
+    launch_k(k_summary, dim3(1), dim3(256), b.smem_frames ? sm : 0, s, pdl, fa, b);
 }
 
 

@@ -87,7 +87,7 @@ int EngineImpl::finalize()
     if (!have_model) return set_err(SHAPE_E_STATE, "finalize: no model set");
     if (dd.empty() && lc.empty() && ps.empty()) return set_err(SHAPE_E_STATE, "finalize: no datasets");
     mem.release();
-    invalidate_graphs();
+    dev_params.clear();
     for (int f = 0; f < 3; f++) tuned[f] = 0;
     d_work_sorted = nullptr;
     d_sides = nullptr; d_msum_part = d_msum = nullptr;
@@ -188,7 +188,11 @@ int EngineImpl::finalize()
             h.item0 = (int)chi2_items.size();
             int D = F.ndel * F.ndop, chunk = CHI2_ITEM;
             for (int st = 0; st < D; st += chunk)
-                chi2_items.push_back(Chi2Item{fi, st, std::min(chunk, D - st)});
+            {
+                const int cnt = std::min(chunk, D - st);
+                chi2_items.push_back(Chi2Item{fi, cnt, st / F.ndop + 1, (st + cnt - 1) / F.ndop + 1,
+                                              nview > 1 ? -1 : h.view, 0, g.fit_base + st});
+            }
             h.nitems = (int)chi2_items.size() - h.item0;
             fh.push_back(h);
             add_view(g, F.pos_n, F.km_per_pixel);
@@ -416,7 +420,7 @@ int EngineImpl::finalize()
         memset(&c0, 0, sizeof c0);
         c0.items = d_chi2_items; c0.nitems = (int)chi2_items.size();
         c0.obs = d_obs; c0.oov = d_oov; c0.fit = d_fit64;
-        c0.geoms = d_geoms; c0.frame_view = d_frame_view; c0.partials = d_partials;
+        c0.states = d_states; c0.partials = d_partials;
         c0.o2pre = nullptr;
         launch_chi2_partials(c0, 0, s);
         CK(cudaMemcpy2DAsync(d_o2pre, 2 * sizeof(double), d_partials, 6 * sizeof(double), 2 * sizeof(double),
@@ -461,11 +465,6 @@ int EngineImpl::finalize()
     CK(cudaMemsetAsync(d_seen, 0, nf, s));
     CK(cudaStreamSynchronize(s));
 
-    if (!stream2) {
-        CK(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&stream3, cudaStreamNonBlocking));
-        for (auto &e : evf) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
     CK(configure_raster_f64());
     CK(configure_raster_f32());
     CK(configure_lc_finalize());
@@ -495,7 +494,7 @@ int EngineImpl::finalize()
 // its constants are recomputed as finalize computes them and the changed
 // elements copied to the device on the engine stream, ahead of the next
 // evaluation. Every kernel reads them through the device arrays, so the
-// captured graphs stay valid.
+// next launches see them.
 int EngineImpl::set_frame_view(int fi, const double ae[9], const double oe[9], const double spin[3],
                                double deloff, double dopoff)
 {
@@ -624,7 +623,7 @@ int EngineImpl::realize_views()
 // Spin realization inside the evaluation: one source per radar frame and
 // lightcurve point (its epoch, dataset record and orbital spin), device
 // copies of the frames, points and delay-Doppler sets it rebuilds views
-// from, and the pinned spin state and offsets the graph copies in.
+// from, and the pinned spin state and offsets each evaluation copies in.
 int EngineImpl::setup_spin_device()
 {
     n_spin_src = 0;
@@ -684,7 +683,6 @@ int EngineImpl::setup_spin_device()
                            cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
     n_spin_src = (int)src.size();
-    invalidate_graphs();
     return SHAPE_OK;
 }
 
@@ -996,8 +994,7 @@ double EngineImpl::penalty_sum(const double *ms)
 int EngineImpl::tune_bins()
 {
     cudaStream_t s = stream;
-    fill_params(h_params);
-    CK(cudaMemcpyAsync(d_r, h_params, sizeof(double) * npar(), cudaMemcpyHostToDevice, s));
+    if (int rc0 = upload_params()) return rc0;
     launch_realize(md, s);
     launch_reset_state(d_states, nviews, d_bin_count, ntiles, s);
     launch_xform_f64(d_geoms, nviews, md.vx, nv, d_vt64, s);
@@ -1066,42 +1063,47 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (e == cudaSuccess) return SHAPE_OK;
         return set_err(SHAPE_E_CUDA, std::string(stage) + ": " + cudaGetErrorString(e));
     };
-    // The batched forms run two side branches beside the view transform
-    // (which realizes its vertices on the fly): the state reset and image
-    // clears (stream2), and realize with the facet and vertex normals
-    // (stream3); binning waits for the facet normals and the reset, the
-    // raster for the vertex normals. The plain form and stage timing run
-    // them in line.
-    const bool fork = (form != SHAPE_FORM_PLAIN_FP64) && !marks;
-    cudaStream_t sr = fork ? stream2 : s;
+    // A batched evaluation opens with one launch for realize, the view
+    // transforms, the blank states and the clears (k_front), and its binning
+    // launch carries the vertex normals; the plain form and stage timing run
+    // them one by one, from the uploaded parameters.
+    const bool chain = (form != SHAPE_FORM_PLAIN_FP64) && !marks;
+    const bool fused = fused_chi2 && form != SHAPE_FORM_PLAIN_FP64;
+    // the FP32 form sums Doppler spectra in FP64 (then rounds them once)
+    const bool need64 = fit_elems && (!f32 || !dop_frames.empty());
     if (int rc = enqueue_spin()) return rc;
-    if (fork) {
-        CK(cudaEventRecord(evf[0], s));
-        CK(cudaStreamWaitEvent(stream2, evf[0], 0));
-        CK(cudaStreamWaitEvent(stream3, evf[0], 0));
-        launch_realize_vf(md, stream3);
-        CK(cudaEventRecord(evf[1], stream3));        // vertices, facet normals and areas
-        launch_realize_vn(md, stream3);
-        CK(cudaEventRecord(evf[3], stream3));        // vertex normals
+    if (chain) {
+        FrontArgs fr;
+        memset(&fr, 0, sizeof fr);
+        fr.geoms = d_geoms; fr.nviews = nviews; fr.m = md; fr.vt = d_vt64; fr.states = d_states;
+        int k = 0;
+        auto clear = [&](void *p, size_t bytes) {
+            fr.clear[k] = static_cast<unsigned char *>(p);
+            fr.clear_bytes[k++] = bytes;
+        };
+        clear(d_bin_count, sizeof(int) * (size_t)ntiles);
+        clear(d_seen, nf);
+        if (f32 && fit_elems) clear(d_fit32, sizeof(float) * (size_t)fit_elems);
+        if (need64) clear(d_fit64, sizeof(double) * (size_t)fit_elems);
+        if (!dop_frames.empty()) clear(d_ovf, sizeof(double) * dop_frames.size() * DOP_MAXOVERFLOW);
+        if (fused) clear(d_chi2_counters, sizeof(int) * (fh.size() + 1));
+        if (int rc_ = front_params(fr)) return rc_;
+        launch_front(fr, s);
+        if (int rc_ = launched("realize and transform")) return rc_;
     } else {
         launch_realize(md, s);
+        mark(0);
+        if (int rc_ = launched("realize")) return rc_;
+        launch_reset_state(d_states, nviews, d_bin_count, ntiles, s);
+        if (f32 && fit_elems) CK(cudaMemsetAsync(d_fit32, 0, sizeof(float) * fit_elems, s));
+        if (need64) CK(cudaMemsetAsync(d_fit64, 0, sizeof(double) * fit_elems, s));
+        CK(cudaMemsetAsync(d_seen, 0, nf, s));
+        if (!dop_frames.empty())
+            CK(cudaMemsetAsync(d_ovf, 0, sizeof(double) * dop_frames.size() * DOP_MAXOVERFLOW, s));
+        if (fused) CK(cudaMemsetAsync(d_chi2_counters, 0, sizeof(int) * (fh.size() + 1), s));
+        mark(1);
+        if (int rc_ = launched("state reset")) return rc_;
     }
-    mark(0);
-    if (int rc_ = launched("realize")) return rc_;
-    launch_reset_state(d_states, nviews, d_bin_count, ntiles, sr);
-    if (fit_elems) {
-        if (f32) CK(cudaMemsetAsync(d_fit32, 0, sizeof(float) * fit_elems, sr));
-        // the FP32 form sums Doppler spectra in FP64 (then rounds them once)
-        if (!f32 || !dop_frames.empty()) CK(cudaMemsetAsync(d_fit64, 0, sizeof(double) * fit_elems, sr));
-    }
-    CK(cudaMemsetAsync(d_seen, 0, nf, sr));
-    if (!dop_frames.empty())
-        CK(cudaMemsetAsync(d_ovf, 0, sizeof(double) * dop_frames.size() * DOP_MAXOVERFLOW, sr));
-    const bool fused = fused_chi2 && form != SHAPE_FORM_PLAIN_FP64;
-    if (fused) CK(cudaMemsetAsync(d_chi2_counters, 0, sizeof(int) * (fh.size() + 1), sr));
-    if (fork) CK(cudaEventRecord(evf[2], stream2));   // reset and clears done
-    mark(1);
-    if (int rc_ = launched("state reset")) return rc_;
 
     RasterArgs ra;
     memset(&ra, 0, sizeof ra);
@@ -1129,8 +1131,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     Chi2Args ca;
     ca.obs = d_obs; ca.oov = d_oov;
     ca.fit = ra.fit;
-    ca.geoms = d_geoms;
-    ca.frame_view = d_frame_view;
+    ca.states = d_states;
     ca.partials = d_partials;
     ca.o2pre = d_o2pre;
 
@@ -1172,25 +1173,19 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
                 lv.items = d_lc_items + pt_items[2 * pt];
                 lv.nitems = pt_items[2 * pt + 1];
                 lv.partials = d_lc_partials + pt_items[2 * pt];
-                launch_lc_photo(lv, 0, s);
+                launch_lc_photo(lv, s, false);
             }
             if (int rc_ = launched(g.kind == VIEW_RADAR ? "radar view chain" : "lightcurve view chain")) return rc_;
         }
     } else {
-        // graph-captured chain: each kernel after the first is a programmatic
+        // each kernel of the chain after the first is a programmatic
         // dependent launch of the one before it (stage timing keeps plain
         // launches so its events separate the stages)
-        const bool pdl = fork;
-        if (fork) launch_xform_realize_f64(d_geoms, nviews, md, d_vt64, s);
-        else launch_xform_f64(d_geoms, nviews, md.vx, nv, d_vt64, s);
+        const bool pdl = chain;
+        if (!chain) launch_xform_f64(d_geoms, nviews, md.vx, nv, d_vt64, s);
         mark(2);
         if (int rc_ = launched("view transform")) return rc_;
-        if (fork) {
-            CK(cudaStreamWaitEvent(s, evf[1], 0));
-            CK(cudaStreamWaitEvent(s, evf[2], 0));
-        }
-        launch_bin_f64(d_geoms, 0, nviews, md, d_vt64, d_states, d_bin_count, d_bin_ids, cap, s, pdl);
-        if (fork) CK(cudaStreamWaitEvent(s, evf[3], 0));
+        launch_bin_f64(d_geoms, 0, nviews, md, d_vt64, d_states, d_bin_count, d_bin_ids, cap, s, pdl, chain);
         mark(3);
         if (int rc_ = launched("binning")) return rc_;
         // one CTA per tile, heaviest tiles first (empty tiles sort last and
@@ -1214,7 +1209,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (f32) {
             launch_raster_f32(rr, s);
             launch_raster_f64(rl, s);
-            launch_dop_fit_f32(d_dop_frames, (int)dop_frames.size(), d_fh, d_geoms, d_fit64, d_fit32, s);
+            launch_dop_fit_f32(d_dop_frames, (int)dop_frames.size(), d_fh, d_geoms, d_fit64, d_fit32, s, pdl);
         } else {
             launch_raster_f64(rr, s);
             launch_raster_f64(rl, s);
@@ -1231,7 +1226,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
             la.items = d_lc_items;
             la.nitems = (int)lc_items.size();
             // lightcurve views hold FP64 cosines in both forms
-            launch_lc_photo(la, 0, s);
+            launch_lc_photo(la, s, pdl);
         }
         mark(6);
         if (int rc_ = launched("lightcurve photometry")) return rc_;
@@ -1248,7 +1243,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         oa.n = (int)dop_frames.size();
         oa.frames = d_dop_frames; oa.fh = d_fh; oa.geoms = d_geoms; oa.states = d_states;
         oa.ovf = d_ovf; oa.out = d_ovf_out;
-        launch_doppler_overflow(oa, s);
+        launch_doppler_overflow(oa, s, chain);
         if (int rc_ = launched("Doppler overflow")) return rc_;
     }
     if (!psf.empty()) {
@@ -1256,7 +1251,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         pa.nframes = (int)psf.size();
         pa.frames = d_psf; pa.pts = d_lcpts; pa.geoms = d_geoms; pa.states = d_states;
         pa.bimg = d_ps_b; pa.obs = d_ps_obs; pa.oov = d_ps_oov; pa.fit = d_ps_fit; pa.res = d_ps_res;
-        launch_poset_frames(pa, s);
+        launch_poset_frames(pa, s, chain);
         if (int rc_ = launched("plane-of-sky frames")) return rc_;
     }
     if (!lcdev.empty()) {
@@ -1270,7 +1265,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
             sm = (b == 0 || sm == 0) ? 0 : std::max(sm, b);
         }
         lf.smem_per_set = sm;
-        launch_lc_finalize(lf, s);
+        launch_lc_finalize(lf, s, chain);
         if (int rc_ = launched("lightcurve finalize")) return rc_;
     }
     SummaryArgs sa;
@@ -1282,14 +1277,14 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     sa.dof = dof; sa.dof_radar = dof_deldop + dof_doppler; sa.bad_objfactor = bad_objfactor;
     sa.nitems = (int)chi2_items.size();
     // the bad-diameter factor depends only on host-side scale factors and is
-    // applied by evaluate(), so captured graphs stay valid when it changes
+    // applied by evaluate()
     sa.baddiam = 0;
     sa.baddiam_logfactor = 0.0;
     // the summary kernel writes the pinned host summary directly (mapped
     // memory), so an evaluation needs no device-to-host copy after it
     sa.out = d_summary_map;
-    if (fused) launch_chi2_summary(ca, fa, sa, d_chi2_counters, f32 ? 1 : 0, s, fork, fused_smem);
-    else launch_summary(fa, sa, s);
+    if (fused) launch_chi2_summary(ca, fa, sa, d_chi2_counters, f32 ? 1 : 0, s, chain, fused_smem);
+    else launch_summary(fa, sa, s, chain && (!chi2_items.empty() || !lcdev.empty() || !psf.empty()));
     mark(7);
     CK(cudaGetLastError());
     return SHAPE_OK;
@@ -1299,14 +1294,16 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
 // and copies excluded).
 int EngineImpl::kernels_per_eval(int form) const
 {
-    int n = 2 + 1;                       // realize (vertices + facets, vertex normals), state reset
+    // front and binning, or realize (vertices + facets, vertex normals) and the
+    // state reset
+    int n = form == SHAPE_FORM_PLAIN_FP64 ? 3 : 2;
     n += (spin_device && n_spin_src > 0) ? 1 : 0;   // view realization from the spin state
     if (form == SHAPE_FORM_PLAIN_FP64) {
         for (int v = 0; v < nviews; v++)
             n += 3 + ((geoms[v].kind == VIEW_RADAR && fh[geoms[v].frame_index].view == v) ||
                               geoms[v].kind == VIEW_LC_SUN ? 1 : 0);
     } else {
-        n += 3;                          // transform, bin, raster
+        n += 1;                          // raster
         if (work_radar > 0 && work_radar < (int)work.size())
             n += 1;                      // radar and lightcurve / sky views in two launches
         if (form == SHAPE_FORM_BATCHED_FP32 && !dop_frames.empty())
@@ -1321,6 +1318,47 @@ int EngineImpl::kernels_per_eval(int form) const
     return n + 1;                        // finalize + summary (with the chi-square partials when fused)
 }
 
+// Every parameter to the device on the engine stream.
+int EngineImpl::upload_params()
+{
+    dev_params.clear();
+    fill_params(h_params);
+    CK(cudaMemcpyAsync(d_r, h_params, sizeof(double) * npar(), cudaMemcpyHostToDevice, stream));
+    dev_params.assign(h_params, h_params + npar());
+    return SHAPE_OK;
+}
+
+// The parameters of a batched evaluation: what differs from the device's
+// arrays travels in k_front's arguments when it is a few numbers (a trial
+// moves one to a few), else everything is uploaded first.
+int EngineImpl::front_params(FrontArgs &fr)
+{
+    bool fits = (int)dev_params.size() == npar() && 3 * ncomp <= FrontArgs::SCALES;
+    const int BLOCK = 512;
+    for (int b = 0; b < nv && fits; b += BLOCK) {
+        const int n = std::min(BLOCK, nv - b);
+        if (memcmp(&r[b], &dev_params[b], sizeof(double) * n) == 0) continue;
+        for (int i = b; i < b + n && fits; i++) {
+            if (memcmp(&r[i], &dev_params[i], sizeof(double)) == 0) continue;
+            if ((fits = fr.nchange < FrontArgs::CHANGES)) {
+                fr.change_at[fr.nchange] = i;
+                fr.change_to[fr.nchange++] = r[i];
+            }
+        }
+    }
+    if (!fits) {
+        fr.nscale = fr.nchange = 0;
+        return upload_params();
+    }
+    fr.r_out = d_r;
+    fr.scale_out = d_scale;
+    fr.nscale = 3 * ncomp;
+    effective_scale(fr.scale, nullptr, nullptr);
+    for (int k = 0; k < fr.nchange; k++) dev_params[fr.change_at[k]] = fr.change_to[k];
+    memcpy(&dev_params[nv], fr.scale, sizeof(double) * fr.nscale);
+    return SHAPE_OK;
+}
+
 int EngineImpl::evaluate(int form, shape_eval_summary *out)
 {
     int rc = launch(form);
@@ -1329,14 +1367,13 @@ int EngineImpl::evaluate(int form, shape_eval_summary *out)
 }
 
 // Enqueues one evaluation on the engine stream and returns without waiting:
-// parameters host->device, the kernel sequence (a graph replay for the
-// batched forms), the summary device->host, then event ev1.
+// the parameters, the kernel sequence, the summary (written to mapped host
+// memory), then event ev1.
 int EngineImpl::launch(int form)
 {
     if (!finalized) return set_err(SHAPE_E_STATE, "evaluate before finalize");
     if (form < 0 || form > 2) return set_err(SHAPE_E_ARG, "unknown form");
     cudaStream_t s = stream;
-    fill_params(h_params);
     fill_spin();
     std::vector<double> sc(3 * (size_t)ncomp);
     effective_scale(sc.data(), &pending_baddiam, &pending_bdl);
@@ -1346,42 +1383,31 @@ int EngineImpl::launch(int form)
     }
     if (form == SHAPE_FORM_PLAIN_FP64) {
         CK(cudaEventRecord(ev0, s));
-        CK(cudaMemcpyAsync(d_r, h_params, sizeof(double) * npar(), cudaMemcpyHostToDevice, s));
-        int rc = enqueue(form);
-        if (rc) return rc;
+        int rc = upload_params();
+        if (rc || (rc = enqueue(form)) != SHAPE_OK) return rc;
         if (!pen_type.empty() && (rc = enqueue_model_sums()) != SHAPE_OK) return rc;
         CK(cudaEventRecord(ev1, s));
     } else {
-        if (gexec[form] && graph_keep_pos[form] != keep_pos) {
-            cudaGraphExecDestroy(gexec[form]);
-            gexec[form] = nullptr;
-        }
-        if (!gexec[form]) {
-            if (!tuned[form]) {
-                if (tune_mode < 0) {
-                    int rc = autotune(form);
-                    if (rc) return rc;
-                } else {
-                    raster_variant[form] = tune_mode;
-                    raster_persistent[form] = 0;
-                    tuned[form] = 1;
-                }
+        if (!tuned[form]) {
+            if (tune_mode < 0) {
+                int rc = autotune(form);
+                if (rc) return rc;
+            } else {
+                raster_variant[form] = tune_mode;
+                raster_persistent[form] = 0;
+                tuned[form] = 1;
             }
-            // baddiam factors are baked into the summary launch: graphs are
-            // rebuilt if the flag changes (rare: a scale factor <= 0.01).
-            cudaGraph_t graph;
-            CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            cudaMemcpyAsync(d_r, h_params, sizeof(double) * npar(), cudaMemcpyHostToDevice, s);
-            int rc = enqueue(form);
-            cudaError_t ce = cudaStreamEndCapture(s, &graph);
-            if (rc) { if (ce == cudaSuccess) cudaGraphDestroy(graph); return rc; }
-            CK(ce);
-            CK(cudaGraphInstantiate(&gexec[form], graph, 0));
-            cudaGraphDestroy(graph);
-            graph_keep_pos[form] = keep_pos;
         }
+        // Straight launches, not a captured graph: the chain is four launches
+        // (a radar engine's) that need not wait for one another's launch, and
+        // the first starts sooner than a graph's first node (one frame 49.4 us
+        // between the events as a graph, 42.0 launched; 64 frames 153.5 and
+        // 149.3), and its arguments carry the trial's parameters.
         CK(cudaEventRecord(ev0, s));
-        CK(cudaGraphLaunch(gexec[form], s));
+        if (int rc = enqueue(form)) {
+            dev_params.clear();          // the launches may not have stored them
+            return rc;
+        }
         if (!pen_type.empty()) {
             int rc = enqueue_model_sums();
             if (rc) return rc;
@@ -1492,7 +1518,7 @@ void tune_file_save()
 
 // Measures the raster stage of this form with each kernel and grid (one
 // untimed and three timed eager runs each, the minimum kept) and keeps the
-// fastest. Runs outside any capture, before the form's graph is built.
+// fastest. Runs before the form's first evaluation.
 int EngineImpl::autotune(int form)
 {
     const TuneKey key{device, form, form == SHAPE_FORM_BATCHED_FP32 ? fp32_exact : 0, nviews, nf,
@@ -1510,7 +1536,7 @@ int EngineImpl::autotune(int form)
         }
     }
     cudaStream_t s = stream;
-    CK(cudaMemcpyAsync(d_r, h_params, sizeof(double) * npar(), cudaMemcpyHostToDevice, s));
+    if (int rc0 = upload_params()) return rc0;
     cudaEvent_t ev[8];
     for (auto &x : ev) CK(cudaEventCreate(&x));
     int best = 0, rc = SHAPE_OK;
@@ -2158,9 +2184,8 @@ int shape_engine_stage_times(shape_engine *h, int form, double *ms, int max)
     cudaSetDevice(E.device);
     cudaEvent_t ev[9];
     for (auto &x : ev) cudaEventCreate(&x);
-    E.fill_params(E.h_params);
     E.fill_spin();
-    cudaMemcpyAsync(E.d_r, E.h_params, sizeof(double) * E.npar(), cudaMemcpyHostToDevice, E.stream);
+    if (int rc0 = E.upload_params()) return rc0;
     cudaEventRecord(ev[0], E.stream);
     int rc = E.enqueue(form, ev + 1);
     cudaError_t ce = cudaStreamSynchronize(E.stream);
@@ -2272,11 +2297,6 @@ int shape_engine_set_fp32_exact(shape_engine *h, int exact)
 {
     if (!h || (exact != 0 && exact != 1)) return shape::set_err(SHAPE_E_ARG, "set_fp32_exact: 0 or 1");
     shape::EngineImpl &E = h->impl;
-    if (E.fp32_exact != exact && E.gexec[SHAPE_FORM_BATCHED_FP32]) {   // the captured graph has the other kernel
-        cudaSetDevice(E.device);
-        cudaGraphExecDestroy(E.gexec[SHAPE_FORM_BATCHED_FP32]);
-        E.gexec[SHAPE_FORM_BATCHED_FP32] = nullptr;
-    }
     if (E.fp32_exact != exact) E.tuned[SHAPE_FORM_BATCHED_FP32] = 0;
     E.fp32_exact = exact;
     return SHAPE_OK;
@@ -2288,7 +2308,6 @@ int shape_engine_set_spin_device(shape_engine *h, int on)
     shape::EngineImpl &E = h->impl;
     if (E.finalized) cudaSetDevice(E.device);
     if (on == E.spin_device) return SHAPE_OK;
-    E.invalidate_graphs();
     E.spin_device = on;
     if (!E.finalized) return SHAPE_OK;
     if (on) {
@@ -2436,7 +2455,6 @@ int shape_engine_set_raster_tuning(shape_engine *h, int mode)
     if (!h || mode < -1 || mode > 1) return shape::set_err(SHAPE_E_ARG, "set_raster_tuning: -1, 0 or 1");
     shape::EngineImpl &E = h->impl;
     if (E.finalized) cudaSetDevice(E.device);
-    E.invalidate_graphs();
     E.tune_mode = mode;
     for (int f = 0; f < 3; f++) E.tuned[f] = 0;
     return SHAPE_OK;

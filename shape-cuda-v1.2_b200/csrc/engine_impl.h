@@ -1,5 +1,5 @@
 // EngineImpl: host-side state of one engine (model, datasets, device
-// arenas, graphs). Shared by engine.cu (evaluation, C ABI) and server.cu
+// arenas). Shared by engine.cu (evaluation, C ABI) and server.cu
 // (continuous-batching request loop).
 #pragma once
 
@@ -82,11 +82,6 @@ struct EngineImpl {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // side branch of the batched graph (state reset, image clears, vertex
-    // normals) and its fork / join events
-    cudaStream_t stream2 = nullptr;   // batched graph branches: state reset and clears
-    cudaStream_t stream3 = nullptr;   // ... and realize (vertices, facet and vertex normals)
-    cudaEvent_t evf[4] = {nullptr, nullptr, nullptr, nullptr};
     float last_ms = 0.f;
 
     // model (host)
@@ -210,18 +205,13 @@ struct EngineImpl {
     double *h_params = nullptr;             // r[nv], scale[3]
     shape_eval_summary *h_summary = nullptr;
 
-    // graphs per form
-    cudaGraphExec_t gexec[3] = {nullptr, nullptr, nullptr};
     int keep_pos = 0;
-    int graph_keep_pos[3] = {0, 0, 0};
     int last_form = -1;
 
     ~EngineImpl() { release(); }
 
     void release()
     {
-        for (auto &g : gexec)
-            if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         mem.release();
         if (h_params) { cudaFreeHost(h_params); h_params = nullptr; }
         if (h_summary) { cudaFreeHost(h_summary); h_summary = nullptr; }
@@ -230,17 +220,7 @@ struct EngineImpl {
         if (h_spin_off) { cudaFreeHost(h_spin_off); h_spin_off = nullptr; }
         if (ev0) { cudaEventDestroy(ev0); ev0 = nullptr; }
         if (ev1) { cudaEventDestroy(ev1); ev1 = nullptr; }
-        for (auto &e : evf)
-            if (e) { cudaEventDestroy(e); e = nullptr; }
-        if (stream2) { cudaStreamDestroy(stream2); stream2 = nullptr; }
-        if (stream3) { cudaStreamDestroy(stream3); stream3 = nullptr; }
         if (stream) { cudaStreamDestroy(stream); stream = nullptr; }
-    }
-
-    void invalidate_graphs()
-    {
-        for (auto &g : gexec)
-            if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     }
 
     int finalize();
@@ -259,7 +239,7 @@ struct EngineImpl {
     int realize_views();
     int refresh_views();
     // spin realization inside each evaluation (principal-axis rotators):
-    // the graph copies the spin state and offsets from pinned memory and
+    // it copies the spin state and offsets from pinned memory and
     // k_realize_views rebuilds every view from them
     int spin_device = 0;
     int n_spin_src = 0;
@@ -272,6 +252,10 @@ struct EngineImpl {
     int setup_spin_device();
     void fill_spin();
     int enqueue_spin();
+    // the parameters that the device arrays hold (empty: unknown)
+    std::vector<double> dev_params;
+    int upload_params();
+    int front_params(FrontArgs &fr);
     int enqueue(int form, cudaEvent_t *marks = nullptr);
     int launch(int form);
     int poll();

@@ -11,11 +11,14 @@ namespace shape {
 
 // Programmatic dependent launch (batched forms): a kernel launched with
 // launch_k(..., pdl = true) may be scheduled before the previous kernel on
-// its stream has finished, and waits here, before its first access to that
-// kernel's outputs, until it has (a no-op after an ordinary launch). The
-// previous kernel does not trigger early, so waiting blocks take no SM
-// slots from it; what is saved is the launch latency between the two.
+// its stream has finished, and waits in grid_dep_wait, before its first access
+// to that kernel's outputs, until it has (a no-op after an ordinary launch).
+// grid_dep_trigger at a kernel's start lets the next one's blocks become
+// resident once every block of this one has started, so they take no slots
+// from it and the launch latency between the two is hidden. Kernel k + 2 needs
+// no trigger of kernel k's: kernel k + 1 finishes only after its own wait.
 #ifdef __CUDACC__
+__device__ __forceinline__ void grid_dep_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
 
@@ -125,19 +128,51 @@ void launch_reset_state(FrameState *st, int nviews, int *bin_count, int ntiles, 
 // pdl: programmatic dependent launch (launch_k)
 void launch_xform_f64(const FrameGeom *g, int nviews, const double4 *vx, int nv, double4 *vt,
                       cudaStream_t s, bool pdl = false);
-// the transform of vertices realized on the fly (no dependency on k_realize_vf)
-void launch_xform_realize_f64(const FrameGeom *g, int nviews, const ModelDev &m, double4 *vt, cudaStream_t s);
+// the first launch of a batched evaluation (k_front)
+struct FrontArgs {
+    static constexpr int CLEARS = 6;
+    const FrameGeom *geoms;
+    int nviews;
+    ModelDev m;
+    double4 *vt;
+    FrameState *states;
+    // parameter changes since the device arrays were last written: the scale
+    // factors (of up to SCALES / 3 components) and up to CHANGES deviations
+    // travel with the launch, which also stores them, instead of a copy of all
+    // of them ahead of it (5 us before the first kernel could start)
+    static constexpr int SCALES = 24, CHANGES = 8;
+    double scale[SCALES];
+    int nscale;                        // 0: the arrays hold the parameters
+    int nchange, change_at[CHANGES];
+    double change_to[CHANGES];
+    double *r_out, *scale_out;
+    unsigned char *clear[CLEARS];      // arrays to clear (16-byte aligned) and their bytes
+    size_t clear_bytes[CLEARS];
+    int nb_xform, nb_model;            // blocks of the first two ranges (set by launch_front)
+};
+void launch_front(const FrontArgs &a, cudaStream_t s);
+// the vertex normals as extra blocks of k_bin (nv 0: none)
+struct VnormalArgs {
+    int nv;
+    const int *af_ptr, *af_idx;
+    double4 *vn;
+    float4 *vnf;
+};
 void launch_bin_f64(const FrameGeom *g, int view0, int nviews, const ModelDev &m, const double4 *vt,
-                    FrameState *st, int *bin_count, int2 *bin_ids, int cap, cudaStream_t s, bool pdl = false);
+                    FrameState *st, int *bin_count, int2 *bin_ids, int cap, cudaStream_t s, bool pdl = false,
+                    bool vnormals = false);
 
-struct Chi2Item { int frame; int start; int count; };
+// One chi-square item: count bins of a frame's image from element base of the
+// image arrays, lying in rows row0..row1 (1-based); view: the frame's view,
+// whose delay limits tell which rows hold footprints (-1: a smeared frame,
+// whose other views reach other rows).
+struct Chi2Item { int frame, count, row0, row1, view, pad; long long base; };
 struct Chi2Args {
     const Chi2Item *items;
     int nitems;
     const double *obs, *oov;
     const void *fit;             // double or float
-    const FrameGeom *geoms;      // radar views (for fit_base)
-    const int *frame_view;       // global deldop frame -> view index
+    const FrameState *states;
     double *partials;            // [nitems * 6]: o2, m2, om + compensations
     // [nitems * 2]: each item's o2 partial (sum and compensation), computed
     // once per dataset by the same code; null: o2 is summed per launch
@@ -190,8 +225,8 @@ struct DopOvfArgs {
 // FP32 form: the Doppler frames' FP64 sums rounded into the float fit
 // images the chi-square reads (one block per Doppler frame).
 void launch_dop_fit_f32(const int *dop_frames, int n, const FrameHost *fh, const FrameGeom *geoms,
-                        const double *fit64, float *fit32, cudaStream_t s);
-void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s);
+                        const double *fit64, float *fit32, cudaStream_t s, bool pdl);
+void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s, bool pdl);
 
 struct LcArgs {
     int npoints;
@@ -211,7 +246,7 @@ struct LcArgs {
     double mincosine_seen;
     int mark_seen;
 };
-void launch_lc_photo(const LcArgs &a, int fp32, cudaStream_t s);
+void launch_lc_photo(const LcArgs &a, cudaStream_t s, bool pdl);
 
 struct LcSetDev {
     int npts, n;                // calc points, observed points
@@ -236,7 +271,7 @@ struct LcFinalizeArgs {
 constexpr size_t LC_FINALIZE_SMEM_MAX = 160 * 1024;
 size_t lc_finalize_smem(int npts, int n);
 cudaError_t configure_lc_finalize();
-void launch_lc_finalize(const LcFinalizeArgs &a, cudaStream_t s);
+void launch_lc_finalize(const LcFinalizeArgs &a, cudaStream_t s, bool pdl);
 
 // Spin realization inside an evaluation (spin.cu; principal-axis
 // rotators): one thread per radar frame (its epoch view) or lightcurve point
@@ -281,7 +316,7 @@ struct PosetArgs {
     double *fit;                // fit images
     shape_poset_result *res;    // per-frame results
 };
-void launch_poset_frames(const PosetArgs &a, cudaStream_t s);
+void launch_poset_frames(const PosetArgs &a, cudaStream_t s, bool pdl);
 struct SummaryArgs {
     int nsets;
     const SetRec *sets;
@@ -306,7 +341,7 @@ constexpr size_t SUMMARY_SMEM_MAX = 160 * 1024;
 size_t summary_smem(int nframes, int nitems, int *with_partials);
 cudaError_t configure_summary();
 // per-frame finalize (as launch_finalize_frames) fused with the totals
-void launch_summary(const FinalizeArgs &fa, const SummaryArgs &a, cudaStream_t s);
+void launch_summary(const FinalizeArgs &fa, const SummaryArgs &a, cudaStream_t s, bool pdl);
 
 // Chi-square partials + per-frame finalize + totals in one launch (the
 // batched forms). Its shared staging (chi2_summary_smem bytes of dynamic

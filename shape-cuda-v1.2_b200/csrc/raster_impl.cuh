@@ -813,6 +813,7 @@ template <typename T, int NT, bool MAPS>
 __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? RASTER_WARPS_F32 : RASTER_WARPS_F64) * 32 / NT)
 k_raster(const __grid_constant__ RasterArgs a)
 {
+    grid_dep_trigger();
     grid_dep_wait();
     constexpr int PP = TILE_PIX / NT;          // pixels per thread
     __shared__ TileShared<T, NT> sh;
