@@ -641,94 +641,6 @@ __global__ void k_doppler_overflow(DopOvfArgs a)
 
 // ------------------------------------------------------------ lightcurves
 
-// posmask (src/shape/posmask.c:58-174) and apply_photo
-// (src/shape/apply_photo.c:85-133, 226-248) per POS pixel of one
-// lightcurve point; brightness summed per work item (fixed order within a
-// block, items summed in order by k_lc_finalize).
-template <typename T>
-__global__ void k_lc_photo(LcArgs a)
-{
-    grid_dep_trigger();
-    grid_dep_wait();
-    __shared__ double red[32];
-    for (int it = blockIdx.x; it < a.nitems; it += gridDim.x) {
-        int2 item = a.items[it];
-        const LcPointDev &P = a.pts[item.x];
-        const FrameGeom &go = a.geoms[P.obs_view];
-        const FrameGeom &gs = a.geoms[P.sun_view];
-        const int n = go.n, side = go.side;
-        const long long npix = (long long)side * side;
-        const double *Z = a.z + go.pos_base;
-        T *CE = static_cast<T *>(a.cose) + go.pos_base;
-        const T *CI = static_cast<const T *>(a.cosi) + go.pos_base;
-        const double *ZI = a.zill + gs.pos_base;
-        const int *F = a.f + go.pos_base;
-        const int *FI = a.fill + gs.pos_base;
-        const double bignum = 0.99 * HUGENUMBER;
-        // a plane-of-sky frame keeps its brightness image (pos->b of
-        // apply_photo, zero where nothing is lit)
-        double *Bimg = (a.bimg && P.b_base >= 0) ? a.bimg + P.b_base : nullptr;
-        double bsum = 0.0;
-        long long pend = (long long)item.y + a.chunk;
-        if (pend > npix) pend = npix;
-        for (long long p = item.y + threadIdx.x; p < pend; p += blockDim.x) {
-            double cose = (double)CE[p];
-            if (cose == 0.0) {
-                if (Bimg) Bimg[p] = 0.0;
-                continue;
-            }
-            int i = (int)(p / side) - n, j = (int)(p % side) - n;
-            double xin[3] = {i * go.kmpp, j * go.kmpp, (double)Z[p]};
-            double x[3];
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                x[r] = 0.0;
-                x[r] += P.so[3 * r + 0] * xin[0];
-                x[r] += P.so[3 * r + 1] * xin[1];
-                x[r] += P.so[3 * r + 2] * xin[2];
-            }
-            double i0 = x[0] * P.pixels_per_km, j0 = x[1] * P.pixels_per_km;
-            int im = iround_(i0), jm = iround_(j0);
-#define ZILL(a_, b_) ((double)ZI[(long long)((a_) + n) * side + ((b_) + n)])
-            if (fabs(i0) < n && fabs(j0) < n && ZILL(im, jm) > -bignum &&
-                F[p] != FI[(long long)(im + n) * side + (jm + n)]) {
-                if (posmask_zill(ZI, n, side, i0, j0, im, jm) - x[2] > P.mask_tol) {
-                    cose = 0.0;
-                    CE[p] = (T)0;
-                }
-            }
-#undef ZILL
-            double cosi = (double)CI[p];
-            int f = F[p];
-            if (a.mark_seen && cose > a.mincosine_seen && cosi > a.mincosine_seen && f >= 0)
-                a.seen[f] = 1;
-            double bv = 0.0;
-            if (cose > 0.0 && cosi > 0.0 && f >= 0) {
-                double b;
-                if (P.law_type == SHAPE_OPTLAW_LAMBERT)
-                    b = P.intensityfactor * P.scale * cosi;
-                else if (P.law_type == SHAPE_OPTLAW_LOMMEL)
-                    b = P.intensityfactor * P.scale * cosi / (cosi + cose);
-                else
-                    b = P.intensityfactor * cosi * (P.s_ls / (cosi + cose) + P.s_l);
-                bsum += b;
-                bv = b;
-            }
-            if (Bimg) Bimg[p] = bv;
-        }
-        for (int off = 16; off > 0; off >>= 1)
-            bsum += __shfl_down_sync(0xffffffffu, bsum, off);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = bsum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w];
-            a.partials[it] = s;
-        }
-        __syncthreads();
-    }
-}
-
 // A radar frame's badradar term of the objective (src/shape/calc_fits.c:
 // 545-550): dof * log-factor / views, summed over the views whose
 // footprint was too wide; the flag when any of them was. One view: the
@@ -812,19 +724,22 @@ __device__ double poset_sample(const double *B, int n, int side, int mode, doubl
 #undef IM
 }
 
-// One block per plane-of-sky frame: the fit image by resampim (with
-// rebinning when the grid undersamples the rendering by an integer factor
+// gridDim.x blocks per plane-of-sky frame (blockIdx.y), each a slice of its fit
+// grid and of its sky pixels: the fit image by resampim (with rebinning when the grid undersamples the rendering by an integer factor
 // and image_rebin is set; cubic convolution clipped at 0), checkposet's
 // test of the lit pixels' corners against the rotated fit grid
 // (src/util/checkposet.c), chi2_poset's sums with the floating
-// calibration (src/shape/chi2.c) and the views' posbnd terms.
-__global__ void k_poset_frames(PosetArgs a)
+// calibration (src/shape/chi2.c) and the views' posbnd terms. The block that
+// finishes a frame last merges the blocks' sums in block order. One block per
+// frame left the chip idle: the stage of three frames of 181^2 pixels took
+// 120 us, with 17 blocks a frame 27.
+__global__ void __launch_bounds__(256) k_poset_frames(PosetArgs a)
 {
     grid_dep_trigger();
     grid_dep_wait();
     __shared__ double red[5][32];
     __shared__ int redi[32];
-    const PosetFrameDev F = a.frames[blockIdx.x];
+    const PosetFrameDev F = a.frames[blockIdx.y];
     const LcPointDev &P = a.pts[F.point];
     const FrameGeom &go = a.geoms[P.obs_view], &gs = a.geoms[P.sun_view];
     const int n = go.n, side = go.side;
@@ -848,7 +763,8 @@ __global__ void k_poset_frames(PosetArgs a)
     const double x1s = F.x0 - ((xt2 - 1) / 2.0) * dxx - ((yt2 - 1) / 2.0) * dxy;
     const double y1s = F.y0 - ((xt2 - 1) / 2.0) * dyx - ((yt2 - 1) / 2.0) * dyy;
     double o2 = 0.0, m2 = 0.0, om = 0.0;
-    for (int p = threadIdx.x; p < ncol * nrow; p += blockDim.x) {
+    const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (int p = t0; p < ncol * nrow; p += step) {
         const int i = p / nrow + 1, j = p % nrow + 1;
         double v;
         if (rebin) {
@@ -873,7 +789,7 @@ __global__ void k_poset_frames(PosetArgs a)
     double xmin = xl1, xmax = xl2, ymin = yl1, ymax = yl2;
     int bad = 0;
     const int cside = side + 1;
-    for (int c = threadIdx.x; c < cside * cside; c += blockDim.x) {
+    for (int c = t0; c < cside * cside; c += step) {
         const int ci = c / cside - n, cj = c % cside - n;      // corner (ci, cj): ci, cj = -n..n+1
         bool lit = false;
         for (int di = -1; di <= 0 && !lit; di++)
@@ -910,13 +826,35 @@ __global__ void k_poset_frames(PosetArgs a)
         redi[wid] = bad;
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
+    double *part = a.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * POSET_PART;
+    __shared__ int s_last;
+    if (threadIdx.x == 0) {
+        o2 = m2 = om = 0.0;
+        for (int w = 0; w < nw; w++) {
+            o2 += red[0][w]; m2 += red[1][w]; om += red[2][w];
+            xmin = fmin(xmin, ext[0][w]); xmax = fmax(xmax, ext[1][w]);
+            ymin = fmin(ymin, ext[2][w]); ymax = fmax(ymax, ext[3][w]);
+            bad |= redi[w];
+        }
+        part[0] = o2; part[1] = m2; part[2] = om;
+        part[3] = xmin; part[4] = xmax; part[5] = ymin; part[6] = ymax;
+        part[7] = bad;
+        __threadfence();                                      // the partials before the count
+        s_last = (atomicAdd(&a.counters[blockIdx.y], 1) == (int)gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!s_last || threadIdx.x != 0) return;
+    __threadfence();
     o2 = m2 = om = 0.0;
-    for (int w = 0; w < nw; w++) {
-        o2 += red[0][w]; m2 += red[1][w]; om += red[2][w];
-        xmin = fmin(xmin, ext[0][w]); xmax = fmax(xmax, ext[1][w]);
-        ymin = fmin(ymin, ext[2][w]); ymax = fmax(ymax, ext[3][w]);
-        bad |= redi[w];
+    bad = 0;
+    const double *all = a.part + (size_t)blockIdx.y * gridDim.x * POSET_PART;
+#pragma unroll 4
+    for (int b = 0; b < (int)gridDim.x; b++) {
+        const double *q = all + (size_t)b * POSET_PART;
+        o2 += __ldcg(q); m2 += __ldcg(q + 1); om += __ldcg(q + 2);
+        xmin = fmin(xmin, __ldcg(q + 3)); xmax = fmax(xmax, __ldcg(q + 4));
+        ymin = fmin(ymin, __ldcg(q + 5)); ymax = fmax(ymax, __ldcg(q + 6));
+        bad |= __ldcg(q + 7) != 0.0;
     }
     shape_poset_result r;
     r.o2 = o2; r.m2 = m2; r.om = om;
@@ -929,7 +867,7 @@ __global__ void k_poset_frames(PosetArgs a)
     r.posbnd_logsum = 0.0;
     if (so.outbnd) r.posbnd_logsum += 0.5 * F.dof * view_logfactor(go, so);
     if (ss.outbnd) r.posbnd_logsum += 0.5 * F.dof * view_logfactor(gs, ss);
-    a.res[blockIdx.x] = r;
+    a.res[blockIdx.y] = r;
 }
 
 // Natural cubic spline second derivatives and evaluation (the role of
@@ -937,25 +875,19 @@ __global__ void k_poset_frames(PosetArgs a)
 //   h[i-1] y2[i-1] + 2 (h[i-1] + h[i]) y2[i] + h[i] y2[i+1]
 //     = 6 ((y[i+1]-y[i])/h[i] - (y[i]-y[i-1])/h[i-1]),   y2[0] = y2[n-1] = 0,
 // is solved with each row divided by its span x[i+1] - x[i-1] (lower
-// coefficient w = h[i-1]/span, diagonal 2, upper 1 - w): forward
-// elimination keeps each row's multiplier of y2[i+1] in y2[i] and its
-// eliminated right-hand side in r[i], back substitution forms
-// y2[i] = y2[i] y2[i+1] + r[i]. The reference solves the span-scaled rows in
-// this order, so the FP64 fits are bit-identical to its.
-__device__ void spline_natural_dev(const double *x, const double *y, int n, double *y2, double *r)
+// coefficient w = h[i-1]/span, diagonal 2, upper 1 - w): forward elimination
+// keeps each row's multiplier of y2[i+1] in y2[i] and its eliminated right-hand
+// side, back substitution forms y2[i] = mult[i] y2[i+1] + r[i]. The reference
+// solves the span-scaled rows in this order, so the FP64 fits are bit-identical
+// to its. Multipliers and pivots depend on the epochs only and come from the
+// host (spline_plan); what remains serial is r[i] = (rhs[i] - w r[i-1]) / piv
+// and the back substitution. The quotient is Markstein's: q = RN(a RN(1/b)),
+// then q + RN(1/b) (a - q b) with the residual exact in a fused multiply-add,
+// which is RN(a / b); three dependent operations instead of a division's ten.
+__device__ inline double div_by(double a, double b, double rb)
 {
-    if (n < 1) return;
-    y2[0] = r[0] = 0.0;
-    for (int i = 1; i < n - 1; i++) {
-        const double span = x[i + 1] - x[i - 1];
-        const double w = (x[i] - x[i - 1]) / span;
-        const double piv = w * y2[i - 1] + 2.0;
-        y2[i] = (w - 1.0) / piv;
-        const double dslope = (y[i + 1] - y[i]) / (x[i + 1] - x[i]) - (y[i] - y[i - 1]) / (x[i] - x[i - 1]);
-        r[i] = (6.0 * dslope / span - w * r[i - 1]) / piv;
-    }
-    if (n > 1) y2[n - 1] = 0.0;
-    for (int i = n - 2; i >= 0; i--) y2[i] = y2[i] * y2[i + 1] + r[i];
+    const double q = a * rb;
+    return fma(rb, fma(-q, b, a), q);
 }
 
 __device__ double splint_dev(const double *x, const double *y, const double *y2, int n, double t)
@@ -971,95 +903,110 @@ __device__ double splint_dev(const double *x, const double *y, const double *y2,
            ((wl * wl * wl - wl) * y2[lo] + (wh * wh * wh - wh) * y2[hi]) * (h * h) / 6.0;
 }
 
-// One block per lightcurve set: y from brightness partials, spline to the
+// One block per lightcurve set: y from the tiles' brightness, spline to the
 // observation epochs, chi2_lghtcrv (src/shape/chi2.c:1125-1170), posbnd sum
 // (src/shape/calc_fits.c:1651-1679, 1947).
 //
-// The recurrences (spline elimination, the chi-square sums, the log-factor
-// sum) stay serial in the reference's order, so results are bit-identical to
-// it; when a.smem_per_set > 0 their operands are first gathered into shared
-// memory by the whole block, so the serial loops run at shared-memory latency
-// instead of one global round trip per step.
-__global__ void k_lc_finalize(LcFinalizeArgs a)
+// The recurrences (spline elimination and back substitution, the chi-square
+// sums, the log-factor sum) stay serial in the reference's order, so results
+// are bit-identical to it; everything else, their operands included, is formed
+// by the whole block first (in shared memory when a.smem_per_set > 0, else in
+// the set's scratch). What bounds it is their latency: with each step's slopes,
+// pivot and division inside the recurrence, the finalize and summary stage of
+// four sets of 200 points took 128 us; it takes 55.
+__global__ void __launch_bounds__(1024) k_lc_finalize(LcFinalizeArgs a)
 {
     grid_dep_trigger();
     grid_dep_wait();
     extern __shared__ double lsm[];
     const LcSetDev &S = a.sets[blockIdx.x];
     const int np = S.npts, n = S.n;
-    const bool use_sm = a.smem_per_set > 0;
-    // shared layout: x y y2 cp [np] | t obs oov fit [n] | lo ls [np] (doubles), flags [np] (int)
-    double *x = use_sm ? lsm : const_cast<double *>(S.x);
-    double *y = use_sm ? lsm + np : S.y;
-    double *y2 = use_sm ? lsm + 2 * np : S.y2;
-    double *cp = use_sm ? lsm + 3 * np : S.fit + n;       // global path: fit tail is scratch
-    double *tt = use_sm ? lsm + 4 * np : const_cast<double *>(S.t);
-    double *obs = use_sm ? tt + n : const_cast<double *>(S.obs);
-    double *oov = use_sm ? tt + 2 * n : const_cast<double *>(S.oov);
-    double *fit = use_sm ? tt + 3 * n : S.fit;
-    double *lo = tt + 4 * n, *ls = lo + np;
-    int *pflag = reinterpret_cast<int *>(ls + np);
-    for (int k = threadIdx.x; k < np; k += blockDim.x) {
-        int pt = S.pt0 + k;
-        int it0 = a.pt_items[2 * pt], cnt = a.pt_items[2 * pt + 1];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    // work arrays: y, y2, r, lower coefficients, pivots and their reciprocals
+    // [np]; the chi-square terms [2 n]
+    double *y = a.smem_per_set > 0 ? lsm : S.scratch, *y2 = y + np, *r = y2 + np, *ll = r + np, *pv = ll + np,
+           *rpv = pv + np, *m2t = rpv + np, *omt = m2t + n;
+    const double *w = S.spl, *piv = w + np, *rpiv = piv + np, *mult = rpiv + np, *span = mult + np;
+    __shared__ int s_bnd;
+    if (tid == 0) s_bnd = 0;
+    __syncthreads();
+    // a warp per point: its observer view's tiles in a fixed order
+    for (int k = wid; k < np; k += nw) {
+        const LcPointDev &P = a.pts[S.pt0 + k];
+        const FrameGeom &go = a.geoms[P.obs_view];
+        const double *part = a.tile_part + go.tile_base;
+        const int nt = go.tiles_x * go.tiles_x;
         double sum = 0.0;
-        for (int it = it0; it < it0 + cnt; it++) sum += a.partials[it];
-        sum = (sum == 0.0) ? 1.0e-40 : sum;
-        y[k] = sum;
-        if (use_sm) {
-            S.y[k] = sum;
-            x[k] = S.x[k];
-            // per-point posbnd log-factor terms, summed serially below
-            const LcPointDev &P = a.pts[pt];
+        for (int t = lane; t < nt; t += 32) sum += part[t];
+        for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
+        if (lane == 0) {
+            sum = (sum == 0.0) ? 1.0e-40 : sum;
+            y[k] = S.y[k] = sum;
             const FrameState &so = a.states[P.obs_view], &ss = a.states[P.sun_view];
-            lo[k] = so.outbnd ? 0.5 * view_logfactor(a.geoms[P.obs_view], so) : 0.0;
-            ls[k] = ss.outbnd ? 0.5 * view_logfactor(a.geoms[P.sun_view], ss) : 0.0;
-            pflag[k] = (so.outbnd ? 1 : 0) | (ss.outbnd ? 2 : 0);
+            // a point's two posbnd terms are added one after the other
+            double l0 = 0.0, l1 = 0.0;
+            if (so.outbnd) { s_bnd = 1; l0 = 0.5 * view_logfactor(go, so); }
+            if (ss.outbnd) { s_bnd = 1; l1 = 0.5 * view_logfactor(a.geoms[P.sun_view], ss); }
+            ll[k] = l0;
+            y2[k] = l1;
         }
     }
-    if (use_sm)
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            tt[k] = S.t[k];
-            obs[k] = S.obs[k];
-            oov[k] = S.oov[k];
-        }
     __syncthreads();
-    if (threadIdx.x == 0) spline_natural_dev(x, y, np, y2, cp);
+    double lsum = 0.0;
+    if (tid == 0 && s_bnd)
+        for (int k = 0; k < np; k++) { lsum += ll[k]; lsum += y2[k]; }
     __syncthreads();
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        double v = splint_dev(x, y, y2, np, tt[k]) / 1;
-        fit[k] = v;
-        if (use_sm) S.fit[k] = v;
+    for (int i = 1 + tid; i < np - 1; i += blockDim.x) {
+        const double dslope = (y[i + 1] - y[i]) / (S.x[i + 1] - S.x[i]) - (y[i] - y[i - 1]) / (S.x[i] - S.x[i - 1]);
+        r[i] = 6.0 * dslope / span[i];
+        y2[i] = mult[i];
+        ll[i] = w[i];
+        pv[i] = piv[i];
+        rpv[i] = rpiv[i];
     }
-    if (use_sm)
-        for (int k = threadIdx.x; k < np; k += blockDim.x) S.y2[k] = y2[k];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double o2 = 0.0, m2 = 0.0, om = 0.0;
+    if (tid == 0) {
+        double rp = 0.0;
+        r[0] = 0.0;
+#pragma unroll 4
+        for (int i = 1; i < np - 1; i++) {
+            rp = div_by(r[i] - ll[i] * rp, pv[i], rpv[i]);
+            r[i] = rp;
+        }
+        double yn = 0.0;
+        y2[np - 1] = 0.0;
+#pragma unroll 4
+        for (int i = np - 2; i > 0; i--) {
+            yn = y2[i] * yn + r[i];
+            y2[i] = yn;
+        }
+        y2[0] = 0.0;
+    }
+    __syncthreads();
+    for (int k = tid; k < n; k += blockDim.x) {
+        const double v = splint_dev(S.x, y, y2, np, S.t[k]) / 1;
+        S.fit[k] = v;
+        m2t[k] = v * v * S.oov[k];
+        omt[k] = v * S.obs[k] * S.oov[k];
+    }
+    for (int k = tid; k < np; k += blockDim.x) S.y2[k] = y2[k];
+    __syncthreads();
+    if (tid == 0) {
+        double m2 = 0.0, om = 0.0;
+#pragma unroll 8
         for (int k = 0; k < n; k++) {
-            o2 += obs[k] * obs[k] * oov[k];
-            m2 += fit[k] * fit[k] * oov[k];
-            om += fit[k] * obs[k] * oov[k];
+            m2 += m2t[k];
+            om += omt[k];
         }
+        const double o2 = S.o2;
         double cal = S.cal_in;
         if (S.cal_floating)
             cal = (om > 0.0) ? om / m2 : SHAPE_TINYCALFACT;
-        double chi2 = S.weight * (o2 - 2 * cal * om + cal * cal * m2);
-        int posbnd = 0;
-        double lsum = 0.0;
-        for (int k = 0; k < np; k++) {
-            if (use_sm) {
-                if (pflag[k] & 1) { posbnd = 1; lsum += lo[k]; }
-                if (pflag[k] & 2) { posbnd = 1; lsum += ls[k]; }
-            } else {
-                const LcPointDev &P = a.pts[S.pt0 + k];
-                const FrameState &so = a.states[P.obs_view], &ss = a.states[P.sun_view];
-                if (so.outbnd) { posbnd = 1; lsum += 0.5 * view_logfactor(a.geoms[P.obs_view], so); }
-                if (ss.outbnd) { posbnd = 1; lsum += 0.5 * view_logfactor(a.geoms[P.sun_view], ss); }
-            }
-        }
         double *o = a.set_out + 4 * blockIdx.x;
-        o[0] = cal; o[1] = chi2; o[2] = posbnd; o[3] = lsum;
+        o[0] = cal;
+        o[1] = S.weight * (o2 - 2 * cal * om + cal * cal * m2);
+        o[2] = s_bnd;
+        o[3] = lsum;
     }
 }
 
@@ -1424,21 +1371,15 @@ void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s, bool pdl)
 void launch_poset_frames(const PosetArgs &a, cudaStream_t s, bool pdl)
 {
     if (a.nframes <= 0) return;
-    launch_k(k_poset_frames, dim3(a.nframes), dim3(256), 0, s, pdl, a);
-}
-
-void launch_lc_photo(const LcArgs &a, cudaStream_t s, bool pdl)
-{
-    int blocks = a.nitems < 8 * 148 ? a.nitems : 8 * 148;
-    if (blocks <= 0) return;
-    launch_k(k_lc_photo<double>, dim3(blocks), dim3(256), 0, s, pdl, a);
+    launch_k(k_poset_frames, dim3(a.blocks, a.nframes), dim3(256), 0, s, pdl, a);
 }
 
 // Shared memory one set needs (0 when it exceeds the block's budget: the
 // kernel then works on the global arrays).
+size_t lc_finalize_words(int npts, int n) { return 6 * (size_t)npts + 2 * (size_t)n; }
 size_t lc_finalize_smem(int npts, int n)
 {
-    size_t b = sizeof(double) * (6 * (size_t)npts + 4 * (size_t)n) + sizeof(int) * (size_t)npts;
+    size_t b = sizeof(double) * lc_finalize_words(npts, n);
     return b <= LC_FINALIZE_SMEM_MAX ? b : 0;
 }
 
@@ -1451,7 +1392,7 @@ cudaError_t configure_lc_finalize()
 void launch_lc_finalize(const LcFinalizeArgs &a, cudaStream_t s, bool pdl)
 {
     if (a.nsets <= 0) return;
-    launch_k(k_lc_finalize, dim3(a.nsets), dim3(256), a.smem_per_set, s, pdl, a);
+    launch_k(k_lc_finalize, dim3(a.nsets), dim3(1024), a.smem_per_set, s, pdl, a);
 }
 
 // Shared memory of the summary: per-frame terms, then (when they fit) the

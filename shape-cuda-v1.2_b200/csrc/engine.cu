@@ -82,6 +82,22 @@ void radar_set_consts(FrameGeom &g, const shape_deldop_set &S, const shape_eval_
     g.law = law;
 }
 
+// The natural spline's elimination over the epochs x[0..n) (k_lc_finalize), in
+// the reference's operations: w, pivots, their reciprocals, the multipliers of
+// y2[i+1] in y2[i], the spans.
+static void spline_plan(const double *x, int n, double *out)
+{
+    double *w = out, *piv = w + n, *rpiv = piv + n, *mult = rpiv + n, *span = mult + n;
+    for (int i = 0; i < n; i++) { w[i] = mult[i] = 0.0; piv[i] = rpiv[i] = span[i] = 1.0; }
+    for (int i = 1; i < n - 1; i++) {
+        span[i] = x[i + 1] - x[i - 1];
+        w[i] = (x[i] - x[i - 1]) / span[i];
+        piv[i] = w[i] * mult[i - 1] + 2.0;
+        rpiv[i] = 1.0 / piv[i];
+        mult[i] = (w[i] - 1.0) / piv[i];
+    }
+}
+
 int EngineImpl::finalize()
 {
     if (!have_model) return set_err(SHAPE_E_STATE, "finalize: no model set");
@@ -95,7 +111,7 @@ int EngineImpl::finalize()
     cap = fixed_cap > 0 ? fixed_cap : 512;
     geoms.clear(); fh.clear(); work.clear(); view_work0.clear(); view_nwork.clear();
     chi2_items.clear(); frame_view.clear(); dop_extra.clear(); set_delpp.clear(); set_doppp.clear();
-    lcpts.clear(); lc_items.clear(); pt_items.clear(); lcdev.clear(); dop_frames.clear();
+    lcpts.clear(); lcdev.clear(); dop_frames.clear();
 
     const int nframes = (int)frames.size();
     const int npts = (int)points.size();
@@ -211,7 +227,6 @@ int EngineImpl::finalize()
     // lightcurve points: two views each (src/shape/calc_fits.c:1634-1716);
     // a plane-of-sky frame is rendered the same way (calc_poset,
     // src/shape/calc_fits.c:1205-1266) and keeps its brightness image
-    const int LC_CHUNK = 4096;
     auto add_point = [&](const shape_lghtcrv_point &P, const shape_optical_law &law, int set, long long b_base) {
         LcPointDev pd;
         memset(&pd, 0, sizeof pd);
@@ -245,13 +260,6 @@ int EngineImpl::finalize()
         pd.mask_tol = params.mask_tol;
         pd.pixels_per_km = 1 / P.km_per_pixel;
         pd.b_base = b_base;
-        int side = 2 * P.pos_n + 1;
-        long long np = (long long)side * side;
-        pt_items.push_back((int)lc_items.size());
-        int cnt = 0;
-        for (long long p0 = 0; p0 < np; p0 += LC_CHUNK, cnt++)
-            lc_items.push_back(make_int2((int)lcpts.size(), (int)p0));
-        pt_items.push_back(cnt);
         lcpts.push_back(pd);
     };
     for (size_t s = 0; s < lc.size(); s++) {
@@ -264,13 +272,12 @@ int EngineImpl::finalize()
         L.npts = lc[s].npts;
         L.n = S.n;
         L.pt0 = lc[s].pt0;
-        L.item0 = (int)lc_items.size();
         L.weight = S.weight;
         L.dof = S.dof;
         L.cal_in = S.cal;
         L.cal_floating = S.cal_floating;
+        for (int k = 0; k < S.n; k++) L.o2 += lc[s].obs[k] * lc[s].obs[k] * lc[s].oov[k];
         for (int k = 0; k < lc[s].npts; k++) add_point(points[lc[s].pt0 + k], S.law, (int)s, -1);
-        L.nitems = (int)lc_items.size() - L.item0;
         lcdev.push_back(L);
     }
     // plane-of-sky frames after every lightcurve point: their views'
@@ -354,14 +361,24 @@ int EngineImpl::finalize()
     AL(d_chi2_counters, fh.size() + 1);
     AL(d_fh, fh.size()); AL(d_results, fh.size());
     AL(d_set_delpp, set_delpp.size()); AL(d_set_doppp, set_doppp.size()); AL(d_dop_extra, dop_extra.size());
-    AL(d_lcpts, lcpts.size()); AL(d_lc_items, lc_items.size()); AL(d_pt_items, pt_items.size());
-    AL(d_lc_partials, lc_items.size());
+    AL(d_lcpts, lcpts.size());
+    AL(d_lc_part, lcpts.empty() ? 0 : (size_t)ntiles);
     AL(d_lcsets, lcdev.size()); AL(d_lc_out, 4 * lcdev.size());
     AL(d_lc_dof, lcdev.size()); AL(d_lc_npts, lcdev.size());
     AL(d_setrecs, setrecs.size());
     AL(d_psf, psf.size()); AL(d_ps_res, psf.size());
     AL(d_ps_obs, (size_t)ps_img_elems); AL(d_ps_oov, (size_t)ps_img_elems); AL(d_ps_fit, (size_t)ps_img_elems);
     AL(d_ps_b, (size_t)ps_b_elems);
+    // blocks per plane-of-sky frame: a fit sample or eight sky corners a
+    // thread, at most 64 (three frames of 181^2 pixels take 17)
+    ps_blocks = 1;
+    for (const PosetFrameDev &d : psf) {
+        const long long side = geoms[lcpts[d.point].obs_view].side + 1;
+        const long long w = std::max((long long)d.ncol * d.nrow, side * side / 8);
+        ps_blocks = std::max(ps_blocks, (int)std::min<long long>(64, (w + 255) / 256));
+    }
+    AL(d_ps_part, psf.size() * ps_blocks * POSET_PART);
+    AL(d_ps_count, psf.size());
     if (!dop_frames.empty()) {
         AL(d_ovf, dop_frames.size() * DOP_MAXOVERFLOW);
         AL(d_ovf_out, dop_frames.size() * DOP_OVF_TERMS);
@@ -371,7 +388,17 @@ int EngineImpl::finalize()
     for (auto &L : lc) lc_tot_n += L.set.n;
     AL(d_lc_x, lc_tot_pts); AL(d_lc_y, lc_tot_pts); AL(d_lc_y2, lc_tot_pts);
     AL(d_lc_t, lc_tot_n); AL(d_lc_obs, lc_tot_n); AL(d_lc_oov, lc_tot_n);
-    AL(d_lc_fit, lc_tot_n + lc_tot_pts);
+    AL(d_lc_fit, lc_tot_n);
+    AL(d_lc_spl, 5 * lc_tot_pts);
+    size_t lc_scratch = 0;          // sets whose work arrays exceed shared memory
+    for (auto &L : lc)
+        if (lc_finalize_smem(L.npts, L.set.n) == 0) lc_scratch += lc_finalize_words(L.npts, L.set.n);
+    const bool lc_shared = lc_scratch == 0;
+    if (!lc_shared) {
+        lc_scratch = 0;
+        for (auto &L : lc) lc_scratch += lc_finalize_words(L.npts, L.set.n);
+        AL(d_lc_scratch, lc_scratch);
+    }
 #undef AL
     if (!h_params) CK(cudaMallocHost((void **)&h_params, sizeof(double) * (size_t)npar()));
     else {
@@ -428,15 +455,17 @@ int EngineImpl::finalize()
     }
     if (!lcpts.empty()) {
         CK(cudaMemcpyAsync(d_lcpts, lcpts.data(), sizeof(LcPointDev) * lcpts.size(), cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(d_lc_items, lc_items.data(), sizeof(int2) * lc_items.size(), cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(d_pt_items, pt_items.data(), sizeof(int) * pt_items.size(), cudaMemcpyHostToDevice, s));
-        size_t px = 0, pn = 0;
-        std::vector<double> lcdof, lcnp;
+        size_t px = 0, pn = 0, ps_ = 0;
+        std::vector<double> lcdof, lcnp, spl(5 * lc_tot_pts);
         for (size_t k = 0; k < lc.size(); k++) {
             LcSetDev &L = lcdev[k];
             L.x = d_lc_x + px; L.y = d_lc_y + px; L.y2 = d_lc_y2 + px;
             L.t = d_lc_t + pn; L.obs = d_lc_obs + pn; L.oov = d_lc_oov + pn;
-            L.fit = d_lc_fit + pn + px;   // n outputs followed by npts scratch
+            L.fit = d_lc_fit + pn;
+            L.spl = d_lc_spl + 5 * px;
+            L.scratch = lc_shared ? nullptr : d_lc_scratch + ps_;
+            ps_ += lc_finalize_words(L.npts, L.n);
+            spline_plan(lc[k].x.data(), L.npts, spl.data() + 5 * px);
             CK(cudaMemcpyAsync(d_lc_x + px, lc[k].x.data(), sizeof(double) * L.npts, cudaMemcpyHostToDevice, s));
             CK(cudaMemcpyAsync(d_lc_t + pn, lc[k].t.data(), sizeof(double) * L.n, cudaMemcpyHostToDevice, s));
             CK(cudaMemcpyAsync(d_lc_obs + pn, lc[k].obs.data(), sizeof(double) * L.n, cudaMemcpyHostToDevice, s));
@@ -446,6 +475,7 @@ int EngineImpl::finalize()
             lcdof.push_back(L.dof);
             lcnp.push_back((double)L.npts);
         }
+        CK(cudaMemcpyAsync(d_lc_spl, spl.data(), sizeof(double) * spl.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_lcsets, lcdev.data(), sizeof(LcSetDev) * lcdev.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_lc_dof, lcdof.data(), sizeof(double) * lcdof.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_lc_npts, lcnp.data(), sizeof(double) * lcnp.size(), cudaMemcpyHostToDevice, s));
@@ -1023,20 +1053,20 @@ int EngineImpl::tune_bins()
         int cy = counts[geoms[work[y].x].tile_base + work[y].y];
         return cx > cy;
     });
-    // radar tiles first, lightcurve-view tiles after them, each part in
-    // decreasing count: the batched FP32 form rasters the two parts with
-    // different kernels
-    std::stable_partition(order.begin(), order.end(),
-                          [&](int x) { return geoms[work[x].x].kind == VIEW_RADAR; });
+    // radar tiles first, then sun-view tiles, then the observer views' that
+    // read the sun views' maps, each part in decreasing count
+    auto part = [&](int x) {
+        const int k = geoms[work[x].x].kind;
+        return k == VIEW_RADAR ? 0 : k == VIEW_LC_SUN ? 1 : 2;
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return part(x) < part(y); });
     std::vector<int2> sorted(work.size());
-    work_radar = nonempty_radar = nonempty_lc = 0;
+    for (int k = 0; k < 3; k++) work_n[k] = work_busy[k] = 0;
     for (size_t k = 0; k < work.size(); k++) {
         sorted[k] = work[order[k]];
-        const bool radar = geoms[sorted[k].x].kind == VIEW_RADAR;
-        const bool busy = counts[geoms[sorted[k].x].tile_base + sorted[k].y] > 0;
-        work_radar += radar;
-        nonempty_radar += radar && busy;
-        nonempty_lc += !radar && busy;
+        const int w = part(order[k]);
+        work_n[w]++;
+        work_busy[w] += counts[geoms[sorted[k].x].tile_base + sorted[k].y] > 0;
     }
     if (!d_work_sorted) {
         int rc = mem.alloc(&d_work_sorted, work.size());
@@ -1087,6 +1117,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (need64) clear(d_fit64, sizeof(double) * (size_t)fit_elems);
         if (!dop_frames.empty()) clear(d_ovf, sizeof(double) * dop_frames.size() * DOP_MAXOVERFLOW);
         if (fused) clear(d_chi2_counters, sizeof(int) * (fh.size() + 1));
+        if (!psf.empty()) clear(d_ps_count, sizeof(int) * psf.size());
         if (int rc_ = front_params(fr)) return rc_;
         launch_front(fr, s);
         if (int rc_ = launched("realize and transform")) return rc_;
@@ -1101,6 +1132,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (!dop_frames.empty())
             CK(cudaMemsetAsync(d_ovf, 0, sizeof(double) * dop_frames.size() * DOP_MAXOVERFLOW, s));
         if (fused) CK(cudaMemsetAsync(d_chi2_counters, 0, sizeof(int) * (fh.size() + 1), s));
+        if (!psf.empty()) CK(cudaMemsetAsync(d_ps_count, 0, sizeof(int) * psf.size(), s));
         mark(1);
         if (int rc_ = launched("state reset")) return rc_;
     }
@@ -1135,30 +1167,24 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     ca.partials = d_partials;
     ca.o2pre = d_o2pre;
 
-    LcArgs la;
-    memset(&la, 0, sizeof la);
-    la.pts = d_lcpts; la.geoms = d_geoms; la.states = d_states;
-    la.chunk = 4096;
-    la.z = static_cast<const double *>(d_pos_z); la.cose = d_pos_cose; la.cosi = d_pos_cosi;
-    la.zill = static_cast<const double *>(d_pos_z);
-    la.f = d_pos_f; la.fill = d_pos_f;
-    la.partials = d_lc_partials;
-    la.bimg = d_ps_b;
-    la.seen = d_seen;
-    la.mincosine_seen = params.mincosine_seen;
-    la.mark_seen = params.mark_seen;
+    ra.pts = d_lcpts;
+    ra.lc_part = d_lc_part;
+    ra.bimg = d_ps_b;
 
     if (form == SHAPE_FORM_PLAIN_FP64) {
         // One view at a time, in dataset order, as calc_fits walks frames.
-        for (int v = 0; v < nviews; v++) {
+        for (int v0 = 0; v0 < nviews; v0++) {
+            // a point's sun view (the one after its observer view) is
+            // rendered first: the observer view's shadows read its maps
+            const int v = geoms[v0].kind == VIEW_LC_OBS ? v0 + 1 : geoms[v0].kind == VIEW_LC_SUN ? v0 - 1 : v0;
             launch_xform_f64(d_geoms + v, 1, md.vx, nv, d_vt64, s);
             launch_bin_f64(d_geoms, v, 1, md, d_vt64, d_states, d_bin_count, d_bin_ids, cap, s);
+            const FrameGeom &g = geoms[v];
             RasterArgs rv = ra;
             rv.work = d_work + view_work0[v];
             rv.nwork = view_nwork[v];
-            rv.maps = geoms[v].kind != VIEW_RADAR;
+            rv.mode = g.kind == VIEW_RADAR ? RASTER_RADAR : g.kind == VIEW_LC_SUN ? RASTER_MAPS : RASTER_PHOTO;
             launch_raster_f64(rv, s);
-            const FrameGeom &g = geoms[v];
             if (g.kind == VIEW_RADAR && fh[g.frame_index].view == v) {
                 const FrameHost &h = fh[g.frame_index];
                 Chi2Args cv = ca;
@@ -1167,13 +1193,6 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
                 cv.partials = d_partials + (size_t)h.item0 * 6;
                 cv.o2pre = d_o2pre + (size_t)h.item0 * 2;
                 launch_chi2_partials(cv, 0, s);
-            } else if (g.kind == VIEW_LC_SUN) {
-                int pt = g.frame_index;
-                LcArgs lv = la;
-                lv.items = d_lc_items + pt_items[2 * pt];
-                lv.nitems = pt_items[2 * pt + 1];
-                lv.partials = d_lc_partials + pt_items[2 * pt];
-                launch_lc_photo(lv, s, false);
             }
             if (int rc_ = launched(g.kind == VIEW_RADAR ? "radar view chain" : "lightcurve view chain")) return rc_;
         }
@@ -1193,27 +1212,25 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         // one CTA per tile that was non-empty when the bins were tuned (they
         // lead each part of the sorted list); the grid-stride loop visits the
         // tiles after them, empty then, so those cost no CTA launches of
-        // their own. Radar tiles and lightcurve / sky tiles are two launches:
-        // the first shades and synthesizes in the form's arithmetic, the
-        // second shades and writes maps in FP64 in both forms.
-        ra.work = d_work_sorted;
+        // their own. Radar tiles, sun-view tiles and the observer views' tiles
+        // are launches of their own (RASTER_*): the first shades and
+        // synthesizes in the form's arithmetic, the others shade, write maps
+        // and do the photometry in FP64 in both forms.
         ra.pdl = pdl ? 1 : 0;
         ra.variant = raster_variant[form];
-        RasterArgs rr = ra, rl = ra;
-        rr.nwork = work_radar;
-        rr.grid = raster_grid(form, nonempty_radar, rr, f32);
-        rl.work = d_work_sorted + work_radar;
-        rl.nwork = (int)work.size() - work_radar;
-        rl.maps = 1;
-        rl.grid = raster_grid(form, nonempty_lc, rl, false);
-        if (f32) {
-            launch_raster_f32(rr, s);
-            launch_raster_f64(rl, s);
-            launch_dop_fit_f32(d_dop_frames, (int)dop_frames.size(), d_fh, d_geoms, d_fit64, d_fit32, s, pdl);
-        } else {
-            launch_raster_f64(rr, s);
-            launch_raster_f64(rl, s);
+        int w0 = 0;
+        for (int k = 0; k < 3; k++) {
+            RasterArgs rk = ra;
+            rk.mode = k;
+            rk.work = d_work_sorted + w0;
+            rk.nwork = work_n[k];
+            w0 += work_n[k];
+            const bool k32 = f32 && k == RASTER_RADAR;
+            rk.grid = raster_grid(form, work_busy[k], rk, k32);
+            if (k32) launch_raster_f32(rk, s);
+            else launch_raster_f64(rk, s);
         }
+        if (f32) launch_dop_fit_f32(d_dop_frames, (int)dop_frames.size(), d_fh, d_geoms, d_fit64, d_fit32, s, pdl);
         mark(4);
         if (int rc_ = launched("raster")) return rc_;
         ca.items = d_chi2_items;
@@ -1222,14 +1239,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (!chi2_items.empty() && !fused) launch_chi2_partials(ca, f32 ? 1 : 0, s);
         mark(5);
         if (int rc_ = launched("chi-square partials")) return rc_;
-        if (!lc_items.empty()) {
-            la.items = d_lc_items;
-            la.nitems = (int)lc_items.size();
-            // lightcurve views hold FP64 cosines in both forms
-            launch_lc_photo(la, s, pdl);
-        }
         mark(6);
-        if (int rc_ = launched("lightcurve photometry")) return rc_;
     }
     FinalizeArgs fa;
     memset(&fa, 0, sizeof fa);
@@ -1251,6 +1261,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         pa.nframes = (int)psf.size();
         pa.frames = d_psf; pa.pts = d_lcpts; pa.geoms = d_geoms; pa.states = d_states;
         pa.bimg = d_ps_b; pa.obs = d_ps_obs; pa.oov = d_ps_oov; pa.fit = d_ps_fit; pa.res = d_ps_res;
+        pa.blocks = ps_blocks; pa.part = d_ps_part; pa.counters = d_ps_count;
         launch_poset_frames(pa, s, chain);
         if (int rc_ = launched("plane-of-sky frames")) return rc_;
     }
@@ -1258,7 +1269,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         LcFinalizeArgs lf;
         lf.nsets = (int)lcdev.size();
         lf.sets = d_lcsets; lf.pts = d_lcpts; lf.geoms = d_geoms; lf.states = d_states;
-        lf.pt_items = d_pt_items; lf.partials = d_lc_partials; lf.set_out = d_lc_out;
+        lf.tile_part = d_lc_part; lf.set_out = d_lc_out;
         size_t sm = 1;
         for (const LcSetDev &L : lcdev) {
             size_t b = lc_finalize_smem(L.npts, L.n);
@@ -1300,16 +1311,12 @@ int EngineImpl::kernels_per_eval(int form) const
     n += (spin_device && n_spin_src > 0) ? 1 : 0;   // view realization from the spin state
     if (form == SHAPE_FORM_PLAIN_FP64) {
         for (int v = 0; v < nviews; v++)
-            n += 3 + ((geoms[v].kind == VIEW_RADAR && fh[geoms[v].frame_index].view == v) ||
-                              geoms[v].kind == VIEW_LC_SUN ? 1 : 0);
+            n += 3 + (geoms[v].kind == VIEW_RADAR && fh[geoms[v].frame_index].view == v ? 1 : 0);
     } else {
-        n += 1;                          // raster
-        if (work_radar > 0 && work_radar < (int)work.size())
-            n += 1;                      // radar and lightcurve / sky views in two launches
+        for (int k : work_n) n += k > 0;  // raster: radar, sun and observer views
         if (form == SHAPE_FORM_BATCHED_FP32 && !dop_frames.empty())
             n += 1;                      // FP32: Doppler spectra rounded from their FP64 sums
         n += (chi2_items.empty() || fused_chi2) ? 0 : 1;   // fused: counted with the summary
-        n += lc_items.empty() ? 0 : 1;
     }
     n += lcdev.empty() ? 0 : 1;          // lightcurve finalize
     n += psf.empty() ? 0 : 1;            // plane-of-sky frames

@@ -127,8 +127,6 @@ struct EngineImpl {
     std::vector<int> frame_view;
     std::vector<double> dop_extra, set_delpp, set_doppp;
     std::vector<LcPointDev> lcpts;
-    std::vector<int2> lc_items;
-    std::vector<int> pt_items;
     int nviews = 0, ntiles = 0;
     long long fit_elems = 0, pos_elems = 0;
     int cap = 512;
@@ -163,9 +161,8 @@ struct EngineImpl {
     shape_deldop_result *d_results = nullptr;
     double *d_set_delpp = nullptr, *d_set_doppp = nullptr, *d_dop_extra = nullptr;
     LcPointDev *d_lcpts = nullptr;
-    int2 *d_lc_items = nullptr;
-    int *d_pt_items = nullptr;
-    double *d_lc_partials = nullptr;
+    double *d_lc_part = nullptr;      // brightness of each tile (observer views)
+    double *d_lc_spl = nullptr, *d_lc_scratch = nullptr;
     LcSetDev *d_lcsets = nullptr;
     double *d_lc_x = nullptr, *d_lc_t = nullptr, *d_lc_obs = nullptr, *d_lc_oov = nullptr;
     double *d_lc_y = nullptr, *d_lc_y2 = nullptr, *d_lc_fit = nullptr, *d_lc_out = nullptr;
@@ -178,6 +175,9 @@ struct EngineImpl {
     PosetFrameDev *d_psf = nullptr;
     double *d_ps_obs = nullptr, *d_ps_oov = nullptr, *d_ps_fit = nullptr, *d_ps_b = nullptr;
     shape_poset_result *d_ps_res = nullptr;
+    int ps_blocks = 1;
+    double *d_ps_part = nullptr;
+    int *d_ps_count = nullptr;
     SetRec *d_setrecs = nullptr;
     shape_eval_summary *d_summary_map = nullptr;   // device address of the mapped pinned h_summary
     std::vector<LcSetDev> lcdev;
@@ -289,10 +289,9 @@ struct EngineImpl {
     // bin tuning results
     int2 *d_work_sorted = nullptr;
     int tuned_max_count = 0, tuned_nonempty = 0;
-    // the sorted work list holds radar tiles first (work_radar of them, the
-    // first nonempty_radar non-empty at tuning), then lightcurve-view tiles
-    // (nonempty_lc non-empty at tuning)
-    int work_radar = 0, nonempty_radar = 0, nonempty_lc = 0;
+    // the sorted work list holds radar, sun-view and observer-view tiles
+    // (RASTER_*): tiles of each part, and its first ones non-empty at tuning
+    int work_n[3] = {0, 0, 0}, work_busy[3] = {0, 0, 0};
     int fixed_cap = 0;            // > 0: bin capacity set by the caller, no autotuning
     int fp32_exact = 1;           // shape_engine_set_fp32_exact (part of the tuning key only)
     // Raster kernel per form (RasterArgs::variant) and grid (0: one CTA per

@@ -57,6 +57,9 @@ struct ModelDev {
     int4 *fvi;                         // corner indices, padded
 };
 
+// What a raster launch does with its views (k_raster).
+enum { RASTER_RADAR, RASTER_MAPS, RASTER_PHOTO };
+
 struct RasterArgs {
     const FrameGeom *geoms;
     const int2 *work;          // (view, tile) items
@@ -90,9 +93,12 @@ struct RasterArgs {
     int accumulate;
     unsigned char *won;
     int variant;               // 0: 256 threads per tile, 1: 128
-    // 1: lightcurve, sky and single POS views (shading and maps, FP64 in
-    // both forms); 0: radar views (shading and delay-Doppler synthesis)
-    int maps;
+    int mode;                  // RASTER_*
+    // RASTER_PHOTO: the views' points, the tiles' brightness sums and the
+    // brightness images of sky frames (LcPointDev::b_base)
+    const LcPointDev *pts;
+    double *lc_part;
+    double *bimg;
 };
 
 // core.cu (FP64, no FMA contraction)
@@ -130,7 +136,7 @@ void launch_xform_f64(const FrameGeom *g, int nviews, const double4 *vx, int nv,
                       cudaStream_t s, bool pdl = false);
 // the first launch of a batched evaluation (k_front)
 struct FrontArgs {
-    static constexpr int CLEARS = 6;
+    static constexpr int CLEARS = 7;
     const FrameGeom *geoms;
     int nviews;
     ModelDev m;
@@ -228,32 +234,17 @@ void launch_dop_fit_f32(const int *dop_frames, int n, const FrameHost *fh, const
                         const double *fit64, float *fit32, cudaStream_t s, bool pdl);
 void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s, bool pdl);
 
-struct LcArgs {
-    int npoints;
-    const LcPointDev *pts;
-    const FrameGeom *geoms;
-    const FrameState *states;
-    const int2 *items;          // (point, pixel start) work items
-    int nitems;
-    int chunk;                  // pixels per item
-    const double *z, *zill;     // POS depth maps (FP64 in both forms)
-    const void *cosi;           // T POS map
-    void *cose;                 // masked in place, as posmask does
-    const int *f, *fill;
-    double *partials;           // brightness partial per item
-    double *bimg;               // brightness images of plane-of-sky frames (LcPointDev::b_base)
-    unsigned char *seen;
-    double mincosine_seen;
-    int mark_seen;
-};
-void launch_lc_photo(const LcArgs &a, cudaStream_t s, bool pdl);
-
 struct LcSetDev {
     int npts, n;                // calc points, observed points
     int pt0;                    // first calc point (global)
-    int item0, nitems;          // photo items of this set's points are contiguous
     const double *x, *t, *obs, *oov;  // device arrays
+    // the spline's elimination, which depends on the epochs only: the lower
+    // coefficients w, the pivots and their reciprocals, the multipliers of
+    // y2[i+1] in y2[i] and the spans ([5 * npts])
+    const double *spl;
     double *y, *y2, *fit;       // device outputs
+    double *scratch;            // work arrays of a set too large for shared memory (null: none)
+    double o2;                  // sum obs^2 / var in order
     double weight, dof, cal_in;
     int cal_floating;
 };
@@ -263,12 +254,12 @@ struct LcFinalizeArgs {
     const LcPointDev *pts;
     const FrameGeom *geoms;
     const FrameState *states;
-    const int *pt_items;        // per point: first item, count (2 ints)
-    const double *partials;
+    const double *tile_part;    // brightness of each tile (RASTER_PHOTO)
     double *set_out;            // per set: cal, chi2, posbnd flag, logfactor sum
     size_t smem_per_set;        // dynamic shared memory (lc_finalize_smem of the largest set), 0: global
 };
 constexpr size_t LC_FINALIZE_SMEM_MAX = 160 * 1024;
+size_t lc_finalize_words(int npts, int n);   // doubles of a set's work arrays
 size_t lc_finalize_smem(int npts, int n);
 cudaError_t configure_lc_finalize();
 void launch_lc_finalize(const LcFinalizeArgs &a, cudaStream_t s, bool pdl);
@@ -302,9 +293,10 @@ void launch_realize_views(const SpinRealizeArgs &a, cudaStream_t s);
 
 struct SetRec { int type; int first; int count; };   // type 0 deldop (frames), 1 lightcurve (set index), 2 plane-of-sky (frames)
 
-// Plane-of-sky frames (calc_poset after apply_photo, and chi2_poset): one
-// block per frame resamples the brightness image onto the fit grid,
+// Plane-of-sky frames (calc_poset after apply_photo, and chi2_poset): blocks
+// blocks per frame resample the brightness image onto the fit grid,
 // checks that the grid holds every lit pixel and forms the chi-square.
+constexpr int POSET_PART = 8;
 struct PosetArgs {
     int nframes;
     const PosetFrameDev *frames;
@@ -315,6 +307,9 @@ struct PosetArgs {
     const double *obs, *oov;    // observed images and 1/variance
     double *fit;                // fit images
     shape_poset_result *res;    // per-frame results
+    int blocks;                 // blocks per frame
+    double *part;               // [nframes * blocks * POSET_PART] their sums and extremes
+    int *counters;              // [nframes] finished blocks, zero before the launch
 };
 void launch_poset_frames(const PosetArgs &a, cudaStream_t s, bool pdl);
 struct SummaryArgs {
