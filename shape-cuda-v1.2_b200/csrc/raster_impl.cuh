@@ -52,6 +52,9 @@ namespace shape {
 template <typename T> __device__ inline T tsin(T x);
 template <> __device__ inline double tsin<double>(double x) { return sin(x); }
 template <> __device__ inline float tsin<float>(float x) { return sinf(x); }
+template <typename T> __device__ inline T tsinpi(T x);
+template <> __device__ inline double tsinpi<double>(double x) { return sinpi(x); }
+template <> __device__ inline float tsinpi<float>(float x) { return sinpif(x); }
 template <typename T> __device__ inline T tpow(T x, T y);
 template <> __device__ inline double tpow<double>(double x, double y) { return pow(x, y); }
 template <> __device__ inline float tpow<float>(float x, float y) { return powf(x, y); }
@@ -447,6 +450,122 @@ __device__ inline bool pixel_dd_scatter_lean(const RasterArgs &a, const FrameGeo
     return true;
 }
 
+// ---- Frames with other responses, and Doppler spectra: footprints of at most
+// STAGE_COLS columns with up to 3 x 3 sinc^2 points per pixel. A pixel's column
+// weights are staged in shared memory (a row per lane of the warp; no local
+// arrays) and added from there.
+constexpr int STAGE_COLS = 11;             // odd: a warp's rows start in different banks
+template <typename T> struct StageRow { T w[STAGE_COLS]; };
+
+// Writes the pixel's Doppler weights (zero beyond the footprint) and returns
+// the cross-section over the sum of all responses, so that a bin's
+// contribution is the returned value x its delay response x its column's
+// weight (src/shape/pos2deldop.c:432-496). Each of the NS x NS sinc^2 points of
+// column k is sin^2(pi x)/(pi x)^2 at x = x0 - k, and sin^2(pi x) = sin^2(pi x0)
+// for every column: NS^2 sines per pixel instead of NS^2 per column.
+template <typename T, int NS>
+__device__ inline T stage_columns(const FrameGeom &g, const PixDD<T> &d, T *w)
+{
+    T frac;
+    int i0;
+    if constexpr (sizeof(T) == 4) { frac = d.dfrac; i0 = d.ifl - d.idop_min; }
+    else { const T fl = floor(d.dopPOS); frac = d.dopPOS - fl; i0 = (int)fl - d.idop_min; }
+    const int nc = d.idop_max - d.idop_min + 1;
+    T x0[NS * NS], s2[NS * NS];
+#pragma unroll
+    for (int i = 0; i < NS; i++)
+#pragma unroll
+        for (int j = 0; j < NS; j++) {
+            const T x = frac + (NS > 1 ? (T)(g.dopdiff_bl + i * g.yincr + j * g.xincr) : (T)0);
+            const T sn = tsinpi<T>(x - rint(x));
+            x0[i * NS + j] = x;
+            s2[i * NS + j] = sn * sn * (T)0.10132118364233778;        // 1 / pi^2
+        }
+    T sum = 0;
+    for (int c = 0; c < STAGE_COLS; c++) {
+        T v = 0;
+        if (c < nc) {
+#pragma unroll
+            for (int k = 0; k < NS * NS; k++) {
+                const T x = x0[k] + (T)(i0 - c);
+                const T r = quick_rcp(x);
+                // the reference's |pi x| > 1e-4
+                v += (fabs((T)3.141592653589793 * x) > (T)1.0e-4) ? s2[k] * r * r : (T)1;
+            }
+            if (NS > 1) v = v / (NS * NS);
+            sum += v;
+        }
+        w[c] = v;
+    }
+    return sum;
+}
+template <typename T>
+__device__ __noinline__ T stage_pixel(const RasterArgs &a, const FrameGeom &g, T cose, PixDD<T> d, T *w)
+{
+    const T sdop = g.nsinc2 == 1 ? stage_columns<T, 1>(g, d, w)
+                 : g.nsinc2 == 2 ? stage_columns<T, 2>(g, d, w) : stage_columns<T, 3>(g, d, w);
+    T sdel = 1;                            // a spectrum's delay response
+    if (!g.dop1d) {
+        const DDC<T> k = load_ddc<T>(g);
+        sdel = 0;
+        for (int e = d.idel_min; e <= d.idel_max; e++)
+            sdel += del_resp<T>(g, k, d.delPOS, sizeof(T) == 4 ? d.ddel0 - (T)(e - d.idel_min) : d.delPOS - (T)e, e);
+    }
+    return radlaw_call<T>(a.laws[g.law], cose) * (T)g.kmpp * (T)g.kmpp * d.codefactor / (sdel * sdop);
+}
+// Whether stage_pixel serves the frame and the footprint.
+template <typename T>
+__device__ inline bool stage_fits(const FrameGeom &g, const PixDD<T> &d)
+{
+    return g.nsinc2 <= 3 && d.idop_max - d.idop_min < STAGE_COLS;
+}
+// The rows of a staged delay-Doppler footprint, added to the frame's image.
+template <typename T>
+__device__ __noinline__ void scatter_staged(const FrameGeom &g, PixDD<T> d, T amp, const T *w, T *fit)
+{
+    const DDC<T> k = load_ddc<T>(g);
+    const int nc = d.idop_max - d.idop_min + 1;
+    for (int e = d.idel_min; e <= d.idel_max; e++) {
+        const T ad = amp * del_resp<T>(g, k, d.delPOS, sizeof(T) == 4 ? d.ddel0 - (T)(e - d.idel_min) : d.delPOS - (T)e, e);
+        if (ad == (T)0) continue;
+        T *cell = fit + (long long)(e - 1) * g.ndop + (d.idop_min - 1);
+        if constexpr (sizeof(T) == 4) {
+            // aligned 16-byte reductions; lanes outside the footprint add zero
+            const int mis = (int)((reinterpret_cast<uintptr_t>(cell) >> 2) & 3);
+            float4 *grp = reinterpret_cast<float4 *>(cell - mis);
+            for (int c = -mis; c < nc; c += 4, grp++) {
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) v[j] = (c + j >= 0 && c + j < nc) ? ad * w[c + j] : 0.0f;
+                atomicAdd(grp, make_float4(v[0], v[1], v[2], v[3]));
+            }
+        } else {
+            for (int c = 0; c < nc; c++) atomicAdd(cell + c, ad * w[c]);
+        }
+    }
+}
+// The staged spectra of a warp's pixels (mask: the lanes that have one; o1, amp:
+// each lane's first column and factor), added to the frame's spectrum: lane l
+// sums column cb + l over the warp's pixels in FP64 and adds it once, where one
+// atomic per pixel and column met on the few hundred bins that all of a
+// spectrum's pixels share. All lanes of the warp call it together.
+template <typename T, typename A>
+__device__ inline void add_spectra(unsigned mask, int o1, T amp, int c1, int c2, const StageRow<T> *rows, A *spec)
+{
+    const int lane = threadIdx.x & 31;
+    for (int cb = c1; cb <= c2; cb += 32) {
+        const int c = cb + lane;
+        double sum = 0.0;
+        for (unsigned m = mask; m; m &= m - 1) {
+            const int p = __ffs(m) - 1;
+            const int k = c - __shfl_sync(0xffffffffu, o1, p);
+            const T ap = __shfl_sync(0xffffffffu, amp, p);
+            if (k >= 0 && k < STAGE_COLS) sum += (double)(ap * rows[p].w[k]);
+        }
+        if (c <= c2 && sum != 0.0) atomicAdd(spec + (c - 1), (A)sum);
+    }
+}
+
 // A Doppler pixel whose footprint leaves the spectrum adds its contributions
 // to the frame's overflow spectrum instead (src/shape/pos2doppler.c:399-414):
 // the same weights as pixel_dd_scatter's generic path (one row, delay
@@ -519,6 +638,7 @@ struct TileShared {
             unsigned short cand[TILE_PIX][CAND];     // bin entries that may cover the pixel
         };
         PixelHit hit[TILE_PIX];                      // slow path: the outcome
+        StageRow<T> stage[NT];                       // phase C: a row per thread
     };
     double xs[TILE_W], ys[TILE_W];         // pixel centres
     double pz[TILE_PIX];                   // radar views: the shaded pixels' depth and cos(e)
@@ -1119,13 +1239,32 @@ k_raster(const __grid_constant__ RasterArgs a)
                 // FP32 as 16-byte vector reductions, FP64 as scalar atomics
                 // (both measured faster than a shared-memory accumulator
                 // flushed per tile).
-                if (dd.ok) {
-                    T *fit = static_cast<T *>(a.fit) + g.fit_base;
-                    if (sizeof(T) == 4 && g.dop1d) pixel_dd_scatter<T, double>(a, g, cosa, dd, a.fit64 + g.fit_base);
-                    else if (!pixel_dd_scatter_lean<T>(a, g, cosa, dd, fit)) pixel_dd_scatter<T, T>(a, g, cosa, dd, fit);
-                } else if (g.dop1d && lit) {
-                    S.any_overflow = 1;
-                    pixel_dop_overflow<T>(a, g, cosa, dd);
+                T *fit = static_cast<T *>(a.fit) + g.fit_base;
+                T *row = sh.stage[tid].w;
+                if (g.dop1d) {
+                    // a spectrum is summed in FP64 in both forms
+                    double *spec = (sizeof(T) == 4 ? a.fit64 : static_cast<double *>(a.fit)) + g.fit_base;
+                    const bool staged_px = dd.ok && stage_fits(g, dd);
+                    const T amp = staged_px ? stage_pixel<T>(a, g, cosa, dd, row) : (T)0;
+                    __syncwarp();
+                    const unsigned mask = __ballot_sync(0xffffffffu, staged_px);
+                    const int c1 = warp_min(staged_px ? dd.idop_min : INT_MAX);
+                    const int c2 = warp_max(staged_px ? dd.idop_max : INT_MIN);
+                    add_spectra<T, double>(mask, dd.idop_min, amp, c1, c2, &sh.stage[tid & ~31], spec);
+                    __syncwarp();
+                    if (dd.ok && !staged_px) {
+                        pixel_dd_scatter<T, double>(a, g, cosa, dd, spec);
+                    } else if (lit && !dd.ok) {
+                        S.any_overflow = 1;
+                        pixel_dop_overflow<T>(a, g, cosa, dd);
+                    }
+                } else if (dd.ok && !pixel_dd_scatter_lean<T>(a, g, cosa, dd, fit)) {
+                    if (stage_fits(g, dd)) {
+                        const T amp = stage_pixel<T>(a, g, cosa, dd, row);
+                        scatter_staged<T>(g, dd, amp, row, fit);
+                    } else {
+                        pixel_dd_scatter<T, T>(a, g, cosa, dd, fit);
+                    }
                 }
             }
         }
