@@ -7,6 +7,8 @@
 
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -216,6 +218,7 @@ struct EngineImpl {
         if (h_params) { cudaFreeHost(h_params); h_params = nullptr; }
         if (h_summary) { cudaFreeHost(h_summary); h_summary = nullptr; }
         if (h_msum) { cudaFreeHost(h_msum); h_msum = nullptr; }
+        if (h_read) { cudaFreeHost(h_read); h_read = nullptr; h_read_bytes = 0; }
         if (h_spin) { cudaFreeHost(h_spin); h_spin = nullptr; }
         if (h_spin_off) { cudaFreeHost(h_spin_off); h_spin_off = nullptr; }
         if (ev0) { cudaEventDestroy(ev0); ev0 = nullptr; }
@@ -258,6 +261,14 @@ struct EngineImpl {
     int front_params(FrontArgs &fr);
     int enqueue(int form, cudaEvent_t *marks = nullptr);
     int launch(int form);
+    // device ranges to copy out (bytes 0: skipped), and the pinned buffer they
+    // pass through: grown on demand, at most READBACK_MAX bytes
+    struct ReadBack { void *dst; const void *src; size_t bytes; };
+    static constexpr size_t READBACK_MAX = (size_t)4 << 20;
+    unsigned char *h_read = nullptr;
+    size_t h_read_bytes = 0;
+    std::mutex read_mu;
+    int read_back(std::initializer_list<ReadBack> parts);
     int poll();
     int finish(shape_eval_summary *out);
     int pending_baddiam = 0;
