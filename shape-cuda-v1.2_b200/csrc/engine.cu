@@ -123,6 +123,7 @@ int EngineImpl::finalize()
         g.n = n;
         g.side = 2 * n + 1;
         g.kmpp = kmpp;
+        g.ikm = 1.0 / kmpp;
         g.tiles_x = (g.side + TILE_W - 1) / TILE_W;
         g.tile_base = tile_base;
         g.vt_base = (int)geoms.size() * nv;

@@ -41,7 +41,7 @@ struct FrameGeom {
     double off[3];       // orbit offset added to the view-frame vertices (posvis's orbit_offset; 0 here otherwise)
     double wscale;       // weight of this view's cross-section in its frame: 1 / views of a smeared frame
     int no_seen;         // 1: a smeared frame's view other than the frame's epoch view (marks no seen facets)
-    double kmpp;
+    double kmpp, ikm;    // km per pixel and its reciprocal
     int n, side;         // POS half width, 2n+1
     int tiles_x;         // tiles per POS side
     int tile_base;       // first tile of this view in the tile arrays

@@ -167,6 +167,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     if (orbit_offset)
         for (int k = 0; k < 3; k++) g.off[k] = orbit_offset[k];
     g.kmpp = view->km_per_pixel;
+    g.ikm = 1.0 / g.kmpp;
     g.n = n;
     g.side = side;
     g.tiles_x = tiles_x;
@@ -377,6 +378,7 @@ static int pos2deldop_impl(int device, const shape_pos_view *view, const shape_p
     g.n = n;
     g.side = side;
     g.kmpp = view->km_per_pixel;
+    g.ikm = 1.0 / g.kmpp;
     g.ndel = frame->ndel;
     g.ndop = frame->ndop;
     radar_set_consts(g, *set, *par, 0, 0);

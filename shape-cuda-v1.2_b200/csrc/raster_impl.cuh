@@ -36,12 +36,18 @@
 #include "posmask_dev.cuh"
 
 // Resident warps per SM that the register allocation must allow (FP32 /
-// FP64). The kernels wait on dependent loads more than they issue, so warps
-// count: 64 uneven frames in FP32 with 128-thread CTAs take 0.102 / 0.104 /
-// 0.108 ms at 32 / 40 / 48 warps and 0.127 / 0.117 / 0.113 with 256; 800
-// lightcurve points in FP64 1.89 / 1.58 / 1.60 at 24 / 32 / 40.
+// FP64), and the share of the SM's 256 KB that the CTAs' shared memory may
+// take; the rest is L1, where the facets' vertices and the spills live. The
+// kernels wait on those loads more than they issue, so both count. 128-thread
+// CTAs, ms: 64 uneven frames in FP32 at 40 warps 0.106 with all of it shared
+// and 0.105 with 80 %, at 32 warps 0.104, 0.099 with 80 % and 0.099 with 65;
+// 800 lightcurve points in FP64 at 32 warps 1.73, 1.63 and 1.74, at 24 2.02,
+// 1.94 and 1.90; 16 frames of 511^2 0.222 and 0.214 at 40, 0.204 and 0.192 at 32.
 #ifndef RASTER_WARPS_F32
-#define RASTER_WARPS_F32 40
+#define RASTER_WARPS_F32 32
+#endif
+#ifndef RASTER_SHARED_PCT
+#define RASTER_SHARED_PCT 80
 #endif
 #ifndef RASTER_WARPS_F64
 #define RASTER_WARPS_F64 32
@@ -1033,7 +1039,7 @@ k_raster(const __grid_constant__ RasterArgs a)
         bool slow = count > a.cap || count > 65536;      // a candidate is held in 16 bits
         const bool staged = count <= NT;
         if (!slow) {
-            const float ikm = (float)(1.0 / g.kmpp);
+            const float ikm = (float)g.ikm;
             for (int k = tid; k < count; k += NT) {
                 const int2 e = bin[k];
                 const FacetTerms q = facet_terms(vt, a.fvi[e.x]);
@@ -1292,9 +1298,7 @@ inline void launch_raster_t(const RasterArgs &a, cudaStream_t s)
     with_raster_kernel<T>(a, [&](auto kern, int nt) { launch_k(kern, dim3(grid), dim3(nt), 0, s, a.pdl != 0, a); });
 }
 
-// Called once per device before any launch (not inside stream capture): the
-// kernels run several CTAs per SM, which needs the largest shared-memory
-// carveout.
+// Called once per device before any launch (not inside stream capture).
 template <typename T>
 inline cudaError_t configure_raster_t()
 {
@@ -1303,8 +1307,7 @@ inline cudaError_t configure_raster_t()
     for (a.mode = RASTER_RADAR; a.mode <= (sizeof(T) == 8 ? RASTER_PHOTO : RASTER_RADAR); a.mode++)
         for (a.variant = 0; a.variant < 2 && e == cudaSuccess; a.variant++)
             with_raster_kernel<T>(a, [&](auto kern, int) {
-                e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         cudaSharedmemCarveoutMaxShared);
+                e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, RASTER_SHARED_PCT);
             });
     return e;
 }
