@@ -411,109 +411,59 @@ __device__ inline KSum shfl_ksum(KSum a, int off)
     return b;
 }
 
-// Per (frame, chunk) partial sums of chi2_deldop (src/shape/chi2.c:436-441):
-// o2 = sum obs^2/var, m2 = sum fit^2/var, om = sum fit*obs/var, each
-// product in the reference's order, accumulated with compensation.
-template <typename T>
-__device__ void chi2_item_warp(const Chi2Args &a, int it, const Chi2Item &item, double *part);
-
-// Resident 256-thread blocks per SM of the chi-square kernels: a warp keeps
-// its item's 48 loads in flight, so residency trades against registers (on
-// 64 uneven frames: 3 blocks, 80 registers, 28.6 us; 2 blocks, 120
-// registers, 31.5 us; 4 blocks, 64 registers, 30.7 us).
-#ifndef CHI2_MIN_BLOCKS
-#define CHI2_MIN_BLOCKS 3
-#endif
-
-// One warp per item, items in grid-stride order over the block's warps.
-template <typename T>
-__global__ void __launch_bounds__(CHI2_THREADS, CHI2_MIN_BLOCKS) k_chi2_partials(Chi2Args a)
+// Sum of obs^2 / var of each radar frame (src/shape/chi2.c:436-441), which
+// depends on the data only: one block per frame, once per dataset.
+__global__ void __launch_bounds__(256) k_frame_o2(const FrameHost *fh, const FrameGeom *geoms, const double *obs,
+                                                  const double *oov, double *o2)
 {
-    const int wpb = blockDim.x >> 5;
-    for (int it = blockIdx.x * wpb + (threadIdx.x >> 5); it < a.nitems; it += gridDim.x * wpb)
-        chi2_item_warp<T>(a, it, a.items[it], a.partials + (size_t)it * 6);
+    __shared__ double red[8][2];
+    const FrameGeom &g = geoms[fh[blockIdx.x].view];
+    const long long n = (long long)g.ndel * g.ndop;
+    KSum q = {0, 0};
+    for (long long k = threadIdx.x; k < n; k += blockDim.x) {
+        const double ob = obs[g.fit_base + k];
+        q.add(ob * ob * oov[g.fit_base + k]);
+    }
+    for (int off = 16; off > 0; off >>= 1) q.merge(shfl_ksum(q, off));
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) { red[wid][0] = q.s; red[wid][1] = q.c; }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    q = {0, 0};
+    for (int w = 0; w < 8; w++) q.merge(KSum{red[w][0], red[w][1]});
+    o2[2 * blockIdx.x] = q.s;
+    o2[2 * blockIdx.x + 1] = q.c;
 }
 
-// A frame's three sums from its item partials (6 per item: o2, m2, om, each
-// a compensated sum and its compensation) in one fixed order: lane l of a
-// warp merges items l, l+32, l+64, ... in turn, then the lanes' sums merge
-// pairwise (l with l+16, l+8, ..., l+1), and the frame's start values (a
-// Doppler frame's overflow o2 and m2, else 0) take the result last.
-// frame_sums_warp does this with the 32 lanes; frame_sums_serial computes
-// the same numbers in one thread, so the batched and plain forms agree
-// bit for bit.
-__device__ inline void ksum_take(KSum &q, const double *p)
-{
-    q.add(p[0]);
-    q.c += p[1];
-}
-__device__ void frame_sums_warp(const double *part, int nitems, const double start[3], KSum out[3], bool via_l2)
+// A frame's m2 and om from its items' partial sums (a compensated sum and its
+// compensation each): lane l merges items l, l + 32, ..., then the lanes merge
+// pairwise, a fixed order; read through L2 (other warps wrote them).
+__device__ inline void frame_sums_warp(const double *part, int nitems, KSum &m2, KSum &om)
 {
     const int lane = threadIdx.x & 31;
-    KSum q[3] = {{0, 0}, {0, 0}, {0, 0}};
-    for (int it = lane; it < nitems; it += 32)
-        for (int k = 0; k < 3; k++) {
-            double p[2];
-            p[0] = via_l2 ? __ldcg(part + (size_t)it * 6 + 2 * k) : part[(size_t)it * 6 + 2 * k];
-            p[1] = via_l2 ? __ldcg(part + (size_t)it * 6 + 2 * k + 1) : part[(size_t)it * 6 + 2 * k + 1];
-            ksum_take(q[k], p);
-        }
-    for (int off = 16; off > 0; off >>= 1)
-        for (int k = 0; k < 3; k++) q[k].merge(shfl_ksum(q[k], off));
-    for (int k = 0; k < 3; k++) {
-        out[k].s = start[k];
-        out[k].c = 0.0;
-        out[k].merge(q[k]);
+    m2 = om = KSum{0, 0};
+    for (int k = lane; k < nitems; k += 32) {
+        const double *p = part + 4 * k;
+        const KSum a = {__ldcg(p), __ldcg(p + 1)}, b = {__ldcg(p + 2), __ldcg(p + 3)};
+        m2.merge(a);
+        om.merge(b);
     }
-}
-__device__ void frame_sums_serial(const double *part, int nitems, const double start[3], KSum out[3])
-{
-    KSum q[32][3];
-    for (int l = 0; l < 32; l++)
-        for (int k = 0; k < 3; k++) q[l][k] = KSum{0, 0};
-    for (int it = 0; it < nitems; it++)
-        for (int k = 0; k < 3; k++) ksum_take(q[it & 31][k], part + (size_t)it * 6 + 2 * k);
-    for (int off = 16; off > 0; off >>= 1)
-        for (int l = 0; l < off; l++)
-            for (int k = 0; k < 3; k++) q[l][k].merge(q[l + off][k]);
-    for (int k = 0; k < 3; k++) {
-        out[k].s = start[k];
-        out[k].c = 0.0;
-        out[k].merge(q[0][k]);
+    for (int off = 16; off > 0; off >>= 1) {
+        m2.merge(shfl_ksum(m2, off));
+        om.merge(shfl_ksum(om, off));
     }
 }
 
-// A frame's chi-square terms: chi2_deldop's sums, calibration and
-// chi-square (src/shape/chi2.c:436-460) from the frame's item partials.
-// part: the chi-square partials (6 per item), in global or shared memory;
-// part0: the index of the frame's first item in part. One thread.
-__device__ inline void frame_start(const FinalizeArgs &a, const FrameHost &h, double start[3])
+// A frame's chi-square terms (src/shape/chi2.c:436-460).
+__device__ void frame_chi2_from_sums(const FrameHost &h, const KSum &so2, const KSum &sm2, const KSum &som,
+                                     shape_deldop_result &r)
 {
-    // a Doppler frame's sums start from its overflow spectrum's o2 and m2
-    // (src/shape/chi2.c:745-747)
-    const double *ovf = (h.dop_index >= 0) ? a.ovf_out + (size_t)h.dop_index * DOP_OVF_TERMS : nullptr;
-    start[0] = ovf ? ovf[0] : 0.0;
-    start[1] = ovf ? ovf[1] : 0.0;
-    start[2] = 0.0;
-}
-__device__ void frame_chi2_from_sums(const FrameHost &h, const KSum q[3], shape_deldop_result &r)
-{
-    double o2 = q[0].value(), m2 = q[1].value(), om = q[2].value();
+    const double o2 = so2.value(), m2 = sm2.value(), om = som.value();
     double cal = h.cal_in;
     if (h.cal_floating)
         cal = (om > 0.0) ? om / m2 : SHAPE_TINYCALFACT;
     r.o2 = o2; r.m2 = m2; r.om = om; r.cal = cal;
     r.chi2 = h.weight * (o2 - 2 * cal * om + cal * cal * m2);
-}
-__device__ void finalize_frame_chi2(const FinalizeArgs &a, int fr, const double *part, int part0,
-                                    shape_deldop_result &r)
-{
-    const FrameHost &h = a.fh[fr];
-    double start[3];
-    frame_start(a, h, start);
-    KSum q[3];
-    frame_sums_serial(part + (size_t)part0 * 6, h.nitems, start, q);
-    frame_chi2_from_sums(h, q, r);
 }
 
 // A frame's posvis / pos2deldop outputs (limits, flags, log-factors), which
@@ -567,34 +517,18 @@ __device__ void finalize_frame_geom(const FinalizeArgs &a, int fr, shape_deldop_
     }
 }
 
-// Per-frame results: both parts, stored in a.results[fr].
-__device__ shape_deldop_result finalize_frame(const FinalizeArgs &a, int fr, const double *part, int part0)
+// Overflow spectrum of a Doppler frame (src/shape/pos2doppler.c:451-499), by one
+// warp: sums over the bins inside the frame's Doppler limits (count of nonzero
+// bins, squares over the noise variance, cross section and its mean bin) and
+// the flag of a model wider than the overflow spectrum.
+__device__ void doppler_overflow_warp(const FinalizeArgs &a, const FrameHost &h)
 {
-    shape_deldop_result r;
-    finalize_frame_chi2(a, fr, part, part0, r);
-    finalize_frame_geom(a, fr, r);
-    a.results[fr] = r;
-    return r;
-}
-
-
-// Overflow spectra of the Doppler frames (src/shape/pos2doppler.c:451-499):
-// one block per frame sums the bins inside the frame's Doppler limits
-// (count of nonzero bins, squares over the noise variance, cross section and
-// its mean bin) and flags a model wider than the overflow spectrum.
-__global__ void k_doppler_overflow(DopOvfArgs a)
-{
-    grid_dep_trigger();
-    grid_dep_wait();
-    __shared__ double red[4][32];
-    const int k = blockIdx.x;
-    const int fr = a.frames[k];
-    const FrameHost &h = a.fh[fr];
+    const int lane = threadIdx.x & 31;
     const FrameGeom &g = a.geoms[h.view];
     const FrameState &st = a.states[h.view];
-    double *out = a.out + (size_t)k * DOP_OVF_TERMS;
+    double *out = a.ovf_out + (size_t)h.dop_index * DOP_OVF_TERMS;
     if (!st.any_overflow) {
-        if (threadIdx.x < DOP_OVF_TERMS) out[threadIdx.x] = 0.0;
+        if (lane < DOP_OVF_TERMS) out[lane] = 0.0;
         return;
     }
     const double *ov = a.ovf + g.ovf_base;
@@ -602,7 +536,7 @@ __global__ void k_doppler_overflow(DopOvfArgs a)
     const int idop0 = g.idop0;
     const int j1 = max(st.idoplim[0] + idop0, 0), j2 = min(st.idoplim[1] + idop0, DOP_MAXOVERFLOW - 1);
     double o2 = 0.0, m2 = 0.0, xs = 0.0, dm = 0.0;
-    for (int j = j1 + (int)threadIdx.x; j <= j2; j += blockDim.x) {
+    for (int j = j1 + lane; j <= j2; j += 32) {
         const double v = ov[j];
         if (v != 0.0) {
             o2 += 1.0;
@@ -617,29 +551,16 @@ __global__ void k_doppler_overflow(DopOvfArgs a)
         xs += __shfl_down_sync(0xffffffffu, xs, o);
         dm += __shfl_down_sync(0xffffffffu, dm, o);
     }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) { red[0][w] = o2; red[1][w] = m2; red[2][w] = xs; red[3][w] = dm; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        o2 = m2 = xs = dm = 0.0;
-        for (int ww = 0; ww < (int)(blockDim.x >> 5); ww++) {
-            o2 += red[0][ww]; m2 += red[1][ww]; xs += red[2][ww]; dm += red[3][ww];
-        }
-        if (xs != 0.0) dm /= xs;
-        out[0] = o2; out[1] = m2; out[2] = xs; out[3] = dm;
-        const int lo = st.idoplim[0] + idop0, hi = st.idoplim[1] + idop0;
-        if (lo < 0 || hi >= DOP_MAXOVERFLOW) {
-            const double dopfactor = (max(hi, DOP_MAXOVERFLOW) - min(lo, 0)) / (1.0 * DOP_MAXOVERFLOW);
-            out[4] = 1.0;
-            out[5] = log(dopfactor);
-        } else {
-            out[4] = 0.0;
-            out[5] = 0.0;
-        }
+    if (lane != 0) return;
+    if (xs != 0.0) dm /= xs;
+    out[0] = o2; out[1] = m2; out[2] = xs; out[3] = dm;
+    out[4] = out[5] = 0.0;
+    const int lo = st.idoplim[0] + idop0, hi = st.idoplim[1] + idop0;
+    if (lo < 0 || hi >= DOP_MAXOVERFLOW) {
+        out[4] = 1.0;
+        out[5] = log((max(hi, DOP_MAXOVERFLOW) - min(lo, 0)) / (1.0 * DOP_MAXOVERFLOW));
     }
 }
-
-// ------------------------------------------------------------ lightcurves
 
 // A radar frame's badradar term of the objective (src/shape/calc_fits.c:
 // 545-550): dof * log-factor / views, summed over the views whose
@@ -1015,73 +936,18 @@ __global__ void __launch_bounds__(1024) k_lc_finalize(LcFinalizeArgs a)
 // (src/shape/calc_fits.c:407-409, 511-550, 1947) and the objective's
 // bad-model multipliers (src/shape/bestfit.c:806-866), no penalties.
 //
-// The totals are serial sums in dataset order (the reference's order). With
-// a.smem_frames set, each frame's thread leaves its chi2 and dof-weighted
-// log-factor terms in shared memory, so the serial pass reads shared memory
-// instead of waiting on one global load per frame.
-template <typename Term>
-__device__ void summary_totals(const SummaryArgs &a, Term term);
-
-__global__ void k_summary(FinalizeArgs fa, SummaryArgs a)
+// The totals are serial sums in dataset order (the reference's order). One
+// warp: its lanes read 32 radar frames' results at a time (through L2, other
+// warps of the launch may have written them), and every lane adds the values
+// it is handed by shuffles, so the sums wait on no load.
+__device__ void totals_warp(const SummaryArgs &a)
 {
-    grid_dep_wait();
-    extern __shared__ double ssm[];
-    const bool use_sm = a.smem_frames;
-    double *s_chi2 = ssm, *s_plog = ssm + fa.nframes, *s_blog = ssm + 2 * (size_t)fa.nframes;
-    unsigned char *s_flag = reinterpret_cast<unsigned char *>(ssm + 3 * (size_t)fa.nframes);
-    // the chi-square partials are copied to shared memory by the whole block
-    // first, so each frame's serial merge reads shared memory
-    const double *part = fa.partials;
-    if (use_sm && a.smem_partials) {
-        // partials start at the first 16-byte boundary after the flags
-        const size_t poff = (25 * (size_t)fa.nframes + 15) & ~(size_t)15;
-        double *sp = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(ssm) + poff);
-        // 16-byte loads, eight in flight per thread before their stores
-        const double2 *src = reinterpret_cast<const double2 *>(fa.partials);
-        double2 *dst = reinterpret_cast<double2 *>(sp);
-        const int n2 = 3 * a.nitems;
-#pragma unroll 8
-        for (int k = threadIdx.x; k < n2; k += blockDim.x) dst[k] = src[k];
-        __syncthreads();
-        part = sp;
-    }
-    // per-frame results (one thread per frame), then the totals
-    for (int fr = threadIdx.x; fr < fa.nframes; fr += blockDim.x) {
-        const shape_deldop_result r = finalize_frame(fa, fr, part, fa.fh[fr].item0);
-        if (use_sm) {
-            s_chi2[fr] = r.chi2;
-            s_plog[fr] = a.fh[fr].dof * r.posbnd_logfactor;
-            s_blog[fr] = frame_blog(a.fh[fr], r.badradar_logfactor);
-            s_flag[fr] = (r.outbnd ? 1 : 0) | (frame_bad(a.fh[fr], r.badradar) ? 2 : 0);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (use_sm)
-        summary_totals(a, [&](int f, double &c, double &pl, double &bl, int &fl) {
-            c = s_chi2[f]; pl = s_plog[f]; bl = s_blog[f]; fl = s_flag[f];
-        });
-    else
-        summary_totals(a, [&](int f, double &c, double &pl, double &bl, int &fl) {
-            const shape_deldop_result &r = a.results[f];
-            c = r.chi2;
-            pl = a.fh[f].dof * r.posbnd_logfactor;
-            bl = frame_blog(a.fh[f], r.badradar_logfactor);
-            fl = (r.outbnd ? 1 : 0) | (frame_bad(a.fh[f], r.badradar) ? 2 : 0);
-        });
-}
-
-// The totals: serial sums over the sets in dataset order (the reference's
-// order, src/shape/chi2.c:270-300 and calc_fits.c:407-409), the flags and
-// the objective. term(f, chi2, dof*posbnd_logfactor, dof*badradar_logfactor,
-// flags) gives radar frame f's terms (flags: 1 outbnd, 2 badradar).
-template <typename Term>
-__device__ void summary_totals(const SummaryArgs &a, Term term)
-{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
     double chi2 = 0.0, chi2_dd = 0.0, chi2_lc = 0.0, chi2_ps = 0.0, plog = 0.0, blog = 0.0, pslog = 0.0;
     int posbnd = 0, badradar = 0, badposet = 0;
     for (int s = 0; s < a.nsets; s++) {
-        const SetRec &R = a.sets[s];
+        const SetRec R = a.sets[s];
         double cs = 0.0;
         if (R.type == 2) {
             // plane-of-sky frames: chi2_poset's frame sum; calc_poset's
@@ -1095,13 +961,22 @@ __device__ void summary_totals(const SummaryArgs &a, Term term)
             }
             chi2_ps += cs;
         } else if (R.type == 0) {
-            for (int f = R.first; f < R.first + R.count; f++) {
-                double c, pl, bl;
-                int fl;
-                term(f, c, pl, bl, fl);
-                cs += c;
-                if (fl & 1) { posbnd = 1; plog += pl; }
-                if (fl & 2) { badradar = 1; blog += bl; }
+            for (int f0 = 0; f0 < R.count; f0 += 32) {
+                const int nb = min(32, R.count - f0), f = R.first + f0 + min(lane, nb - 1);
+                const shape_deldop_result *r = a.results + f;
+                const FrameHost &h = a.fh[f];
+                const double c = __ldcg(&r->chi2);
+                const bool out = lane < nb && __ldcg(&r->outbnd), bad = lane < nb && frame_bad(h, __ldcg(&r->badradar));
+                const unsigned mo = __ballot_sync(full, out), mb = __ballot_sync(full, bad);
+                double pl = 0.0, bl = 0.0;
+                if (mo) pl = h.dof * __ldcg(&r->posbnd_logfactor);
+                if (mb) bl = frame_blog(h, __ldcg(&r->badradar_logfactor));
+#pragma unroll 8
+                for (int k = 0; k < nb; k++) cs += __shfl_sync(full, c, k);
+                for (unsigned m = mo; m; m &= m - 1) plog += __shfl_sync(full, pl, __ffs(m) - 1);
+                for (unsigned m = mb; m; m &= m - 1) blog += __shfl_sync(full, bl, __ffs(m) - 1);
+                posbnd |= mo != 0;
+                badradar |= mb != 0;
             }
             chi2_dd += cs;
         } else {
@@ -1113,6 +988,7 @@ __device__ void summary_totals(const SummaryArgs &a, Term term)
         }
         chi2 += cs;
     }
+    if (lane != 0) return;
     shape_eval_summary out;
     out.chi2 = chi2;
     out.dof = a.dof;
@@ -1135,137 +1011,166 @@ __device__ void summary_totals(const SummaryArgs &a, Term term)
     *a.out = out;
 }
 
-// One item's chi-square partial sums, left by lane 0 of the calling warp in
-// part[0..5]: each lane sums its 16 bins (lane, lane + 32, ...) in order in
-// plain FP64, then the lanes' sums merge with compensation by warp shuffles
-// (pairwise: l with l+16, l+8, ..., l+1). With a.o2pre set, o2 is the item's
-// precomputed partial and obs / 1/var are read only where the fit is
-// nonzero: a zero fit bin adds exact zeros to m2 and om, so the sums keep
-// their values.
-template <typename T>
-__device__ void chi2_item_warp(const Chi2Args &a, int it, const Chi2Item &item, double *part)
+// The totals of an engine without radar frames.
+__global__ void k_totals(SummaryArgs a)
 {
-    const int lane = threadIdx.x & 31;
-    const long long base = item.base;
-    const T *fit = static_cast<const T *>(a.fit) + base;
-    const double *obs = a.obs + base, *oov = a.oov + base;
-    const bool pre = a.o2pre != nullptr;
-    if (pre && item.view >= 0) {
-        // no footprint reaches the item's rows: its fit is zero
-        const FrameState &st = a.states[item.view];
-        if (item.row1 < st.idellim[0] || item.row0 > st.idellim[1]) {
-            if (lane < 2) part[lane] = a.o2pre[2 * (size_t)it + lane];
-            else if (lane < 6) part[lane] = 0.0;
-            return;
+    grid_dep_wait();
+    totals_warp(a);
+}
+
+// One item's sums of m2 = fit^2/var and om = fit obs/var, left in m2 and om of
+// thread 0 of the block with their compensations. The item is a share of
+// the frame's lit box, the rows and columns that its footprints reach (the
+// union over a smeared frame's views): outside it the fit is zero and adds
+// nothing. Each thread sums its bins in order in plain FP64, then the threads'
+// sums merge with compensation in a fixed order.
+struct Chi2Frame {                             // a frame's constants
+    int view, nviews, nitems, ndel, ndop, dop1d;
+    long long base;
+};
+template <typename T>
+__device__ void chi2_item(const Chi2Args &a, const Chi2Frame &h, const FrameState *states, int k, KSum &m2, KSum &om)
+{
+    constexpr int U = 4;                       // bins a thread keeps in flight
+    const int tid = threadIdx.x, lane = tid & 31;
+    __shared__ double red[CHI2_THREADS / 32][4];
+    int r0 = INT_MAX, r1 = INT_MIN, c0 = INT_MAX, c1 = INT_MIN;
+    for (int v = h.view - h.nviews + 1; v <= h.view; v++) {
+        const FrameState &st = states[v];
+        r0 = min(r0, st.idellim[0]); r1 = max(r1, st.idellim[1]);
+        c0 = min(c0, st.idoplim[0]); c1 = max(c1, st.idoplim[1]);
+    }
+    r0 = max(r0, 1); r1 = min(r1, h.ndel); c0 = max(c0, 1); c1 = min(c1, h.ndop);
+    const int C = c1 - c0 + 1;
+    const int n = (r1 >= r0 && C > 0) ? (r1 - r0 + 1) * C : 0;
+    const int share = (n + h.nitems - 1) / h.nitems;
+    const int b0 = k * share, b1 = min(n, b0 + share);
+    // a spectrum of the FP32 form is summed in FP64 and rounded once, here
+    const bool spectrum = sizeof(T) == 4 && h.dop1d;
+    double sm2 = 0.0, som = 0.0;
+    if (b0 + tid < b1) {
+        int row = (b0 + tid) / C, col = (b0 + tid) - row * C;
+        const int drow = CHI2_THREADS / C, dcol = CHI2_THREADS - drow * C;
+        for (int b = b0 + tid; b < b1; b += CHI2_THREADS * U) {
+            double f[U], ob[U], wv[U];
+#pragma unroll
+            for (int j = 0; j < U; j++) {
+                const bool in = b + CHI2_THREADS * j < b1;
+                const long long p = h.base + (long long)(r0 - 1 + row) * h.ndop + (c0 - 1 + col);
+                f[j] = ob[j] = wv[j] = 0.0;
+                if (in) {
+                    if (spectrum) {
+                        const float v = (float)a.fit64[p];
+                        static_cast<float *>(a.fit)[p] = v;
+                        f[j] = v;
+                    } else {
+                        f[j] = (double)static_cast<const T *>(a.fit)[p];
+                    }
+                    ob[j] = a.obs[p];
+                    wv[j] = a.oov[p];
+                }
+                row += drow;
+                col += dcol;
+                if (col >= C) { col -= C; row++; }
+            }
+#pragma unroll
+            for (int j = 0; j < U; j++) {
+                sm2 += f[j] * f[j] * wv[j];
+                som += f[j] * ob[j] * wv[j];
+            }
         }
     }
-    T ft[CHI2_LANE];
-#pragma unroll
-    for (int j = 0; j < CHI2_LANE; j++) {
-        const int k = lane + 32 * j;
-        ft[j] = (k < item.count) ? fit[k] : (T)0;
-    }
-    double ob[CHI2_LANE], wv[CHI2_LANE];
-#pragma unroll
-    for (int j = 0; j < CHI2_LANE; j++) {
-        const int k = lane + 32 * j;
-        const bool in = (k < item.count) && (!pre || ft[j] != (T)0);
-        ob[j] = in ? obs[k] : 0.0;
-        wv[j] = in ? oov[k] : 0.0;
-    }
-    double so2 = 0.0, sm2 = 0.0, som = 0.0;
-#pragma unroll
-    for (int j = 0; j < CHI2_LANE; j++) {
-        if (lane + 32 * j >= item.count) break;
-        const double f = (double)ft[j];
-        if (!pre) so2 += ob[j] * ob[j] * wv[j];
-        sm2 += f * f * wv[j];
-        som += f * ob[j] * wv[j];
-    }
-    KSum o2 = {so2, 0}, m2 = {sm2, 0}, om = {som, 0};
+    m2 = KSum{sm2, 0};
+    om = KSum{som, 0};
     for (int off = 16; off > 0; off >>= 1) {
-        o2.merge(shfl_ksum(o2, off));
         m2.merge(shfl_ksum(m2, off));
         om.merge(shfl_ksum(om, off));
     }
     if (lane == 0) {
-        if (pre) {
-            o2.s = a.o2pre[2 * (size_t)it];
-            o2.c = a.o2pre[2 * (size_t)it + 1];
-        }
-        part[0] = o2.s; part[1] = o2.c;
-        part[2] = m2.s; part[3] = m2.c;
-        part[4] = om.s; part[5] = om.c;
+        double *r = red[tid >> 5];
+        r[0] = m2.s; r[1] = m2.c; r[2] = om.s; r[3] = om.c;
+    }
+    __syncthreads();
+    if (tid >= 32) return;
+    const int w = lane & (CHI2_THREADS / 32 - 1);
+    m2 = KSum{red[w][0], red[w][1]};
+    om = KSum{red[w][2], red[w][3]};
+    for (int off = CHI2_THREADS / 64; off > 0; off >>= 1) {
+        m2.merge(shfl_ksum(m2, off));
+        om.merge(shfl_ksum(om, off));
     }
 }
 
-// Chi-square partials, per-frame results and totals in one launch, warp by
-// warp with no block barrier: each warp takes (frame, 512-bin) items in
-// grid-stride order. A frame's counter takes one count per item; the warp
-// that makes the frame's last count merges the frame's item partials
-// (frame_sums_warp, the order k_summary's frame_sums_serial reproduces) and
-// writes the frame's chi-square terms (the warp of its first item has written
-// the limits, flags and log-factors), and the warp that completes the last frame computes the totals in
-// dataset order, as k_chi2_partials + k_summary do. Values another warp
-// wrote in this launch are read through L2 (__ldcg) after a fence.
+// Chi-square partials, per-frame results and totals in one launch: a block per
+// (frame, item). A frame's counter takes one count per item; the block that
+// makes the frame's last count merges the frame's item partials and writes its
+// chi-square terms (a block of its own has written the limits, flags and
+// log-factors, and a Doppler frame's overflow terms), and the one that completes the last frame computes the totals in dataset order. Values another
+// block wrote in this launch are read through L2 (__ldcg) after a fence.
 // counters: [nframes] per frame, then the finished frames; zero before the
 // launch.
+//
+// What bounds it is the chain of dependent loads, fences and counts, not the
+// images: a warp per item of 512 bins of the whole image read 12.5 MB of 64
+// frames for their 5 % of lit bins and counted 6100 times (stage 23 us); a block
+// per share of the lit box counts 500 times (17 us).
 template <typename T>
-__global__ void __launch_bounds__(CHI2_THREADS, CHI2_MIN_BLOCKS) k_chi2_summary(Chi2Args ca, FinalizeArgs fa, SummaryArgs sa,
+__global__ void __launch_bounds__(CHI2_THREADS) k_chi2_summary(Chi2Args ca, FinalizeArgs fa, SummaryArgs sa,
                                                                int *counters)
 {
-    extern __shared__ __align__(16) unsigned char stage[];   // chi2_summary_smem bytes (the totals)
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    int it = blockIdx.x * wpb + (threadIdx.x >> 5);
-    Chi2Item item = ca.items[min(it, ca.nitems - 1)];         // constant data: read before the wait
+    const int lane = threadIdx.x & 31, it = blockIdx.x;
+    // constant data: read before the wait
+    const int2 item = ca.items[it];
+    const int fr = item.x;
+    const FrameHost &h = fa.fh[fr];
+    const KSum o2pre = {ca.o2[2 * fr], ca.o2[2 * fr + 1]};
+    const int nitems = h.nitems, item0 = h.item0;
+    const FrameGeom &g = fa.geoms[h.view];
+    const Chi2Frame cf = {h.view, h.nviews, nitems, g.ndel, g.ndop, g.dop1d, g.fit_base};
     grid_dep_wait();
-    for (; it < ca.nitems; it += gridDim.x * wpb, item = ca.items[min(it, ca.nitems - 1)]) {
-        chi2_item_warp<T>(ca, it, item, ca.partials + (size_t)it * 6);
-        const int fr = item.frame;
-        const FrameHost &h = fa.fh[fr];
-        if (it == h.item0 && lane == 0) finalize_frame_geom(fa, fr, fa.results[fr]);
-        int last = 0;
-        __syncwarp();                                         // a skipped item's lanes wrote its partials
-        if (lane == 0) {
-            __threadfence();                                  // the partials before the count
-            last = (atomicAdd(&counters[fr], 1) == h.nitems - 1);
-        }
-        last = __shfl_sync(full, last, 0);
-        if (!last) continue;                                  // warp-uniform
-        __threadfence();
-        double start[3];
-        frame_start(fa, h, start);
-        KSum q[3];
-        frame_sums_warp(ca.partials + (size_t)h.item0 * 6, h.nitems, start, q, true);
-        int lastf = 0;
-        if (lane == 0) {
-            frame_chi2_from_sums(h, q, fa.results[fr]);
-            __threadfence();                                  // the results before the count
-            lastf = (atomicAdd(&counters[fa.nframes], 1) == fa.nframes - 1);
-        }
-        lastf = __shfl_sync(full, lastf, 0);
-        if (!lastf) continue;
-        // the totals: this warp stages every frame's terms in shared memory
-        // (the only warp of the grid that uses it), then lane 0 sums them in
-        // dataset order
-        __threadfence();
-        double *s_chi2 = reinterpret_cast<double *>(stage);
-        double *s_plog = s_chi2 + fa.nframes, *s_blog = s_plog + fa.nframes;
-        unsigned char *s_flag = reinterpret_cast<unsigned char *>(s_blog + fa.nframes);
-        for (int f = lane; f < fa.nframes; f += 32) {
-            const shape_deldop_result *r = fa.results + f;
-            s_chi2[f] = __ldcg(&r->chi2);
-            s_plog[f] = fa.fh[f].dof * __ldcg(&r->posbnd_logfactor);
-            s_blog[f] = frame_blog(fa.fh[f], __ldcg(&r->badradar_logfactor));
-            s_flag[f] = (__ldcg(&r->outbnd) ? 1 : 0) | (frame_bad(fa.fh[f], __ldcg(&r->badradar)) ? 2 : 0);
-        }
+    KSum m2 = {0, 0}, om = {0, 0};
+    if (item.y < 0) {
+        // the frame's geometry block
+        if (threadIdx.x >= 32) return;
+        if (h.dop_index >= 0) doppler_overflow_warp(fa, h);
         __syncwarp();
-        if (lane == 0)
-            summary_totals(sa, [&](int f, double &c, double &pl, double &bl, int &fl) {
-                c = s_chi2[f]; pl = s_plog[f]; bl = s_blog[f]; fl = s_flag[f];
-            });
+        if (lane == 0) finalize_frame_geom(fa, fr, fa.results[fr]);
+    } else {
+        chi2_item<T>(ca, cf, fa.states, item.y, m2, om);
+        if (threadIdx.x >= 32) return;
     }
+    int last = 0;
+    if (lane == 0) {
+        double *part = ca.partials + 4 * (size_t)it;
+        part[0] = m2.s; part[1] = m2.c; part[2] = om.s; part[3] = om.c;
+        __threadfence();                                      // the partials before the count
+        last = (atomicAdd(&counters[fr], 1) == nitems);       // the shares and the geometry
+    }
+    last = __shfl_sync(full, last, 0);
+    if (!last) return;                                        // warp-uniform
+    __threadfence();
+    frame_sums_warp(ca.partials + 4 * (size_t)item0, nitems, m2, om);
+    int lastf = 0;
+    if (lane == 0) {
+        // a Doppler frame's sums start from its overflow spectrum's o2 and m2
+        // (src/shape/chi2.c:745-747)
+        KSum so2 = o2pre, sm2 = m2;
+        if (h.dop_index >= 0) {
+            const double *ovf = fa.ovf_out + (size_t)h.dop_index * DOP_OVF_TERMS;
+            so2 = KSum{__ldcg(ovf), 0};
+            so2.merge(o2pre);
+            sm2 = KSum{__ldcg(ovf + 1), 0};
+            sm2.merge(m2);
+        }
+        frame_chi2_from_sums(h, so2, sm2, om, fa.results[fr]);
+        __threadfence();                                      // the results before the count
+        lastf = fa.nframes == 1 || atomicAdd(&counters[fa.nframes], 1) == fa.nframes - 1;
+    }
+    lastf = __shfl_sync(full, lastf, 0);
+    if (!lastf) return;
+    __threadfence();
+    totals_warp(sa);
 }
 
 }  // namespace
@@ -1332,41 +1237,11 @@ void launch_bin_f64(const FrameGeom *g, int view0, int nviews, const ModelDev &m
 }
 
 
-void launch_chi2_partials(const Chi2Args &a, int fp32, cudaStream_t s)
+void launch_frame_o2(const FrameHost *fh, int nframes, const FrameGeom *geoms, const double *obs, const double *oov,
+                     double *o2, cudaStream_t s)
 {
-    const int wpb = CHI2_THREADS / 32;               // one warp per item
-    const int need = (a.nitems + wpb - 1) / wpb;
-    int blocks = need < 8 * 148 ? need : 8 * 148;
-    if (blocks <= 0) return;
-    if (fp32) k_chi2_partials<float><<<blocks, CHI2_THREADS, 0, s>>>(a);
-    else k_chi2_partials<double><<<blocks, CHI2_THREADS, 0, s>>>(a);
+    if (nframes > 0) k_frame_o2<<<nframes, 256, 0, s>>>(fh, geoms, obs, oov, o2);
 }
-
-// FP32 form: each Doppler frame's FP64 sums rounded once into its float
-// fit bins.
-__global__ void k_dop_fit_f32(const int *dop_frames, const FrameHost *fh, const FrameGeom *geoms,
-                              const double *fit64, float *fit32)
-{
-    grid_dep_trigger();
-    grid_dep_wait();
-    const FrameGeom &g = geoms[fh[dop_frames[blockIdx.x]].view];
-    const long long n = (long long)g.ndel * g.ndop;
-    for (long long j = threadIdx.x; j < n; j += blockDim.x) fit32[g.fit_base + j] = (float)fit64[g.fit_base + j];
-}
-
-void launch_dop_fit_f32(const int *dop_frames, int n, const FrameHost *fh, const FrameGeom *geoms,
-                        const double *fit64, float *fit32, cudaStream_t s, bool pdl)
-{
-    if (n <= 0) return;
-    launch_k(k_dop_fit_f32, dim3(n), dim3(256), 0, s, pdl, dop_frames, fh, geoms, fit64, fit32);
-}
-
-void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s, bool pdl)
-{
-    if (a.n <= 0) return;
-    launch_k(k_doppler_overflow, dim3(a.n), dim3(256), 0, s, pdl, a);
-}
-
 
 void launch_poset_frames(const PosetArgs &a, cudaStream_t s, bool pdl)
 {
@@ -1395,53 +1270,18 @@ void launch_lc_finalize(const LcFinalizeArgs &a, cudaStream_t s, bool pdl)
     launch_k(k_lc_finalize, dim3(a.nsets), dim3(1024), a.smem_per_set, s, pdl, a);
 }
 
-// Shared memory of the summary: per-frame terms, then (when they fit) the
-// chi-square partials; *with_partials tells which.
-size_t summary_smem(int nframes, int nitems, int *with_partials)
-{
-    size_t b = 3 * sizeof(double) * (size_t)nframes + (size_t)nframes;   // terms and flags
-    size_t bp = ((b + 15) & ~(size_t)15) + 6 * sizeof(double) * (size_t)nitems;
-    *with_partials = bp <= SUMMARY_SMEM_MAX;
-    if (*with_partials) return bp;
-    return b <= SUMMARY_SMEM_MAX ? b : 0;
-}
-
-cudaError_t configure_summary()
-{
-    return cudaFuncSetAttribute(k_summary, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SUMMARY_SMEM_MAX);
-}
-
-size_t chi2_summary_smem(int nframes, int max_frame_items)
-{
-    (void)max_frame_items;          // a frame's partials merge in registers
-    return ((size_t)nframes * 25 + 15) & ~(size_t)15;
-}
-
-bool chi2_summary_fits(int nframes, int max_frame_items)
-{
-    return nframes > 0 && chi2_summary_smem(nframes, max_frame_items) <= FUSED_STAGE_BYTES;
-}
-
 void launch_chi2_summary(const Chi2Args &ca, const FinalizeArgs &fa, const SummaryArgs &sa, int *counters,
-                         int fp32, cudaStream_t s, bool pdl, size_t smem)
+                         int fp32, cudaStream_t s, bool pdl)
 {
-    const int wpb = CHI2_THREADS / 32;               // one warp per item
-    const int need = (ca.nitems + wpb - 1) / wpb;
-    const int blocks = need < 8 * 148 ? need : 8 * 148;
-    if (blocks <= 0 || ca.nitems <= 0) return;
-    if (fp32) launch_k(k_chi2_summary<float>, dim3(blocks), dim3(CHI2_THREADS), smem, s, pdl, ca, fa, sa, counters);
-    else launch_k(k_chi2_summary<double>, dim3(blocks), dim3(CHI2_THREADS), smem, s, pdl, ca, fa, sa, counters);
+    const int blocks = ca.nitems;                    // one block per item
+    if (blocks <= 0) return;
+    if (fp32) launch_k(k_chi2_summary<float>, dim3(blocks), dim3(CHI2_THREADS), 0, s, pdl, ca, fa, sa, counters);
+    else launch_k(k_chi2_summary<double>, dim3(blocks), dim3(CHI2_THREADS), 0, s, pdl, ca, fa, sa, counters);
 }
 
-void launch_summary(const FinalizeArgs &fa, const SummaryArgs &a, cudaStream_t s, bool pdl)
+void launch_totals(const SummaryArgs &a, cudaStream_t s, bool pdl)
 {
-    SummaryArgs b = a;
-    int wp = 0;
-    const size_t sm = summary_smem(fa.nframes, a.nitems, &wp);
-    b.smem_frames = (sm > 0 && fa.nframes > 0) ? 1 : 0;
-    b.smem_partials = b.smem_frames && wp;
-    launch_k(k_summary, dim3(1), dim3(256), b.smem_frames ? sm : 0, s, pdl, fa, b);
+    launch_k(k_totals, dim3(1), dim3(32), 0, s, pdl, a);
 }
-
 
 }  // namespace shape

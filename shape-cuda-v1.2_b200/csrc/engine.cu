@@ -203,27 +203,15 @@ int EngineImpl::finalize()
             if (g.dop1d) dop_frames.push_back(fi);
             frame_view.push_back(h.view);
             h.item0 = (int)chi2_items.size();
-            int D = F.ndel * F.ndop, chunk = CHI2_ITEM;
-            for (int st = 0; st < D; st += chunk)
-            {
-                const int cnt = std::min(chunk, D - st);
-                chi2_items.push_back(Chi2Item{fi, cnt, st / F.ndop + 1, (st + cnt - 1) / F.ndop + 1,
-                                              nview > 1 ? -1 : h.view, 0, g.fit_base + st});
-            }
-            h.nitems = (int)chi2_items.size() - h.item0;
+            // a block of 256 threads per 2048 bins, at most 8: a share of the lit
+            // box is then a few bins a thread
+            const int shares = std::max(1, std::min(8, (F.ndel * F.ndop + 2047) / 2048));
+            for (int k3 = 0; k3 < shares; k3++) chi2_items.push_back(make_int2(fi, k3));
+            h.nitems = shares;
+            chi2_items.push_back(make_int2(fi, -1));       // limits, flags, log-factors
             fh.push_back(h);
             add_view(g, F.pos_n, F.km_per_pixel);
         }
-    }
-    {
-        // the fused chi-square / summary kernel needs every frame to own an
-        // item and its staging buffer to hold a frame's partials and the
-        // per-frame terms
-        int max_items = 0;
-        bool every = true;
-        for (const FrameHost &h : fh) { max_items = std::max(max_items, h.nitems); every = every && h.nitems > 0; }
-        fused_chi2 = every && !chi2_items.empty() && chi2_summary_fits((int)fh.size(), max_items);
-        fused_smem = fused_chi2 ? chi2_summary_smem((int)fh.size(), max_items) : 0;
     }
     // lightcurve points: two views each (src/shape/calc_fits.c:1634-1716);
     // a plane-of-sky frame is rendered the same way (calc_poset,
@@ -356,9 +344,9 @@ int EngineImpl::finalize()
     }
     AL(d_pos_f, (size_t)pos_elems);
     AL(d_seen, (size_t)nf);
-    AL(d_chi2_items, chi2_items.size()); AL(d_frame_view, frame_view.size());
-    AL(d_partials, chi2_items.size() * 6);
-    AL(d_o2pre, chi2_items.size() * 2);
+    AL(d_chi2_items, chi2_items.size());
+    AL(d_partials, chi2_items.size() * 4);
+    AL(d_o2, fh.size() * 2);
     AL(d_chi2_counters, fh.size() + 1);
     AL(d_fh, fh.size()); AL(d_results, fh.size());
     AL(d_set_delpp, set_delpp.size()); AL(d_set_doppp, set_doppp.size()); AL(d_dop_extra, dop_extra.size());
@@ -383,7 +371,6 @@ int EngineImpl::finalize()
     if (!dop_frames.empty()) {
         AL(d_ovf, dop_frames.size() * DOP_MAXOVERFLOW);
         AL(d_ovf_out, dop_frames.size() * DOP_OVF_TERMS);
-        AL(d_dop_frames, dop_frames.size());
     }
     size_t lc_tot_pts = points.size(), lc_tot_n = 0;
     for (auto &L : lc) lc_tot_n += L.set.n;
@@ -428,9 +415,7 @@ int EngineImpl::finalize()
         CK(cudaMemcpyAsync(d_oov, oov.data(), sizeof(double) * fit_elems, cudaMemcpyHostToDevice, s));
     }
     if (!chi2_items.empty()) {
-        CK(cudaMemcpyAsync(d_chi2_items, chi2_items.data(), sizeof(Chi2Item) * chi2_items.size(),
-                           cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(d_frame_view, frame_view.data(), sizeof(int) * frame_view.size(),
+        CK(cudaMemcpyAsync(d_chi2_items, chi2_items.data(), sizeof(int2) * chi2_items.size(),
                            cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_fh, fh.data(), sizeof(FrameHost) * fh.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_set_delpp, set_delpp.data(), sizeof(double) * set_delpp.size(),
@@ -440,20 +425,8 @@ int EngineImpl::finalize()
         CK(cudaMemcpyAsync(d_dop_extra, dop_extra.data(), sizeof(double) * dop_extra.size(),
                            cudaMemcpyHostToDevice, s));
     }
-    if (!chi2_items.empty()) {
-        // o2 = sum obs^2/var of each item depends on the data only: summed
-        // once here by the evaluation's own kernel and order, then kept
-        CK(cudaMemsetAsync(d_fit64, 0, sizeof(double) * fit_elems, s));
-        Chi2Args c0;
-        memset(&c0, 0, sizeof c0);
-        c0.items = d_chi2_items; c0.nitems = (int)chi2_items.size();
-        c0.obs = d_obs; c0.oov = d_oov; c0.fit = d_fit64;
-        c0.states = d_states; c0.partials = d_partials;
-        c0.o2pre = nullptr;
-        launch_chi2_partials(c0, 0, s);
-        CK(cudaMemcpy2DAsync(d_o2pre, 2 * sizeof(double), d_partials, 6 * sizeof(double), 2 * sizeof(double),
-                             chi2_items.size(), cudaMemcpyDeviceToDevice, s));
-    }
+    launch_frame_o2(d_fh, (int)fh.size(), d_geoms, d_obs, d_oov, d_o2, s);
+    CK(cudaGetLastError());
     if (!lcpts.empty()) {
         CK(cudaMemcpyAsync(d_lcpts, lcpts.data(), sizeof(LcPointDev) * lcpts.size(), cudaMemcpyHostToDevice, s));
         size_t px = 0, pn = 0, ps_ = 0;
@@ -490,16 +463,12 @@ int EngineImpl::finalize()
             CK(cudaMemcpyAsync(d_ps_oov + b, H.oov.data(), sizeof(double) * H.oov.size(), cudaMemcpyHostToDevice, s));
         }
     }
-    if (!dop_frames.empty())
-        CK(cudaMemcpyAsync(d_dop_frames, dop_frames.data(), sizeof(int) * dop_frames.size(),
-                           cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(d_seen, 0, nf, s));
     CK(cudaStreamSynchronize(s));
 
     CK(configure_raster_f64());
     CK(configure_raster_f32());
     CK(configure_lc_finalize());
-    CK(configure_summary());
     md.nv = nv; md.nf = nf;
     md.a = d_a; md.u = d_u; md.r = d_r; md.scale = d_scale;
     md.vcomp = nullptr;
@@ -1099,7 +1068,6 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     // launch carries the vertex normals; the plain form and stage timing run
     // them one by one, from the uploaded parameters.
     const bool chain = (form != SHAPE_FORM_PLAIN_FP64) && !marks;
-    const bool fused = fused_chi2 && form != SHAPE_FORM_PLAIN_FP64;
     // the FP32 form sums Doppler spectra in FP64 (then rounds them once)
     const bool need64 = fit_elems && (!f32 || !dop_frames.empty());
     if (int rc = enqueue_spin()) return rc;
@@ -1117,7 +1085,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (f32 && fit_elems) clear(d_fit32, sizeof(float) * (size_t)fit_elems);
         if (need64) clear(d_fit64, sizeof(double) * (size_t)fit_elems);
         if (!dop_frames.empty()) clear(d_ovf, sizeof(double) * dop_frames.size() * DOP_MAXOVERFLOW);
-        if (fused) clear(d_chi2_counters, sizeof(int) * (fh.size() + 1));
+        clear(d_chi2_counters, sizeof(int) * (fh.size() + 1));
         if (!psf.empty()) clear(d_ps_count, sizeof(int) * psf.size());
         if (int rc_ = front_params(fr)) return rc_;
         launch_front(fr, s);
@@ -1132,7 +1100,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         CK(cudaMemsetAsync(d_seen, 0, nf, s));
         if (!dop_frames.empty())
             CK(cudaMemsetAsync(d_ovf, 0, sizeof(double) * dop_frames.size() * DOP_MAXOVERFLOW, s));
-        if (fused) CK(cudaMemsetAsync(d_chi2_counters, 0, sizeof(int) * (fh.size() + 1), s));
+        CK(cudaMemsetAsync(d_chi2_counters, 0, sizeof(int) * (fh.size() + 1), s));
         if (!psf.empty()) CK(cudaMemsetAsync(d_ps_count, 0, sizeof(int) * psf.size(), s));
         mark(1);
         if (int rc_ = launched("state reset")) return rc_;
@@ -1161,13 +1129,6 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     ra.keep_pos = keep_pos;
     ra.ovf = d_ovf;
 
-    Chi2Args ca;
-    ca.obs = d_obs; ca.oov = d_oov;
-    ca.fit = ra.fit;
-    ca.states = d_states;
-    ca.partials = d_partials;
-    ca.o2pre = d_o2pre;
-
     ra.pts = d_lcpts;
     ra.lc_part = d_lc_part;
     ra.bimg = d_ps_b;
@@ -1186,15 +1147,6 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
             rv.nwork = view_nwork[v];
             rv.mode = g.kind == VIEW_RADAR ? RASTER_RADAR : g.kind == VIEW_LC_SUN ? RASTER_MAPS : RASTER_PHOTO;
             launch_raster_f64(rv, s);
-            if (g.kind == VIEW_RADAR && fh[g.frame_index].view == v) {
-                const FrameHost &h = fh[g.frame_index];
-                Chi2Args cv = ca;
-                cv.items = d_chi2_items + h.item0;
-                cv.nitems = h.nitems;
-                cv.partials = d_partials + (size_t)h.item0 * 6;
-                cv.o2pre = d_o2pre + (size_t)h.item0 * 2;
-                launch_chi2_partials(cv, 0, s);
-            }
             if (int rc_ = launched(g.kind == VIEW_RADAR ? "radar view chain" : "lightcurve view chain")) return rc_;
         }
     } else {
@@ -1231,32 +1183,19 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
             if (k32) launch_raster_f32(rk, s);
             else launch_raster_f64(rk, s);
         }
-        if (f32) launch_dop_fit_f32(d_dop_frames, (int)dop_frames.size(), d_fh, d_geoms, d_fit64, d_fit32, s, pdl);
         mark(4);
         if (int rc_ = launched("raster")) return rc_;
-        ca.items = d_chi2_items;
-        ca.nitems = (int)chi2_items.size();
-        // fused: the chi-square partials run with the summary, last
-        if (!chi2_items.empty() && !fused) launch_chi2_partials(ca, f32 ? 1 : 0, s);
         mark(5);
-        if (int rc_ = launched("chi-square partials")) return rc_;
         mark(6);
     }
     FinalizeArgs fa;
     memset(&fa, 0, sizeof fa);
     fa.nframes = (int)fh.size();
-    fa.fh = d_fh; fa.geoms = d_geoms; fa.states = d_states; fa.partials = d_partials;
+    fa.fh = d_fh; fa.geoms = d_geoms; fa.states = d_states;
     fa.results = d_results; fa.set_delpp = d_set_delpp; fa.set_doppp = d_set_doppp;
     fa.dop_extra = d_dop_extra;
+    fa.ovf = d_ovf;
     fa.ovf_out = d_ovf_out;
-    if (!dop_frames.empty()) {
-        DopOvfArgs oa;
-        oa.n = (int)dop_frames.size();
-        oa.frames = d_dop_frames; oa.fh = d_fh; oa.geoms = d_geoms; oa.states = d_states;
-        oa.ovf = d_ovf; oa.out = d_ovf_out;
-        launch_doppler_overflow(oa, s, chain);
-        if (int rc_ = launched("Doppler overflow")) return rc_;
-    }
     if (!psf.empty()) {
         PosetArgs pa;
         pa.nframes = (int)psf.size();
@@ -1287,7 +1226,6 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     sa.lc_out = d_lc_out; sa.lc_dof = d_lc_dof; sa.lc_npts = d_lc_npts;
     sa.ps_res = d_ps_res; sa.ps_frames = d_psf; sa.dof_poset = dof_poset;
     sa.dof = dof; sa.dof_radar = dof_deldop + dof_doppler; sa.bad_objfactor = bad_objfactor;
-    sa.nitems = (int)chi2_items.size();
     // the bad-diameter factor depends only on host-side scale factors and is
     // applied by evaluate()
     sa.baddiam = 0;
@@ -1295,8 +1233,18 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     // the summary kernel writes the pinned host summary directly (mapped
     // memory), so an evaluation needs no device-to-host copy after it
     sa.out = d_summary_map;
-    if (fused) launch_chi2_summary(ca, fa, sa, d_chi2_counters, f32 ? 1 : 0, s, chain, fused_smem);
-    else launch_summary(fa, sa, s, chain && (!chi2_items.empty() || !lcdev.empty() || !psf.empty()));
+    if (fh.empty()) {
+        launch_totals(sa, s, chain);
+    } else {
+        Chi2Args ca;
+        ca.items = d_chi2_items; ca.nitems = (int)chi2_items.size();
+        ca.obs = d_obs; ca.oov = d_oov;
+        ca.fit = f32 ? (void *)d_fit32 : (void *)d_fit64;
+        ca.fit64 = d_fit64;
+        ca.partials = d_partials;
+        ca.o2 = d_o2;
+        launch_chi2_summary(ca, fa, sa, d_chi2_counters, f32 ? 1 : 0, s, chain);
+    }
     mark(7);
     CK(cudaGetLastError());
     return SHAPE_OK;
@@ -1311,19 +1259,14 @@ int EngineImpl::kernels_per_eval(int form) const
     int n = form == SHAPE_FORM_PLAIN_FP64 ? 3 : 2;
     n += (spin_device && n_spin_src > 0) ? 1 : 0;   // view realization from the spin state
     if (form == SHAPE_FORM_PLAIN_FP64) {
-        for (int v = 0; v < nviews; v++)
-            n += 3 + (geoms[v].kind == VIEW_RADAR && fh[geoms[v].frame_index].view == v ? 1 : 0);
+        n += 3 * nviews;
     } else {
         for (int k : work_n) n += k > 0;  // raster: radar, sun and observer views
-        if (form == SHAPE_FORM_BATCHED_FP32 && !dop_frames.empty())
-            n += 1;                      // FP32: Doppler spectra rounded from their FP64 sums
-        n += (chi2_items.empty() || fused_chi2) ? 0 : 1;   // fused: counted with the summary
     }
     n += lcdev.empty() ? 0 : 1;          // lightcurve finalize
     n += psf.empty() ? 0 : 1;            // plane-of-sky frames
-    n += dop_frames.empty() ? 0 : 1;     // Doppler overflow spectra
     n += pen_type.empty() ? 0 : (ncomp > 1 ? 3 : 2);   // model sums (and check_surface) for the penalties
-    return n + 1;                        // finalize + summary (with the chi-square partials when fused)
+    return n + 1;                        // chi-square, results and totals
 }
 
 // Every parameter to the device on the engine stream.

@@ -125,7 +125,7 @@ struct EngineImpl {
     std::vector<FrameHost> fh;
     std::vector<int2> work;                 // raster items
     std::vector<int> view_work0, view_nwork;
-    std::vector<Chi2Item> chi2_items;
+    std::vector<int2> chi2_items;
     std::vector<int> frame_view;
     std::vector<double> dop_extra, set_delpp, set_doppp;
     std::vector<LcPointDev> lcpts;
@@ -152,13 +152,10 @@ struct EngineImpl {
     void *d_pos_z = nullptr, *d_pos_cose = nullptr, *d_pos_cosi = nullptr;   // sized for double
     int *d_pos_f = nullptr;
     unsigned char *d_seen = nullptr;
-    Chi2Item *d_chi2_items = nullptr;
-    int *d_frame_view = nullptr;
+    int2 *d_chi2_items = nullptr;
     double *d_partials = nullptr;
-    double *d_o2pre = nullptr;        // per chi-square item: o2 partial (model independent)
-    int *d_chi2_counters = nullptr;   // fused chi-square / summary: per-frame items done, frames done
-    bool fused_chi2 = false;          // batched forms run k_chi2_summary
-    size_t fused_smem = 0;            // its dynamic shared memory
+    double *d_o2 = nullptr;           // per radar frame: sum obs^2 / var
+    int *d_chi2_counters = nullptr;   // per-frame items done, frames done
     FrameHost *d_fh = nullptr;
     shape_deldop_result *d_results = nullptr;
     double *d_set_delpp = nullptr, *d_set_doppp = nullptr, *d_dop_extra = nullptr;
@@ -185,7 +182,6 @@ struct EngineImpl {
     std::vector<LcSetDev> lcdev;
     std::vector<int> dop_frames;        // global indices of the Doppler frames
     double *d_ovf = nullptr, *d_ovf_out = nullptr;
-    int *d_dop_frames = nullptr;
 
     // penalty terms of the objective (shape_engine_set_penalties)
     std::vector<int> pen_type;

@@ -168,24 +168,17 @@ void launch_bin_f64(const FrameGeom *g, int view0, int nviews, const ModelDev &m
                     FrameState *st, int *bin_count, int2 *bin_ids, int cap, cudaStream_t s, bool pdl = false,
                     bool vnormals = false);
 
-// One chi-square item: count bins of a frame's image from element base of the
-// image arrays, lying in rows row0..row1 (1-based); view: the frame's view,
-// whose delay limits tell which rows hold footprints (-1: a smeared frame,
-// whose other views reach other rows).
-struct Chi2Item { int frame, count, row0, row1, view, pad; long long base; };
+// Chi-square items: (frame, share of its lit box) or (frame, -1) for its
+// geometry results, one block each.
 struct Chi2Args {
-    const Chi2Item *items;
+    const int2 *items;
     int nitems;
     const double *obs, *oov;
-    const void *fit;             // double or float
-    const FrameState *states;
-    double *partials;            // [nitems * 6]: o2, m2, om + compensations
-    // [nitems * 2]: each item's o2 partial (sum and compensation), computed
-    // once per dataset by the same code; null: o2 is summed per launch
-    const double *o2pre;
+    void *fit;                   // double or float
+    const double *fit64;         // FP32 form: the Doppler frames' FP64 sums
+    double *partials;            // [nitems * 4]: m2, om + compensations
+    const double *o2;            // [nframes * 2]: sum obs^2 / var and its compensation (launch_frame_o2)
 };
-void launch_chi2_partials(const Chi2Args &a, int fp32, cudaStream_t s);
-
 struct FrameHost {             // per radar frame constants for finalize
     double weight, dof, cal_in;
     int cal_floating, badradar;
@@ -208,31 +201,20 @@ struct FinalizeArgs {
     const FrameHost *fh;
     const FrameGeom *geoms;
     const FrameState *states;
-    const double *partials;
     shape_deldop_result *results;
     const double *set_delpp, *set_doppp;     // per set del/dop per pixel
     const double *dop_extra;                 // per frame
-    const double *ovf_out;                   // per Doppler frame: DOP_OVF_TERMS values
+    const double *ovf;                       // overflow spectra
+    double *ovf_out;                         // per Doppler frame: DOP_OVF_TERMS values
 };
 
-// Doppler overflow spectra (src/shape/pos2doppler.c:451-499): per Doppler
-// frame o2, m2, xsec, mean bin, and the badradar flag and log-factor of a
-// model wider than the overflow spectrum.
+// Doppler overflow terms per Doppler frame (src/shape/pos2doppler.c:451-499):
+// o2, m2, xsec, mean bin, and the badradar flag and log-factor of a model wider
+// than the overflow spectrum.
 constexpr int DOP_OVF_TERMS = 6;
-struct DopOvfArgs {
-    int n;                      // Doppler frames
-    const int *frames;          // their global radar frame indices
-    const FrameHost *fh;
-    const FrameGeom *geoms;
-    const FrameState *states;
-    const double *ovf;          // overflow spectra
-    double *out;                // [n * DOP_OVF_TERMS]
-};
-// FP32 form: the Doppler frames' FP64 sums rounded into the float fit
-// images the chi-square reads (one block per Doppler frame).
-void launch_dop_fit_f32(const int *dop_frames, int n, const FrameHost *fh, const FrameGeom *geoms,
-                        const double *fit64, float *fit32, cudaStream_t s, bool pdl);
-void launch_doppler_overflow(const DopOvfArgs &a, cudaStream_t s, bool pdl);
+// sum obs^2 / var of each radar frame
+void launch_frame_o2(const FrameHost *fh, int nframes, const FrameGeom *geoms, const double *obs, const double *oov,
+                     double *o2, cudaStream_t s);
 
 struct LcSetDev {
     int npts, n;                // calc points, observed points
@@ -328,26 +310,13 @@ struct SummaryArgs {
     int baddiam;
     double baddiam_logfactor;
     shape_eval_summary *out;
-    int nitems;                 // chi-square partial items (6 doubles each)
-    int smem_frames;            // set by launch_summary: per-frame terms staged in shared memory
-    int smem_partials;          // set by launch_summary: partials staged in shared memory too
 };
-constexpr size_t SUMMARY_SMEM_MAX = 160 * 1024;
-size_t summary_smem(int nframes, int nitems, int *with_partials);
-cudaError_t configure_summary();
-// per-frame finalize (as launch_finalize_frames) fused with the totals
-void launch_summary(const FinalizeArgs &fa, const SummaryArgs &a, cudaStream_t s, bool pdl);
-
-// Chi-square partials + per-frame finalize + totals in one launch (the
-// batched forms). Its shared staging (chi2_summary_smem bytes of dynamic
-// shared memory) holds one frame's partials and then every frame's terms;
-// chi2_summary_fits says whether a dataset fits in FUSED_STAGE_BYTES.
-constexpr size_t FUSED_STAGE_BYTES = 24 * 1024;
-size_t chi2_summary_smem(int nframes, int max_frame_items);
-bool chi2_summary_fits(int nframes, int max_frame_items);
-// counters: nframes + 1 ints, zero before the launch
+// Radar frames' chi-square, results and the totals; counters: nframes + 1 ints,
+// zero before the launch
 void launch_chi2_summary(const Chi2Args &ca, const FinalizeArgs &fa, const SummaryArgs &sa, int *counters,
-                         int fp32, cudaStream_t s, bool pdl, size_t smem);
+                         int fp32, cudaStream_t s, bool pdl);
+// the totals alone (no radar frames)
+void launch_totals(const SummaryArgs &a, cudaStream_t s, bool pdl);
 
 // raster_f64.cu / raster_f32.cu
 void launch_raster_f64(const RasterArgs &a, cudaStream_t s);

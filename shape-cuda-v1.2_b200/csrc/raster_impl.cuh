@@ -432,8 +432,7 @@ __device__ inline bool pixel_dd_scatter_lean(const RasterArgs &a, const FrameGeo
 #pragma unroll
     for (int c = 0; c < FAST_COLS; c++) {
         const T x = frac + (T)(i0 - c);        // exact to a T's rounding of its own size
-        const T r = quick_rcp(x);
-        pc[c] = (c < nc) ? r * r : (T)0;
+        pc[c] = (c < nc) ? quick_rcp(x * x) : (T)0;
         sdop += pc[c];
     }
     const T rl = (g.linlaw ? (sizeof(T) == 4 ? (T)g.famp : (T)g.amp) * cose
@@ -494,9 +493,9 @@ __device__ inline T stage_columns(const FrameGeom &g, const PixDD<T> &d, T *w)
 #pragma unroll
             for (int k = 0; k < NS * NS; k++) {
                 const T x = x0[k] + (T)(i0 - c);
-                const T r = quick_rcp(x);
+                const T r2 = quick_rcp(x * x);
                 // the reference's |pi x| > 1e-4
-                v += (fabs((T)3.141592653589793 * x) > (T)1.0e-4) ? s2[k] * r * r : (T)1;
+                v += (fabs((T)3.141592653589793 * x) > (T)1.0e-4) ? s2[k] * r2 : (T)1;
             }
             if (NS > 1) v = v / (NS * NS);
             sum += v;
