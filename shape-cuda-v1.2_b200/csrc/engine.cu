@@ -130,7 +130,9 @@ int EngineImpl::finalize()
         g.pos_base = pos_base;
         view_work0.push_back((int)work.size());
         view_nwork.push_back(g.tiles_x * g.tiles_x);
-        for (int t = 0; t < g.tiles_x * g.tiles_x; t++) work.push_back(make_int2((int)geoms.size(), t));
+        for (int t = 0; t < g.tiles_x * g.tiles_x; t++)
+            work.push_back(make_int4((int)geoms.size(), tile_base + t, -n + (t / g.tiles_x) * TILE_W,
+                                     -n + (t % g.tiles_x) * TILE_W));
         tile_base += g.tiles_x * g.tiles_x;
         pos_base += (long long)g.side * g.side;
         if (g.kind == VIEW_RADAR) radar_lean_consts(g, laws[g.law]);
@@ -409,7 +411,7 @@ int EngineImpl::finalize()
     CK(cudaMemcpyAsync(d_geoms, geoms.data(), sizeof(FrameGeom) * nviews, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(d_laws, laws.data(), sizeof(RadarLawDev) * std::max<size_t>(1, laws.size()),
                        cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(d_work, work.data(), sizeof(int2) * work.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(d_work, work.data(), sizeof(int4) * work.size(), cudaMemcpyHostToDevice, s));
     if (fit_elems) {
         CK(cudaMemcpyAsync(d_obs, obs.data(), sizeof(double) * fit_elems, cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(d_oov, oov.data(), sizeof(double) * fit_elems, cudaMemcpyHostToDevice, s));
@@ -1019,9 +1021,7 @@ int EngineImpl::tune_bins()
     std::vector<int> order(work.size());
     for (size_t k = 0; k < work.size(); k++) order[k] = (int)k;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-        int cx = counts[geoms[work[x].x].tile_base + work[x].y];
-        int cy = counts[geoms[work[y].x].tile_base + work[y].y];
-        return cx > cy;
+        return counts[work[x].y] > counts[work[y].y];
     });
     // radar tiles first, then sun-view tiles, then the observer views' that
     // read the sun views' maps, each part in decreasing count
@@ -1030,19 +1030,19 @@ int EngineImpl::tune_bins()
         return k == VIEW_RADAR ? 0 : k == VIEW_LC_SUN ? 1 : 2;
     };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return part(x) < part(y); });
-    std::vector<int2> sorted(work.size());
+    std::vector<int4> sorted(work.size());
     for (int k = 0; k < 3; k++) work_n[k] = work_busy[k] = 0;
     for (size_t k = 0; k < work.size(); k++) {
         sorted[k] = work[order[k]];
         const int w = part(order[k]);
         work_n[w]++;
-        work_busy[w] += counts[geoms[sorted[k].x].tile_base + sorted[k].y] > 0;
+        work_busy[w] += counts[sorted[k].y] > 0;
     }
     if (!d_work_sorted) {
         int rc = mem.alloc(&d_work_sorted, work.size());
         if (rc) return rc;
     }
-    CK(cudaMemcpyAsync(d_work_sorted, sorted.data(), sizeof(int2) * sorted.size(), cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(d_work_sorted, sorted.data(), sizeof(int4) * sorted.size(), cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));
     return SHAPE_OK;
 }

@@ -123,7 +123,7 @@ struct EngineImpl {
     // derived (host)
     std::vector<FrameGeom> geoms;
     std::vector<FrameHost> fh;
-    std::vector<int2> work;                 // raster items
+    std::vector<int4> work;                 // raster items (RasterArgs::work)
     std::vector<int> view_work0, view_nwork;
     std::vector<int2> chi2_items;
     std::vector<int> frame_view;
@@ -142,7 +142,7 @@ struct EngineImpl {
     FrameGeom *d_geoms = nullptr;
     FrameState *d_states = nullptr;
     RadarLawDev *d_laws = nullptr;
-    int2 *d_work = nullptr;
+    int4 *d_work = nullptr;
     double4 *d_vt64 = nullptr;
     int *d_bin_count = nullptr;
     int2 *d_bin_ids = nullptr;
@@ -294,7 +294,7 @@ struct EngineImpl {
         finalized = false;
     }
     // bin tuning results
-    int2 *d_work_sorted = nullptr;
+    int4 *d_work_sorted = nullptr;
     int tuned_max_count = 0, tuned_nonempty = 0;
     // the sorted work list holds radar, sun-view and observer-view tiles
     // (RASTER_*): tiles of each part, and its first ones non-empty at tuning

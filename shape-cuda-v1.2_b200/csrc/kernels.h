@@ -62,7 +62,10 @@ enum { RASTER_RADAR, RASTER_MAPS, RASTER_PHOTO };
 
 struct RasterArgs {
     const FrameGeom *geoms;
-    const int2 *work;          // (view, tile) items
+    // tiles: (view, index of the tile among all views', first pixel row, first
+    // pixel column); with the last three here, the tile's bin is read without
+    // waiting for the view's constants
+    const int4 *work;
     int nwork;                 // items
     int grid;                  // CTAs (0: one per item); fewer CTAs stride over the rest
     int pdl;                   // programmatic dependent launch (launch_k)

@@ -186,8 +186,9 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
         hfn[f] = make_double4(fn[3 * f], fn[3 * f + 1], fn[3 * f + 2], 0.0);
         hfv[f] = make_int4(fv[3 * f], fv[3 * f + 1], fv[3 * f + 2], 0);
     }
-    std::vector<int2> work(ntiles);
-    for (int t = 0; t < ntiles; t++) work[t] = make_int2(0, t);
+    std::vector<int4> work(ntiles);
+    for (int t = 0; t < ntiles; t++)
+        work[t] = make_int4(0, t, -n + (t / g.tiles_x) * TILE_W, -n + (t % g.tiles_x) * TILE_W);
     int rc = grow(c->vx, sizeof(double4) * nv);
     if (!rc) rc = grow(c->vn, sizeof(double4) * nv);
     if (!rc) rc = grow(c->vt, sizeof(double4) * nv);
@@ -196,7 +197,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     if (!rc) rc = grow(c->geom, sizeof(FrameGeom));
     if (!rc) rc = grow(c->state, sizeof(FrameState));
     if (!rc) rc = grow(c->bin_count, sizeof(int) * ntiles);
-    if (!rc) rc = grow(c->work, sizeof(int2) * ntiles);
+    if (!rc) rc = grow(c->work, sizeof(int4) * ntiles);
     if (!rc) rc = grow(c->z, sizeof(double) * P);
     if (!rc) rc = grow(c->ca, sizeof(double) * P);
     if (!rc) rc = grow(c->cb, sizeof(double) * P);
@@ -208,7 +209,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     PV_CK(cudaMemcpyAsync(c->fn.p, hfn.data(), sizeof(double4) * nf, cudaMemcpyHostToDevice, s));
     PV_CK(cudaMemcpyAsync(c->fvi.p, hfv.data(), sizeof(int4) * nf, cudaMemcpyHostToDevice, s));
     PV_CK(cudaMemcpyAsync(c->geom.p, &g, sizeof g, cudaMemcpyHostToDevice, s));
-    PV_CK(cudaMemcpyAsync(c->work.p, work.data(), sizeof(int2) * ntiles, cudaMemcpyHostToDevice, s));
+    PV_CK(cudaMemcpyAsync(c->work.p, work.data(), sizeof(int4) * ntiles, cudaMemcpyHostToDevice, s));
     // the images' current contents: each pixel starts from them
     PV_CK(cudaMemcpyAsync(c->z.p, Z, sizeof(double) * P, cudaMemcpyHostToDevice, s));
     PV_CK(cudaMemcpyAsync(c->ca.p, CA, sizeof(double) * P, cudaMemcpyHostToDevice, s));
@@ -246,7 +247,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     RasterArgs ra;
     memset(&ra, 0, sizeof ra);
     ra.geoms = dgeom;
-    ra.work = static_cast<const int2 *>(c->work.p);
+    ra.work = static_cast<const int4 *>(c->work.p);
     ra.nwork = ntiles;
     ra.vt = c->vt.p;
     ra.fvi = md.fvi;

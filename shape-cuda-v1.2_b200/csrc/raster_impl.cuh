@@ -986,18 +986,16 @@ k_raster(const __grid_constant__ RasterArgs a)
     const int tid = threadIdx.x, lane = tid & 31;
 
     for (int w = blockIdx.x; w < a.nwork; w += gridDim.x) {
-        const int2 item = a.work[w];
+        const int4 item = a.work[w];
+        const int tile = item.y, ti0 = item.z, tj0 = item.w;
+        const int2 *bin = a.bin_ids + (size_t)tile * a.cap;
+        const int count = a.bin_count[tile];
         const FrameGeom &g = a.geoms[item.x];
-        const int tile = item.y;
-        const int count = a.bin_count[g.tile_base + tile];
         const bool writes_pos = MAPS || a.keep_pos;
         if (count == 0 && !writes_pos) continue;
-        const int tx = tile / g.tiles_x, ty = tile % g.tiles_x;
         const int n = g.n;
-        const int ti0 = -n + tx * TILE_W, tj0 = -n + ty * TILE_W;
         const bool smooth = g.smooth != 0;
         const bool accumulate = MODE == RASTER_MAPS && a.accumulate;
-        const int2 *bin = a.bin_ids + (size_t)(g.tile_base + tile) * a.cap;
         const double4 *vt = static_cast<const double4 *>(a.vt) + g.vt_base;
 
         if (MAPS && count == 0) {
@@ -1020,7 +1018,7 @@ k_raster(const __grid_constant__ RasterArgs a)
                     if (bb >= 0) a.bimg[bb + (q - g.pos_base)] = 0.0;
                 }
             }
-            if (PHOTO && tid == 0) a.lc_part[g.tile_base + tile] = 0.0;
+            if (PHOTO && tid == 0) a.lc_part[tile] = 0.0;
             continue;
         }
         FrameState &S = a.states[item.x];
@@ -1201,7 +1199,7 @@ k_raster(const __grid_constant__ RasterArgs a)
             if (tid == 0) {
                 double v = 0.0;
                 for (int k = 0; k < NT / 32; k++) v += sh.pz[k];
-                a.lc_part[g.tile_base + tile] = v;
+                a.lc_part[tile] = v;
             }
         }
 
