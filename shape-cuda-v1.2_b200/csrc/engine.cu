@@ -1145,7 +1145,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
             RasterArgs rv = ra;
             rv.work = d_work + view_work0[v];
             rv.nwork = view_nwork[v];
-            rv.mode = g.kind == VIEW_RADAR ? RASTER_RADAR : g.kind == VIEW_LC_SUN ? RASTER_MAPS : RASTER_PHOTO;
+            rv.mode = g.kind == VIEW_RADAR ? RASTER_RADAR : g.kind == VIEW_LC_SUN ? RASTER_SUN : RASTER_PHOTO;
             launch_raster_f64(rv, s);
             if (int rc_ = launched(g.kind == VIEW_RADAR ? "radar view chain" : "lightcurve view chain")) return rc_;
         }

@@ -58,7 +58,7 @@ struct ModelDev {
 };
 
 // What a raster launch does with its views (k_raster).
-enum { RASTER_RADAR, RASTER_MAPS, RASTER_PHOTO };
+enum { RASTER_RADAR, RASTER_SUN, RASTER_PHOTO, RASTER_POS };
 
 struct RasterArgs {
     const FrameGeom *geoms;

@@ -264,7 +264,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     ra.pos_f = static_cast<int *>(c->f.p);
     ra.keep_pos = 1;
     ra.accumulate = 1;
-    ra.mode = RASTER_MAPS;
+    ra.mode = RASTER_POS;
     ra.won = static_cast<unsigned char *>(c->won.p);
     launch_raster_f64(ra, s);
     PV_CK(cudaGetLastError());

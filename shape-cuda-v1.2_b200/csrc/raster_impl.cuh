@@ -35,14 +35,18 @@
 #include "kernels.h"
 #include "posmask_dev.cuh"
 
-// Resident warps per SM that the register allocation must allow (FP32 /
-// FP64), and the share of the SM's 256 KB that the CTAs' shared memory may
+// Resident warps per SM that the register allocation must allow (radar views
+// FP32 / FP64, sun and observer views), and the share of the SM's 256 KB that the CTAs' shared memory may
 // take; the rest is L1, where the facets' vertices and the spills live. The
 // kernels wait on those loads more than they issue, so both count. 128-thread
 // CTAs, ms: 64 uneven frames in FP32 at 40 warps 0.106 with all of it shared
 // and 0.105 with 80 %, at 32 warps 0.104, 0.099 with 80 % and 0.099 with 65;
-// 800 lightcurve points in FP64 at 32 warps 1.73, 1.63 and 1.74, at 24 2.02,
-// 1.94 and 1.90; 16 frames of 511^2 0.222 and 0.214 at 40, 0.204 and 0.192 at 32.
+// 16 frames of 511^2 0.222 and 0.214 at 40, 0.204 and 0.192 at 32. The sun and
+// observer views hold less per tile (no synthesis; a sun view no shading
+// either): 800 points' both launches 1.52 at 32 warps, 1.38 at 40 and 1.35 at
+// 48, but 25 points' 0.067, 0.067 and 0.075 (48 leave them half a wave). One
+// share for all of them: a launch that changes it waits until the SM is empty
+// (25 points' evaluation 0.099 with one share, 0.107 with two).
 #ifndef RASTER_WARPS_F32
 #define RASTER_WARPS_F32 32
 #endif
@@ -51,6 +55,9 @@
 #endif
 #ifndef RASTER_WARPS_F64
 #define RASTER_WARPS_F64 32
+#endif
+#ifndef RASTER_WARPS_MAPS
+#define RASTER_WARPS_MAPS 40
 #endif
 
 namespace shape {
@@ -646,11 +653,11 @@ struct TileShared {
         StageRow<T> stage[NT];                       // phase C: a row per thread
     };
     double xs[TILE_W], ys[TILE_W];         // pixel centres
-    double pz[TILE_PIX];                   // radar views: the shaded pixels' depth and cos(e)
-    T pc[TILE_PIX];
     int cnt[TILE_PIX];                     // candidates (may exceed CAND)
-    unsigned more[CAND_MORE];              // further ones: entry | pixel << 16
-    int2 fl[NT];                           // slow path: the current chunk's facets
+    union {
+        unsigned more[CAND_MORE];          // further ones: entry | pixel << 16
+        int2 fl[NT];                       // slow path: the current chunk's facets
+    };
     unsigned long long lim[4];             // the frame's delay and Doppler extremes so far
     int cov[4];                            // ... and covered-pixel bbox
     int n;                                 // entries of more (may exceed CAND_MORE)
@@ -968,21 +975,34 @@ __device__ inline bool photo_shadowed(const RasterArgs &a, const FrameGeom &g, c
 }
 
 // MODE RASTER_RADAR: radar views, shading and delay-Doppler synthesis; POS maps
-// only when a.keep_pos asks for them. RASTER_MAPS (double only): sun views and
-// single POS views, shading and POS maps. RASTER_PHOTO (double only): the
-// observer views of lightcurve points and sky frames, after their sun views:
-// shading, shadows, photometry and POS maps; a tile's brightness goes to
-// a.lc_part. As a kernel of its own, which read the maps back, photometry took
-// 0.70 ms on 800 points after the raster's 1.58; the raster with it takes 1.73.
+// only when a.keep_pos asks for them. RASTER_SUN (double only, as the next two):
+// sun views, depth and facet maps; nothing reads their cosines, so nothing is
+// shaded. RASTER_PHOTO: the observer views of lightcurve points and sky frames,
+// after their sun views: shading, shadows, photometry and POS maps; a tile's
+// brightness goes to a.lc_part (as a kernel of its own, which read the maps
+// back, photometry took 0.70 ms on 800 points). RASTER_POS: single POS views,
+// shading and POS maps on top of what the images hold. 800 points' sun and
+// observer launches took 1.63 ms while sun views and single views were one
+// kernel, 1.52 apart (no spills, no shading) and 1.38 with the resident warps
+// that this allows.
+template <typename T, int MODE> __host__ __device__ constexpr int raster_warps()
+{
+    return MODE == RASTER_SUN || MODE == RASTER_PHOTO ? RASTER_WARPS_MAPS
+         : sizeof(T) == 4 ? RASTER_WARPS_F32 : RASTER_WARPS_F64;
+}
 template <typename T, int NT, int MODE>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? RASTER_WARPS_F32 : RASTER_WARPS_F64) * 32 / NT)
+__global__ void __launch_bounds__(NT, raster_warps<T, MODE>() * 32 / NT)
 k_raster(const __grid_constant__ RasterArgs a)
 {
     grid_dep_trigger();
     grid_dep_wait();
     constexpr int PP = TILE_PIX / NT;          // pixels per thread
-    constexpr bool MAPS = MODE != RASTER_RADAR, PHOTO = MODE == RASTER_PHOTO;
+    constexpr bool MAPS = MODE != RASTER_RADAR, SUN = MODE == RASTER_SUN, PHOTO = MODE == RASTER_PHOTO;
+    constexpr bool accumulate = MODE == RASTER_POS;
     __shared__ TileShared<T, NT> sh;
+    // radar views: the shaded pixels' depth and cos(e)
+    __shared__ double pz[MAPS ? NT / 32 : TILE_PIX];
+    __shared__ T pc[MAPS ? 1 : TILE_PIX];
     const int tid = threadIdx.x, lane = tid & 31;
 
     for (int w = blockIdx.x; w < a.nwork; w += gridDim.x) {
@@ -995,7 +1015,6 @@ k_raster(const __grid_constant__ RasterArgs a)
         if (count == 0 && !writes_pos) continue;
         const int n = g.n;
         const bool smooth = g.smooth != 0;
-        const bool accumulate = MODE == RASTER_MAPS && a.accumulate;
         const double4 *vt = static_cast<const double4 *>(a.vt) + g.vt_base;
 
         if (MAPS && count == 0) {
@@ -1004,13 +1023,13 @@ k_raster(const __grid_constant__ RasterArgs a)
                 const int p = tid + r * NT, pi = ti0 + p / TILE_W, pj = tj0 + p % TILE_W;
                 if (pi > n || pj > n) continue;
                 const long long q = g.pos_base + (long long)(pi + n) * g.side + (pj + n);
-                if (accumulate) {
+                if constexpr (accumulate) {
                     a.won[q] = 0;
                     continue;
                 }
                 static_cast<double *>(a.pos_z)[q] = -SHAPE_HUGENUMBER;
                 a.pos_f[q] = -1;
-                if (g.kind == VIEW_LC_SUN) continue;
+                if (SUN) continue;
                 static_cast<T *>(a.pos_cose)[q] = 0;
                 static_cast<T *>(a.pos_cosi)[q] = 0;
                 if constexpr (PHOTO) {
@@ -1097,9 +1116,9 @@ k_raster(const __grid_constant__ RasterArgs a)
                     if (j1 > sh.cov[3]) atomicMax(&S.cov_j[1], j1);
                 }
             }
-            const bool bistatic_obs = PHOTO || (MAPS && g.kind == VIEW_LC_OBS);
+            const bool bistatic_obs = PHOTO || (accumulate && g.kind == VIEW_LC_OBS);
             // nothing reads the sun view's cosines of a lightcurve or sky frame
-            const bool shade = covered && !(MAPS && g.kind == VIEW_LC_SUN && !accumulate);
+            const bool shade = !SUN && covered;
             const double z = covered ? h.z : -SHAPE_HUGENUMBER;
             const int fac = h.f;
             T cosa = 0, cosb = 0;
@@ -1181,24 +1200,24 @@ k_raster(const __grid_constant__ RasterArgs a)
                     Z[q] = z;
                     a.pos_f[q] = fac;
                 }
-                if (accumulate || g.kind != VIEW_LC_SUN) CE[q] = cosa;   // cos(i) in a sun view (pos->cosill)
-                if (g.kind != VIEW_LC_SUN) CI[q] = cosb;
+                if (!SUN) CE[q] = cosa;   // cos(i) in a sun view (pos->cosill)
+                if (!SUN && g.kind != VIEW_LC_SUN) CI[q] = cosb;
             }
             if constexpr (!MAPS) {
                 if (covered && a.mark_seen && !g.no_seen && (double)cosa > a.mincosine_seen) a.seen[fac] = 1;
-                sh.pz[p] = z;
-                sh.pc[p] = covered ? cosa : (T)0;
+                pz[p] = z;
+                pc[p] = covered ? cosa : (T)0;
             }
         }
 
         if constexpr (PHOTO) {
             // the tile's brightness, in a fixed order
             for (int off = 16; off > 0; off >>= 1) bsum += __shfl_down_sync(0xffffffffu, bsum, off);
-            if (lane == 0) sh.pz[tid >> 5] = bsum;
+            if (lane == 0) pz[tid >> 5] = bsum;
             __syncthreads();
             if (tid == 0) {
                 double v = 0.0;
-                for (int k = 0; k < NT / 32; k++) v += sh.pz[k];
+                for (int k = 0; k < NT / 32; k++) v += pz[k];
                 a.lc_part[tile] = v;
             }
         }
@@ -1212,14 +1231,14 @@ k_raster(const __grid_constant__ RasterArgs a)
             for (int r = 0; r < PP; r++) {
                 const int p = ((tid + r * NT) * 37 + 11) & (TILE_PIX - 1);
                 const int pi = ti0 + p / TILE_W, pj = tj0 + p % TILE_W;
-                const T cosa = sh.pc[p];
+                const T cosa = pc[p];
                 const bool lit = cosa > (T)0;
                 PixPos pp = {0.0, 0.0};
                 PixDD<T> dd;
                 dd.ok = false;
                 if (lit) {
-                    if constexpr (sizeof(T) == 4) dd = pixel_dd_setup_x(g, pi, pj, sh.pz[p], pp);
-                    else dd = pixel_dd_setup(g, pi, pj, sh.pz[p], pp);
+                    if constexpr (sizeof(T) == 4) dd = pixel_dd_setup_x(g, pi, pj, pz[p], pp);
+                    else dd = pixel_dd_setup(g, pi, pj, pz[p], pp);
                 }
                 // delay / Doppler extremes of the frame's lit pixels as dkey
                 // keys: reduced and added only by a warp that holds a value
@@ -1276,12 +1295,14 @@ k_raster(const __grid_constant__ RasterArgs a)
 }
 
 // variant 0: 256 threads per tile; 1: 128 (two pixels a thread, smaller CTAs).
-// f(kernel, threads) for the kernel that a's mode and variant select.
+// f(kernel, threads) for the kernel that a's mode and variant select (a single
+// POS view is one launch of a few tiles: 256 threads).
 template <typename T, typename F>
 inline void with_raster_kernel(const RasterArgs &a, F f)
 {
     if constexpr (sizeof(T) == 8) {
-        if (a.mode == RASTER_MAPS) return a.variant == 1 ? f(k_raster<T, 128, RASTER_MAPS>, 128) : f(k_raster<T, 256, RASTER_MAPS>, 256);
+        if (a.mode == RASTER_SUN) return a.variant == 1 ? f(k_raster<T, 128, RASTER_SUN>, 128) : f(k_raster<T, 256, RASTER_SUN>, 256);
+        if (a.mode == RASTER_POS) return f(k_raster<T, 256, RASTER_POS>, 256);
         if (a.mode == RASTER_PHOTO) return a.variant == 1 ? f(k_raster<T, 128, RASTER_PHOTO>, 128) : f(k_raster<T, 256, RASTER_PHOTO>, 256);
     }
     return a.variant == 1 ? f(k_raster<T, 128, RASTER_RADAR>, 128) : f(k_raster<T, 256, RASTER_RADAR>, 256);
@@ -1301,7 +1322,7 @@ inline cudaError_t configure_raster_t()
 {
     cudaError_t e = cudaSuccess;
     RasterArgs a = {};
-    for (a.mode = RASTER_RADAR; a.mode <= (sizeof(T) == 8 ? RASTER_PHOTO : RASTER_RADAR); a.mode++)
+    for (a.mode = RASTER_RADAR; a.mode <= (sizeof(T) == 8 ? RASTER_POS : RASTER_RADAR); a.mode++)
         for (a.variant = 0; a.variant < 2 && e == cudaSuccess; a.variant++)
             with_raster_kernel<T>(a, [&](auto kern, int) {
                 e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, RASTER_SHARED_PCT);
