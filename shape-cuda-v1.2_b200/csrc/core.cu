@@ -71,15 +71,14 @@ __device__ inline double4 realize_vertex(int i, const double *__restrict__ a, co
 
 // facet normal and area: facnrm (src/shape/facnrm.c:13-25), cross
 // (src/util/cross.c), normalize (src/util/normalize.c)
-__device__ inline void realize_facet(int f, const int *__restrict__ fv, double4 p0, double4 p1, double4 p2,
-                                     double4 *__restrict__ fn, double *__restrict__ area)
+__device__ inline double4 facet_normal(double4 p0, double4 p1, double4 p2, double *area)
 {
     double a0 = p1.x - p0.x, a1 = p1.y - p0.y, a2 = p1.z - p0.z;
     double b0 = p2.x - p1.x, b1 = p2.y - p1.y, b2 = p2.z - p1.z;
     double c0 = a1 * b2 - a2 * b1;
     double c1 = a2 * b0 - a0 * b2;
     double c2 = a0 * b1 - a1 * b0;
-    area[f] = 0.5 * sqrt(c0 * c0 + c1 * c1 + c2 * c2);
+    if (area) *area = 0.5 * sqrt(c0 * c0 + c1 * c1 + c2 * c2);
     double norm = 0.0;
     norm += c0 * c0;
     norm += c1 * c1;
@@ -88,7 +87,7 @@ __device__ inline void realize_facet(int f, const int *__restrict__ fv, double4 
     if (norm != 0.0) {
         c0 /= norm; c1 /= norm; c2 /= norm;
     }
-    fn[f] = make_double4(c0, c1, c2, 0.0);
+    return make_double4(c0, c1, c2, 0.0);
 }
 
 // Vertices and facets in one launch: threads [0, nf) realize a facet from
@@ -104,8 +103,8 @@ __device__ inline void realize_vf(int k, int nv, int nf, const double *__restric
     if (k < nf) {
         int i0 = fv[3 * k + 0], i1 = fv[3 * k + 1], i2 = fv[3 * k + 2];
         fvi[k] = make_int4(i0, i1, i2, 0);
-        realize_facet(k, fv, realize_vertex(i0, a, u, par, vcomp, cxf), realize_vertex(i1, a, u, par, vcomp, cxf),
-                      realize_vertex(i2, a, u, par, vcomp, cxf), fn, area);
+        fn[k] = facet_normal(realize_vertex(i0, a, u, par, vcomp, cxf), realize_vertex(i1, a, u, par, vcomp, cxf),
+                             realize_vertex(i2, a, u, par, vcomp, cxf), &area[k]);
     } else if (k < nf + nv) {
         vx[k - nf] = realize_vertex(k - nf, a, u, par, vcomp, cxf);
     }
@@ -122,15 +121,9 @@ __global__ void k_realize_vf(int nv, int nf, const double *__restrict__ a, const
 
 // vertex normal = normalized sum of attached facet normals, in af order
 // (src/shape/realize_mod.c:550-563)
-__device__ inline void realize_vnormal(int i, const int *__restrict__ af_ptr, const int *__restrict__ af_idx,
-                                       const double4 *__restrict__ fn, double4 *__restrict__ vn,
-                                       float4 *__restrict__ vnf)
+__device__ inline void store_vnormal(int i, double n0, double n1, double n2, double4 *__restrict__ vn,
+                                     float4 *__restrict__ vnf)
 {
-    double n0 = 0.0, n1 = 0.0, n2 = 0.0;
-    for (int j = af_ptr[i]; j < af_ptr[i + 1]; j++) {
-        double4 fnj = fn[af_idx[j]];
-        n0 += fnj.x; n1 += fnj.y; n2 += fnj.z;
-    }
     double norm = 0.0;
     norm += n0 * n0;
     norm += n1 * n1;
@@ -142,6 +135,17 @@ __device__ inline void realize_vnormal(int i, const int *__restrict__ af_ptr, co
     vn[i] = make_double4(n0, n1, n2, 0.0);
     if (vnf) vnf[i] = make_float4((float)n0, (float)n1, (float)n2, 0.0f);
 }
+__device__ inline void realize_vnormal(int i, const int *__restrict__ af_ptr, const int *__restrict__ af_idx,
+                                       const double4 *__restrict__ fn, double4 *__restrict__ vn,
+                                       float4 *__restrict__ vnf)
+{
+    double n0 = 0.0, n1 = 0.0, n2 = 0.0;
+    for (int j = af_ptr[i]; j < af_ptr[i + 1]; j++) {
+        double4 fnj = fn[af_idx[j]];
+        n0 += fnj.x; n1 += fnj.y; n2 += fnj.z;
+    }
+    store_vnormal(i, n0, n1, n2, vn, vnf);
+}
 __global__ void k_realize_vnormals(int nv, const int *__restrict__ af_ptr, const int *__restrict__ af_idx,
                                    const double4 *__restrict__ fn, double4 *__restrict__ vn,
                                    float4 *__restrict__ vnf)
@@ -152,22 +156,10 @@ __global__ void k_realize_vnormals(int nv, const int *__restrict__ af_ptr, const
 
 // ------------------------------------------------------------- transforms
 
-__device__ inline void store_vt(double4 *vt, int i, double x, double y, double z)
-{
-    vt[i] = make_double4(x, y, z, 0.0);
-}
-
 // Vertex coordinates in each view's frame: cotrans(v, oa, x, 1) then
 // += orbit_offset (src/shape/posvis.c:159-166; 0.0 for the engine's views).
-template <typename T4>
-__global__ void k_xform(const FrameGeom *__restrict__ geoms, const double4 *__restrict__ vx, int nv,
-                        T4 *__restrict__ vt)
+__device__ inline double4 view_vertex(const FrameGeom &g, double4 x)
 {
-    grid_dep_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nv) return;
-    const FrameGeom &g = geoms[blockIdx.y];
-    double4 x = vx[i];
     double t[3];
 #pragma unroll
     for (int r = 0; r < 3; r++) {
@@ -177,7 +169,17 @@ __global__ void k_xform(const FrameGeom *__restrict__ geoms, const double4 *__re
         t[r] += g.oa[3 * r + 2] * x.z;
         t[r] += g.off[r];
     }
-    store_vt(vt, g.vt_base + i, t[0], t[1], t[2]);
+    return make_double4(t[0], t[1], t[2], 0.0);
+}
+template <typename T4>
+__global__ void k_xform(const FrameGeom *__restrict__ geoms, const double4 *__restrict__ vx, int nv,
+                        T4 *__restrict__ vt)
+{
+    grid_dep_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nv) return;
+    const FrameGeom &g = geoms[blockIdx.y];
+    vt[g.vt_base + i] = view_vertex(g, vx[i]);
 }
 
 // -------------------------------------------------------------- binning
@@ -192,35 +194,18 @@ __global__ void k_xform(const FrameGeom *__restrict__ geoms, const double4 *__re
 // Facet culling, bounding box, outbnd flag and POSrect bookkeeping of
 // posvis (src/shape/posvis.c:142-199, 322-364), then one bin entry per
 // overlapped 16x16 tile. Bin order is arbitrary; the raster kernel sorts.
-template <typename T4>
-__global__ void __launch_bounds__(256, BIN_MIN_BLOCKS) k_bin(const FrameGeom *__restrict__ geoms, int view0, int nf,
-                      const int4 *__restrict__ fvi, const double4 *__restrict__ fn,
-                      const T4 *__restrict__ vt, FrameState *__restrict__ states,
-                      int *__restrict__ bin_count, int2 *__restrict__ bin_ids, int cap, VnormalArgs vna)
+__device__ inline bool faces_viewer(const FrameGeom &g, const double4 &nb)
 {
-    grid_dep_trigger();
-    grid_dep_wait();
-    int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (vna.nv > 0 && blockIdx.y == gridDim.y - 1) {
-        // the batched graph's last row of blocks: the vertex normals, which
-        // like the binning wait for the facet normals only
-        for (int i = f; i < vna.nv; i += gridDim.x * blockDim.x)
-            realize_vnormal(i, vna.af_ptr, vna.af_idx, fn, vna.vn, vna.vnf);
-        return;
-    }
-    if (f >= nf) return;
-    int v = view0 + blockIdx.y;
-    const FrameGeom &g = geoms[v];
-    // the normal and the corner indices load together (the culling test
-    // does not wait for the indices); the corners follow
-    const double4 nb = fn[f];
-    const int4 c = fvi[f];
     double nz = 0.0;
     nz += g.oa[6] * nb.x;
     nz += g.oa[7] * nb.y;
     nz += g.oa[8] * nb.z;
-    if (!(nz > 0.0)) return;
-    T4 p0 = vt[g.vt_base + c.x], p1 = vt[g.vt_base + c.y], p2 = vt[g.vt_base + c.z];
+    return nz > 0.0;
+}
+// A facet that faces the viewer, its corners in the view's frame: its entries.
+__device__ inline void bin_facet(int f, const FrameGeom &g, const double4 p0, const double4 p1, const double4 p2,
+                                 FrameState &st, int *__restrict__ bin_count, int2 *__restrict__ bin_ids, int cap)
+{
     const double kmpp = g.kmpp;
     const int n = g.n;
     double xmin = dmin_((double)p0.x, dmin_((double)p1.x, (double)p2.x));
@@ -233,7 +218,6 @@ __global__ void __launch_bounds__(256, BIN_MIN_BLOCKS) k_bin(const FrameGeom *__
     double jmax_d = floor(ymax / kmpp + SMALLVAL + 0.5);
     int imin = clamp_lo(imin_d), imax = clamp_hi(imax_d);
     int jmin = clamp_lo(jmin_d), jmax = clamp_hi(jmax_d);
-    FrameState &st = states[v];
     if (imin < -n || imax > n || jmin < -n || jmax > n)
         st.outbnd = 1;
     int i1 = max(imin, -n), i2 = min(imax, n), j1 = max(jmin, -n), j2 = min(jmax, n);
@@ -291,6 +275,32 @@ __global__ void __launch_bounds__(256, BIN_MIN_BLOCKS) k_bin(const FrameGeom *__
             }
         }
 }
+template <typename T4>
+__global__ void __launch_bounds__(256, BIN_MIN_BLOCKS) k_bin(const FrameGeom *__restrict__ geoms, int view0, int nf,
+                      const int4 *__restrict__ fvi, const double4 *__restrict__ fn,
+                      const T4 *__restrict__ vt, FrameState *__restrict__ states,
+                      int *__restrict__ bin_count, int2 *__restrict__ bin_ids, int cap, VnormalArgs vna)
+{
+    grid_dep_trigger();
+    grid_dep_wait();
+    int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (vna.nv > 0 && blockIdx.y == gridDim.y - 1) {
+        // a batched evaluation's last row of blocks: the vertex normals, which
+        // like the binning wait for the facet normals only
+        for (int i = f; i < vna.nv; i += gridDim.x * blockDim.x)
+            realize_vnormal(i, vna.af_ptr, vna.af_idx, fn, vna.vn, vna.vnf);
+        return;
+    }
+    if (f >= nf) return;
+    int v = view0 + blockIdx.y;
+    const FrameGeom &g = geoms[v];
+    // the normal and the corner indices load together (the culling test
+    // does not wait for the indices); the corners follow
+    const double4 nb = fn[f];
+    const int4 c = fvi[f];
+    if (!faces_viewer(g, nb)) return;
+    bin_facet(f, g, vt[g.vt_base + c.x], vt[g.vt_base + c.y], vt[g.vt_base + c.z], states[v], bin_count, bin_ids, cap);
+}
 
 __device__ inline FrameState blank_state()
 {
@@ -326,7 +336,12 @@ __global__ void k_reset_state(FrameState *st, int nviews, int *bin_count, int nt
 // counts, and the cleared images. As separate launches on side branches (a
 // reset kernel and three or four clears after one another) the clears ended
 // 9.8 us after the parameters had arrived and binning started then; as one
-// launch it starts after 2.8 (one frame).
+// launch it starts after 2.8 (one frame). With few facets and views (bin_ids not
+// null) the launch bins as well and sums the vertex normals, both from facets
+// realized once more, and the evaluation has no binning launch: one frame of 2200
+// facets 37.4 us on the device before, 31.0 so. It then bins into states and
+// counts that the launch before it blanked, and blanks the other pair.
+constexpr int VN_BLOCK = 32;               // vertices whose normals a block sums
 struct FrontParams {
     const FrontArgs &a;
     __device__ double r(int i) const
@@ -343,23 +358,57 @@ __global__ void __launch_bounds__(256) k_front(const __grid_constant__ FrontArgs
     grid_dep_trigger();
     const ModelDev &m = a.m;
     const FrontParams par{a};
+    __shared__ double4 normal[256];
     int b = blockIdx.x;
+    if (b < a.nb_bin) {
+        const int bpv = (m.nf + 255) / 256, v = b / bpv, f = (b - v * bpv) * 256 + threadIdx.x;
+        if (f >= m.nf) return;
+        const FrameGeom &g = a.geoms[v];
+        const double4 x0 = realize_vertex(m.fv[3 * f], m.a, m.u, par, m.vcomp, m.cxf);
+        const double4 x1 = realize_vertex(m.fv[3 * f + 1], m.a, m.u, par, m.vcomp, m.cxf);
+        const double4 x2 = realize_vertex(m.fv[3 * f + 2], m.a, m.u, par, m.vcomp, m.cxf);
+        if (!faces_viewer(g, facet_normal(x0, x1, x2, nullptr))) return;
+        bin_facet(f, g, view_vertex(g, x0), view_vertex(g, x1), view_vertex(g, x2), a.states[v], a.bin_count, a.bin_ids,
+                  a.cap);
+        return;
+    }
+    b -= a.nb_bin;
+    if (b < a.nb_vn) {
+        // VN_BLOCK vertices' attached facets lie one after another in af_idx:
+        // their normals by all threads (realized from the corners, as the
+        // facets' own blocks run beside this one), the sums by a thread per
+        // vertex
+        const int i0 = b * VN_BLOCK, i = i0 + threadIdx.x;
+        const int lo = m.af_ptr[i0], hi = m.af_ptr[min(i0 + VN_BLOCK, m.nv)];
+        const bool sums = threadIdx.x < VN_BLOCK && i < m.nv;
+        const int own0 = sums ? m.af_ptr[i] : 0, own1 = sums ? m.af_ptr[i + 1] : 0;
+        double n0 = 0.0, n1 = 0.0, n2 = 0.0;
+        for (int base = lo; base < hi; base += 256) {
+            const int j = base + threadIdx.x;
+            if (j < hi) {
+                const int f = m.af_idx[j];
+                normal[threadIdx.x] = facet_normal(realize_vertex(m.fv[3 * f], m.a, m.u, par, m.vcomp, m.cxf),
+                                                   realize_vertex(m.fv[3 * f + 1], m.a, m.u, par, m.vcomp, m.cxf),
+                                                   realize_vertex(m.fv[3 * f + 2], m.a, m.u, par, m.vcomp, m.cxf),
+                                                   nullptr);
+            }
+            __syncthreads();
+            for (int k = max(own0, base); k < min(own1, base + 256); k++) {
+                const double4 nk = normal[k - base];
+                n0 += nk.x; n1 += nk.y; n2 += nk.z;
+            }
+            __syncthreads();
+        }
+        if (sums) store_vnormal(i, n0, n1, n2, m.vn, m.vnf);
+        return;
+    }
+    b -= a.nb_vn;
     if (b < a.nb_xform) {
         const int bpv = (m.nv + 255) / 256, v = b / bpv;
         const int i = (b - v * bpv) * 256 + threadIdx.x;
         if (i >= m.nv) return;
         const FrameGeom &g = a.geoms[v];
-        const double4 x = realize_vertex(i, m.a, m.u, par, m.vcomp, m.cxf);
-        double t[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            t[k] = 0.0;
-            t[k] += g.oa[3 * k + 0] * x.x;
-            t[k] += g.oa[3 * k + 1] * x.y;
-            t[k] += g.oa[3 * k + 2] * x.z;
-            t[k] += g.off[k];
-        }
-        store_vt(a.vt, g.vt_base + i, t[0], t[1], t[2]);
+        a.vt[g.vt_base + i] = view_vertex(g, realize_vertex(i, m.a, m.u, par, m.vcomp, m.cxf));
         return;
     }
     b -= a.nb_xform;
@@ -368,9 +417,9 @@ __global__ void __launch_bounds__(256) k_front(const __grid_constant__ FrontArgs
         return;
     }
     b -= a.nb_model;
-    const int nb = gridDim.x - a.nb_xform - a.nb_model;
+    const int nb = gridDim.x - a.nb_bin - a.nb_vn - a.nb_xform - a.nb_model;
     const long long t0 = (long long)b * 256 + threadIdx.x, step = (long long)nb * 256;
-    for (long long i = t0; i < a.nviews; i += step) a.states[i] = blank_state();
+    for (long long i = t0; i < a.nviews; i += step) a.blank[i] = blank_state();
     if (b == 0) {
         if (threadIdx.x < a.nscale) a.scale_out[threadIdx.x] = a.scale[threadIdx.x];
         if (threadIdx.x < a.nchange) a.r_out[a.change_at[threadIdx.x]] = a.change_to[threadIdx.x];
@@ -1216,7 +1265,9 @@ void launch_front(const FrontArgs &a0, cudaStream_t s)
     // four 16-byte stores a thread, at most four blocks per SM
     size_t nb = (words + 1023) / 1024;
     nb = nb < 1 ? 1 : nb > 4 * 148 ? 4 * 148 : nb;
-    k_front<<<a.nb_xform + a.nb_model + (int)nb, 256, 0, s>>>(a);
+    a.nb_bin = a.bin_ids ? a.nviews * ((a.m.nf + 255) / 256) : 0;
+    a.nb_vn = a.bin_ids ? (a.m.nv + VN_BLOCK - 1) / VN_BLOCK : 0;
+    k_front<<<a.nb_bin + a.nb_vn + a.nb_xform + a.nb_model + (int)nb, 256, 0, s>>>(a);
 }
 
 void launch_xform_f64(const FrameGeom *g, int nviews, const double4 *vx, int nv, double4 *vt, cudaStream_t s,

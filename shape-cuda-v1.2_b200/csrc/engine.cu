@@ -330,10 +330,12 @@ int EngineImpl::finalize()
     AL(d_fv, (size_t)3 * nf); AL(d_afp, (size_t)nv + 1); AL(d_afi, af_idx.size());
     AL(md.vx, (size_t)nv); AL(md.vn, (size_t)nv); AL(md.fn, (size_t)nf); AL(md.area, (size_t)nf);
     AL(md.fvi, (size_t)nf); AL(md.vnf, (size_t)nv);
-    AL(d_geoms, (size_t)nviews); AL(d_states, (size_t)nviews); AL(d_laws, laws.size());
+    AL(d_geoms, (size_t)nviews); AL(d_states, (size_t)nviews); AL(d_states_next, (size_t)nviews); AL(d_laws, laws.size());
     AL(d_work, work.size());
     AL(d_vt64, (size_t)nviews * nv);
-    AL(d_bin_count, (size_t)ntiles); AL(d_bin_ids, (size_t)ntiles * cap);
+    AL(d_bin_count, (size_t)ntiles); AL(d_bin_count_next, (size_t)ntiles);
+    next_blank = false;
+    AL(d_bin_ids, (size_t)ntiles * cap);
     AL(d_obs, (size_t)fit_elems); AL(d_oov, (size_t)fit_elems);
     // the FP32 raster adds rows of its footprints with aligned 16-byte
     // vector reductions that may reach up to 8 elements past a row's last
@@ -1051,6 +1053,15 @@ int EngineImpl::tune_bins()
 // marks (optional, batched forms only): events recorded after each stage
 // 0 realize, 1 reset, 2 transform, 3 bin, 4 raster, 5 chi2, 6 lightcurve
 // photometry, 7 finalize + summary.
+// Facets x views up to which a batched evaluation bins in its first launch
+// (k_front), which then realizes each facet once per view instead of reading
+// the realized normal and corners, but saves a launch and the wait for it. On
+// the device, separate and in one, us: 1 view of 2200 facets 37.4 and 31.0, 12 of
+// 2200 87 and 83, 9 of 8000 68.7 and 55; 50 of 8000 99 and 98, 64 of 8000 131.9 and
+// 133.6, 16 of 32768 234 and 239, 1600 of 8000 1732 and 1914.
+constexpr long long FRONT_BINS = 131072;
+bool EngineImpl::front_bins() const { return (long long)nviews * nf <= FRONT_BINS; }
+
 int EngineImpl::enqueue(int form, cudaEvent_t *marks)
 {
     cudaStream_t s = stream;
@@ -1065,22 +1076,36 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
     };
     // A batched evaluation opens with one launch for realize, the view
     // transforms, the blank states and the clears (k_front), and its binning
-    // launch carries the vertex normals; the plain form and stage timing run
+    // launch, where it has one, carries the vertex normals; the plain form and stage timing run
     // them one by one, from the uploaded parameters.
     const bool chain = (form != SHAPE_FORM_PLAIN_FP64) && !marks;
+    // few facets and views are binned within that first launch as well, into
+    // the states and counts that the one before it blanked
+    const bool bins = chain && front_bins();
     // the FP32 form sums Doppler spectra in FP64 (then rounds them once)
     const bool need64 = fit_elems && (!f32 || !dop_frames.empty());
     if (int rc = enqueue_spin()) return rc;
     if (chain) {
         FrontArgs fr;
         memset(&fr, 0, sizeof fr);
-        fr.geoms = d_geoms; fr.nviews = nviews; fr.m = md; fr.vt = d_vt64; fr.states = d_states;
+        fr.geoms = d_geoms; fr.nviews = nviews; fr.m = md; fr.vt = d_vt64;
         int k = 0;
         auto clear = [&](void *p, size_t bytes) {
             fr.clear[k] = static_cast<unsigned char *>(p);
             fr.clear_bytes[k++] = bytes;
         };
-        clear(d_bin_count, sizeof(int) * (size_t)ntiles);
+        if (bins) {
+            if (!next_blank) launch_reset_state(d_states_next, nviews, d_bin_count_next, ntiles, s);
+            next_blank = false;
+            std::swap(d_states, d_states_next);
+            std::swap(d_bin_count, d_bin_count_next);
+            fr.states = d_states; fr.bin_count = d_bin_count; fr.bin_ids = d_bin_ids; fr.cap = cap;
+            fr.blank = d_states_next;
+            clear(d_bin_count_next, sizeof(int) * (size_t)ntiles);
+        } else {
+            fr.blank = d_states;
+            clear(d_bin_count, sizeof(int) * (size_t)ntiles);
+        }
         clear(d_seen, nf);
         if (f32 && fit_elems) clear(d_fit32, sizeof(float) * (size_t)fit_elems);
         if (need64) clear(d_fit64, sizeof(double) * (size_t)fit_elems);
@@ -1090,6 +1115,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (int rc_ = front_params(fr)) return rc_;
         launch_front(fr, s);
         if (int rc_ = launched("realize and transform")) return rc_;
+        next_blank = next_blank || bins;
     } else {
         launch_realize(md, s);
         mark(0);
@@ -1157,7 +1183,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         if (!chain) launch_xform_f64(d_geoms, nviews, md.vx, nv, d_vt64, s);
         mark(2);
         if (int rc_ = launched("view transform")) return rc_;
-        launch_bin_f64(d_geoms, 0, nviews, md, d_vt64, d_states, d_bin_count, d_bin_ids, cap, s, pdl, chain);
+        if (!bins) launch_bin_f64(d_geoms, 0, nviews, md, d_vt64, d_states, d_bin_count, d_bin_ids, cap, s, pdl, chain);
         mark(3);
         if (int rc_ = launched("binning")) return rc_;
         // one CTA per tile, heaviest tiles first (empty tiles sort last and
@@ -1254,9 +1280,9 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
 // and copies excluded).
 int EngineImpl::kernels_per_eval(int form) const
 {
-    // front and binning, or realize (vertices + facets, vertex normals) and the
+    // front (and binning), or realize (vertices + facets, vertex normals) and the
     // state reset
-    int n = form == SHAPE_FORM_PLAIN_FP64 ? 3 : 2;
+    int n = form == SHAPE_FORM_PLAIN_FP64 ? 3 : front_bins() ? 1 : 2;
     n += (spin_device && n_spin_src > 0) ? 1 : 0;   // view realization from the spin state
     if (form == SHAPE_FORM_PLAIN_FP64) {
         n += 3 * nviews;

@@ -140,11 +140,12 @@ struct EngineImpl {
     double *d_r = nullptr, *d_scale = nullptr, *d_a = nullptr, *d_u = nullptr;
     int *d_fv = nullptr, *d_afp = nullptr, *d_afi = nullptr;
     FrameGeom *d_geoms = nullptr;
-    FrameState *d_states = nullptr;
+    FrameState *d_states = nullptr, *d_states_next = nullptr;
     RadarLawDev *d_laws = nullptr;
     int4 *d_work = nullptr;
     double4 *d_vt64 = nullptr;
-    int *d_bin_count = nullptr;
+    int *d_bin_count = nullptr, *d_bin_count_next = nullptr;
+    bool next_blank = false;                // d_states_next and d_bin_count_next are blank
     int2 *d_bin_ids = nullptr;
     double *d_obs = nullptr, *d_oov = nullptr;
     double *d_fit64 = nullptr;
@@ -316,6 +317,7 @@ struct EngineImpl {
     int raster_grid(int form, int nonempty, const RasterArgs &a, bool f32) const;
     int evaluate(int form, shape_eval_summary *out);
     int kernels_per_eval(int form) const;
+    bool front_bins() const;
     void fill_params(double *dst) const
     {
         memcpy(dst, r.data(), sizeof(double) * nv);

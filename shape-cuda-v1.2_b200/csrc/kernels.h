@@ -144,7 +144,13 @@ struct FrontArgs {
     int nviews;
     ModelDev m;
     double4 *vt;
+    FrameState *blank;                 // states to blank
+    // binning within the launch (bin_ids null: a launch of its own follows):
+    // into states and counts that an earlier launch has blanked
     FrameState *states;
+    int *bin_count;
+    int2 *bin_ids;
+    int cap;
     // parameter changes since the device arrays were last written: the scale
     // factors (of up to SCALES / 3 components) and up to CHANGES deviations
     // travel with the launch, which also stores them, instead of a copy of all
@@ -157,7 +163,7 @@ struct FrontArgs {
     double *r_out, *scale_out;
     unsigned char *clear[CLEARS];      // arrays to clear (16-byte aligned) and their bytes
     size_t clear_bytes[CLEARS];
-    int nb_xform, nb_model;            // blocks of the first two ranges (set by launch_front)
+    int nb_bin, nb_vn, nb_xform, nb_model;   // blocks of the first ranges (set by launch_front)
 };
 void launch_front(const FrontArgs &a, cudaStream_t s);
 // the vertex normals as extra blocks of k_bin (nv 0: none)
