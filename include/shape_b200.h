@@ -42,10 +42,10 @@ extern "C" {
 /* Evaluation forms. */
 #define SHAPE_FORM_PLAIN_FP64 0   /* per-frame launch sequence, FP64 end to end:
                                      facet maps bit-exact with the reference */
-#define SHAPE_FORM_BATCHED_FP64 1 /* all frames per launch, CUDA graph, FP64 */
-#define SHAPE_FORM_BATCHED_FP32 2 /* all frames per launch, CUDA graph, FP32
-                                     raster/synthesis, FP64 rotations and
-                                     compensated FP64 chi-square */
+#define SHAPE_FORM_BATCHED_FP64 1 /* all frames per launch, FP64 */
+#define SHAPE_FORM_BATCHED_FP32 2 /* all frames per launch, FP64 coverage and
+                                     depths, FP32 shading and synthesis of radar
+                                     views, compensated FP64 chi-square */
 
 typedef struct shape_engine shape_engine;
 
@@ -176,8 +176,8 @@ int shape_engine_get_seen(shape_engine *e, unsigned char *seen);
 int shape_engine_get_realized(shape_engine *e, double *x, double *vn, double *fn,
                               double *area);
 
-/* Runs one evaluation of a batched form without its graph, with CUDA events
- * between stages, and writes the stage times in ms: [0] realize, [1] state
+/* Runs one evaluation of a batched form stage by stage, with CUDA events
+ * between the stages, and writes the stage times in ms: [0] realize, [1] state
  * reset and image clears, [2] view transforms, [3] facet binning,
  * [4] tile raster + delay-Doppler synthesis, [5] chi-square partials,
  * [6] lightcurve shadowing + photometry, [7] finalize + summary. Datasets
@@ -218,14 +218,14 @@ typedef struct shape_vary_options {
 } shape_vary_options;
 int shape_engine_vary_params(shape_engine *e, const shape_vary_options *opt, double out[4]);
 
-/* Raster kernel of the batched forms./* Raster kernel of the batched forms. mode -1 (default): the first batched
+/* Raster kernel of the batched forms. mode -1 (default): the first batched
  * evaluation of each form times four candidates on this engine's datasets
  * (256 or 128 threads per tile, each with one CTA per non-empty tile or a
  * persistent grid of resident CTAs on every SM striding over the tiles)
  * and keeps the fastest; the choice is remembered for engines of the same
  * size class in the process. mode 0 / 1: 256 / 128 threads, one CTA per
  * tile, no timing. Every candidate computes the same images. Radar views
- * and lightcurve / sky views are two launches of the same choice. */
+ * and lightcurve / sky views are launches of the same choice. */
 int shape_engine_set_raster_tuning(shape_engine *e, int mode);
 /* The raster choice of a form: *variant (0: 256 threads per tile, 1: 128),
  * *persistent, and ms[4] (may be NULL) the measured raster
@@ -242,7 +242,7 @@ int shape_engine_get_raster_tuning(shape_engine *e, int form, int *variant, int 
  * extents, shifts and badradar term, src/shape/pos2deldop.c:218-288) are
  * recomputed on the host exactly as at finalize and copied to the device on
  * the engine's stream, so the next evaluation of every form sees them and
- * captured graphs stay valid; the results equal those of an engine built
+ * nothing is rebuilt; the results equal those of an engine built
  * with the new view. Bin capacities keep their tuning (a tile that now
  * overflows takes the ordered full-scan path). Before finalize the frame's
  * descriptor is updated. Workloads a server already took from this engine
@@ -311,13 +311,13 @@ int shape_engine_set_spin_model(shape_engine *e, const shape_spin_state *spin, c
                                 const double *set_omegaoff, const double *frame_t,
                                 const double *frame_orbspin);
 /* Spin realization inside each evaluation (principal-axis rotators): with
- * on = 1 the evaluation graph copies the spin state and dataset offsets
+ * on = 1 the evaluation copies the spin state and dataset offsets
  * from pinned memory and a kernel realizes every radar frame's and
  * lightcurve point's ae (and a frame's spin vector) and view constants
  * before the raster, as shape_realize_spin and the host setup do (the
  * device's sin and cos may differ from the C library's in the last place).
  * shape_engine_set_spin_param then only records the value: a spin trial is
- * a graph replay with no host realization or view upload. Needs the spin
+ * an evaluation with no host realization or view upload. Needs the spin
  * model (SHAPE_E_STATE without it) of a principal-axis rotator and single-
  * view frames (SHAPE_E_UNSUPPORTED otherwise); set_frame_view and
  * set_point_view are refused while it is on. on = 0 realizes on the host
@@ -328,8 +328,7 @@ int shape_engine_set_spin_device(shape_engine *e, int on);
 int shape_engine_get_frame_view(shape_engine *e, int global_frame, double ae[9], double spin[3]);
 /* One spin parameter (SHAPE_PAR_SPIN_* / ANGLEOFF / OMEGAOFF) of the spin
  * model: set re-realizes every view and copies the view constants to the
- * device on the engine's stream (the next evaluation, graph replays
- * included, sees them). */
+ * device on the engine's stream (the next evaluation sees them). */
 int shape_engine_set_spin_param(shape_engine *e, int kind, int index, double value);
 int shape_engine_get_spin_param(shape_engine *e, int kind, int index, double *value);
 /* Tuning state after finalize: [0] bin capacity, [1] largest tile count of
@@ -383,8 +382,7 @@ typedef struct shape_fit_result {
  * objective starting from (value, value + step), then Brent-minimise it to
  * tol*|x| + abstol, adopt the minimum, and iterate over all parameters
  * until the objective's fractional decrease in an iteration is below
- * term_prec. Each trial is one device evaluation (a graph replay in the
- * batched forms). trace (optional, 2*trace_max doubles) receives the
+ * term_prec. Each trial is one device evaluation. trace (optional, 2*trace_max doubles) receives the
  * (parameter number, trial value) of every trial in order. */
 int shape_engine_bestfit(shape_engine *e, const shape_fit_param *params, int nparams,
                          const shape_fit_options *opt, shape_fit_result *res, double *trace,

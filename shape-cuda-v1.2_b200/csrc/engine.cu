@@ -1375,8 +1375,8 @@ int EngineImpl::launch(int form)
                 tuned[form] = 1;
             }
         }
-        // Straight launches, not a captured graph: the chain is four launches
-        // (a radar engine's) that need not wait for one another's launch, and
+        // Straight launches, not a captured graph: the chain is three or four
+        // launches (a radar engine's) that need not wait for one another's launch, and
         // the first starts sooner than a graph's first node (one frame 49.4 us
         // between the events as a graph, 42.0 launched; 64 frames 153.5 and
         // 149.3), and its arguments carry the trial's parameters.

@@ -1,6 +1,6 @@
 // bestfit driver of the SHAPE B200 engine: one-parameter-at-a-time line
 // minimisations of the objective (src/shape/bestfit.c:250-704), every trial
-// evaluated on the device (a CUDA-graph replay for the batched forms).
+// evaluated on the device.
 //
 // The two line searches are written from their published descriptions:
 //  - bracketing by golden-ratio expansion with parabolic extrapolation

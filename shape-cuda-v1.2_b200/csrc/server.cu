@@ -2,8 +2,8 @@
 //
 // A workload is a model with its datasets, registered once from a
 // configured engine. The server keeps device-resident INSTANCES of
-// workloads (each an engine with its own device arenas, stream and captured
-// evaluation graph). Requests (a workload and its scale factors) are
+// workloads (each an engine with its own device arenas and
+// stream). Requests (a workload and its scale factors) are
 // submitted as they arrive and served by a scheduler thread:
 //   - completions are polled through each running instance's event;
 //   - admission walks the waiting requests oldest first and admits every
@@ -105,7 +105,7 @@ struct ServerImpl {
         int rc = E.finalize();
         if (rc) return rc;
         shape_eval_summary s;
-        rc = E.evaluate(wl[w].form, &s);       // captures the evaluation graph
+        rc = E.evaluate(wl[w].form, &s);       // tunes the form
         if (rc) return rc;
         wl[w].footprint = E.footprint();
         I->workload = w;

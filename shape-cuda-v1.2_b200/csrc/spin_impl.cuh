@@ -1,5 +1,5 @@
 // Principal-axis spin realization shared by the host (shape_realize_spin)
-// and the device (the evaluation graph's view realization): realize_spin's
+// and the device (an evaluation's view realization): realize_spin's
 // per-view steps (src/shape/realize_spin.c:41-285) with inteuler's
 // principal-axis branch (src/shape/inteuler.c) and euler2mat
 // (src/util/euler.c), in the reference's operation order. The host's sin

@@ -1,5 +1,5 @@
 // View geometry shared by the host (engine setup, the one-view operations)
-// and the device (spin realization inside the evaluation graph): FP64 in
+// and the device (spin realization inside the evaluation): FP64 in
 // the reference's operation order, so both give the same values (square
 // roots are correctly rounded on both; the one log of a badradar view may
 // differ in its last bit). Compile with FMA contraction off.

@@ -340,7 +340,7 @@ class Engine:
 
     def set_spin_device(self, on=True):
         """Realize the views from the spin model inside each evaluation
-        (principal-axis rotators): spin trials replay the graph only."""
+        (principal-axis rotators): a spin trial is an evaluation only."""
         _chk(self.L.shape_engine_set_spin_device(self.h, 1 if on else 0))
 
     def frame_view(self, frame):
