@@ -8,6 +8,7 @@
 // which POS pixels each facet covers. Expressions keep the reference's
 // association order; sums that the reference starts from a literal 0.0
 // (cotrans, src/util/cotrans.c; mmmul) start from 0.0 here as well.
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 
@@ -341,6 +342,11 @@ __global__ void k_reset_state(FrameState *st, int nviews, int *bin_count, int nt
 // realized once more, and the evaluation has no binning launch: one frame of 2200
 // facets 37.4 us on the device before, 31.0 so. It then bins into states and
 // counts that the launch before it blanked, and blanks the other pair.
+// Views whose vertices a thread writes, from the vertex realized once: as many
+// as leave eight blocks of vertices per SM, at most 8. 1600 views of 4002
+// vertices, evaluation on the device: 1731 us with a view per thread, 1713 with
+// 4, 1711 with 8 and 1712 with 16 (the 205 MB of vertices take 32 us to write).
+constexpr int FRONT_VIEWS = 8, FRONT_GRID = 148 * 8;
 constexpr int VN_BLOCK = 32;               // vertices whose normals a block sums
 struct FrontParams {
     const FrontArgs &a;
@@ -404,11 +410,14 @@ __global__ void __launch_bounds__(256) k_front(const __grid_constant__ FrontArgs
     }
     b -= a.nb_vn;
     if (b < a.nb_xform) {
-        const int bpv = (m.nv + 255) / 256, v = b / bpv;
-        const int i = (b - v * bpv) * 256 + threadIdx.x;
+        const int bpv = (m.nv + 255) / 256, v0 = b / bpv * a.views;
+        const int i = (b % bpv) * 256 + threadIdx.x;
         if (i >= m.nv) return;
-        const FrameGeom &g = a.geoms[v];
-        a.vt[g.vt_base + i] = view_vertex(g, realize_vertex(i, m.a, m.u, par, m.vcomp, m.cxf));
+        const double4 x = realize_vertex(i, m.a, m.u, par, m.vcomp, m.cxf);
+        for (int v = v0; v < min(v0 + a.views, a.nviews); v++) {
+            const FrameGeom &g = a.geoms[v];
+            a.vt[g.vt_base + i] = view_vertex(g, x);
+        }
         return;
     }
     b -= a.nb_xform;
@@ -1258,7 +1267,9 @@ void launch_reset_state(FrameState *st, int nviews, int *bin_count, int ntiles, 
 void launch_front(const FrontArgs &a0, cudaStream_t s)
 {
     FrontArgs a = a0;
-    a.nb_xform = a.nviews * ((a.m.nv + 255) / 256);
+    const long long bpv = (a.m.nv + 255) / 256;
+    a.views = (int)std::min<long long>(FRONT_VIEWS, std::max<long long>(1, bpv * a.nviews / FRONT_GRID));
+    a.nb_xform = (int)(bpv * ((a.nviews + a.views - 1) / a.views));
     a.nb_model = (a.m.nf + a.m.nv + 255) / 256;
     size_t words = (size_t)a.nviews;
     for (size_t n : a.clear_bytes) words = n / 16 > words ? n / 16 : words;

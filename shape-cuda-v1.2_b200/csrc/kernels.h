@@ -163,6 +163,7 @@ struct FrontArgs {
     double *r_out, *scale_out;
     unsigned char *clear[CLEARS];      // arrays to clear (16-byte aligned) and their bytes
     size_t clear_bytes[CLEARS];
+    int views;                         // views whose vertices a thread writes
     int nb_bin, nb_vn, nb_xform, nb_model;   // blocks of the first ranges (set by launch_front)
 };
 void launch_front(const FrontArgs &a, cudaStream_t s);
