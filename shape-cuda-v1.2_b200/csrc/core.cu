@@ -1080,8 +1080,9 @@ __global__ void k_totals(SummaryArgs a)
 // thread 0 of the block with their compensations. The item is a share of
 // the frame's lit box, the rows and columns that its footprints reach (the
 // union over a smeared frame's views): outside it the fit is zero and adds
-// nothing. Each thread sums its bins in order in plain FP64, then the threads'
-// sums merge with compensation in a fixed order.
+// nothing. Each thread adds U bins in plain FP64 and that sum with
+// compensation to its own, then the threads' sums merge with compensation in a
+// fixed order.
 struct Chi2Frame {                             // a frame's constants
     int view, nviews, nitems, ndel, ndop, dop1d;
     long long base;
@@ -1105,7 +1106,7 @@ __device__ void chi2_item(const Chi2Args &a, const Chi2Frame &h, const FrameStat
     const int b0 = k * share, b1 = min(n, b0 + share);
     // a spectrum of the FP32 form is summed in FP64 and rounded once, here
     const bool spectrum = sizeof(T) == 4 && h.dop1d;
-    double sm2 = 0.0, som = 0.0;
+    m2 = om = KSum{0, 0};
     if (b0 + tid < b1) {
         int row = (b0 + tid) / C, col = (b0 + tid) - row * C;
         const int drow = CHI2_THREADS / C, dcol = CHI2_THREADS - drow * C;
@@ -1131,15 +1132,16 @@ __device__ void chi2_item(const Chi2Args &a, const Chi2Frame &h, const FrameStat
                 col += dcol;
                 if (col >= C) { col -= C; row++; }
             }
+            double sm2 = 0.0, som = 0.0;
 #pragma unroll
             for (int j = 0; j < U; j++) {
                 sm2 += f[j] * f[j] * wv[j];
                 som += f[j] * ob[j] * wv[j];
             }
+            m2.add(sm2);
+            om.add(som);
         }
     }
-    m2 = KSum{sm2, 0};
-    om = KSum{som, 0};
     for (int off = 16; off > 0; off >>= 1) {
         m2.merge(shfl_ksum(m2, off));
         om.merge(shfl_ksum(om, off));
@@ -1171,7 +1173,7 @@ __device__ void chi2_item(const Chi2Args &a, const Chi2Frame &h, const FrameStat
 // What bounds it is the chain of dependent loads, fences and counts, not the
 // images: a warp per item of 512 bins of the whole image read 12.5 MB of 64
 // frames for their 5 % of lit bins and counted 6100 times (stage 23 us); a block
-// per share of the lit box counts 500 times (17 us).
+// per share of the lit box (chi2_shares) counts 500 times (17 us).
 template <typename T>
 __global__ void __launch_bounds__(CHI2_THREADS) k_chi2_summary(Chi2Args ca, FinalizeArgs fa, SummaryArgs sa,
                                                                int *counters)

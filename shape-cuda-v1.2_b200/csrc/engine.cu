@@ -98,6 +98,22 @@ static void spline_plan(const double *x, int n, double *out)
     }
 }
 
+// Blocks of 256 threads that sum a frame's chi-square, each a share of its lit
+// box. Images of up to 32768 bins: one per 2048 bins, at most 8, since a lit box
+// is a few per cent of such an image in a fit and each block costs a count
+// (core.cu, k_chi2_summary). Larger ones: one per 4096 bins, 16 bins a thread
+// where all are lit, while the frames' blocks fit the chip four to an SM. The
+// finalize stage with 8 blocks a frame and so, us, FP32: one frame of 512 x 512
+// bins 37.6 and 17.0, of 1024 x 1024 109 and 19, of 2048 x 2048 425 and 24, 16 of
+// 512 x 1024 93 and 44, 64 of 256 x 512 47.8 and 47.7; a share per 8192 or 16384
+// bins 21 and 25 on the first, eight blocks to an SM 29 on the third.
+static int chi2_shares(long long bins, int nframes)
+{
+    const long long small = std::min<long long>(8, (bins + 2047) / 2048);
+    const long long large = std::min<long long>(4 * 148 / nframes, (bins + 4095) / 4096);
+    return (int)std::max<long long>(1, std::max(small, large));
+}
+
 int EngineImpl::finalize()
 {
     if (!have_model) return set_err(SHAPE_E_STATE, "finalize: no model set");
@@ -205,9 +221,7 @@ int EngineImpl::finalize()
             if (g.dop1d) dop_frames.push_back(fi);
             frame_view.push_back(h.view);
             h.item0 = (int)chi2_items.size();
-            // a block of 256 threads per 2048 bins, at most 8: a share of the lit
-            // box is then a few bins a thread
-            const int shares = std::max(1, std::min(8, (F.ndel * F.ndop + 2047) / 2048));
+            const int shares = chi2_shares((long long)F.ndel * F.ndop, nframes);
             for (int k3 = 0; k3 < shares; k3++) chi2_items.push_back(make_int2(fi, k3));
             h.nitems = shares;
             chi2_items.push_back(make_int2(fi, -1));       // limits, flags, log-factors
