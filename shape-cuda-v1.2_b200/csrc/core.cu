@@ -1082,7 +1082,8 @@ __global__ void k_totals(SummaryArgs a)
 // union over a smeared frame's views): outside it the fit is zero and adds
 // nothing. Each thread adds U bins in plain FP64 and that sum with
 // compensation to its own, then the threads' sums merge with compensation in a
-// fixed order.
+// fixed order. A bin whose fit is zero adds exact zeros whatever its observation
+// and variance are (an infinite 1/var included), inside the box as outside.
 struct Chi2Frame {                             // a frame's constants
     int view, nviews, nitems, ndel, ndop, dop1d;
     long long base;
@@ -1135,6 +1136,7 @@ __device__ void chi2_item(const Chi2Args &a, const Chi2Frame &h, const FrameStat
             double sm2 = 0.0, som = 0.0;
 #pragma unroll
             for (int j = 0; j < U; j++) {
+                if (f[j] == 0.0) continue;
                 sm2 += f[j] * f[j] * wv[j];
                 som += f[j] * ob[j] * wv[j];
             }

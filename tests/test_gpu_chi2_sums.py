@@ -48,3 +48,38 @@ def test_small_terms_behind_a_large_one(cuda_device, form, side, pos):
     m2, om = math.fsum(f * f * oov), math.fsum(f * fit * oov)
     assert m2 > 2.0 ** 53
     assert abs(r["m2"] - m2) <= 32 and abs(r["om"] - om) <= 32
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_bins_without_fit_add_nothing(cuda_device, form):
+    """Bins that the model does not light, among them those between the lit ones
+    of its box, leave m2 and om as they are even where 1/var is infinite or the
+    observation is not a number (the sum of obs^2/var is then neither)."""
+    m = synth.harmonic_model()
+    p = synth.eval_params()
+    ds = synth.batched_dataset(1, (151, 151), (200, 200), (200, 200), None, p, seed=3)
+    n = 200 * 200
+    obs = np.random.default_rng(17).standard_normal(n)
+    e = _engine(m, p, ds, obs, np.ones(n))
+    e.evaluate(form)
+    fit, a = e.fit(0), e.results()[0]
+    size = {"m2": a["m2"], "om": np.abs(fit * obs).sum()}
+    e.close()
+    dark = np.nonzero(fit == 0)[0]
+    rows, cols = np.nonzero(fit.reshape(200, 200))
+    box = (dark // 200 >= rows.min()) & (dark // 200 <= rows.max()) & (dark % 200 >= cols.min()) & \
+        (dark % 200 <= cols.max())
+    assert box.sum() > 100
+    oov = np.ones(n)
+    oov[dark[::2]] = np.inf
+    obs[dark[1::2]] = np.nan
+    e = _engine(m, p, ds, obs, oov)
+    e.evaluate(form)
+    b = e.results()[0]
+    e.close()
+    # two evaluations' images differ in the order of their additions: the
+    # forms' own bars
+    tol = 1e-6 if form == eng.FORM_BATCHED_FP32 else 1e-12
+    assert not np.isfinite(b["o2"])
+    for k in size:
+        assert abs(b[k] - a[k]) <= tol * size[k], k
