@@ -443,7 +443,7 @@ int EngineImpl::finalize()
         CK(cudaMemcpyAsync(d_dop_extra, dop_extra.data(), sizeof(double) * dop_extra.size(),
                            cudaMemcpyHostToDevice, s));
     }
-    launch_frame_o2(d_fh, (int)fh.size(), d_geoms, d_obs, d_oov, d_o2, s);
+    launch_frame_o2(d_chi2_items, (int)chi2_items.size(), d_fh, (int)fh.size(), d_geoms, d_obs, d_oov, d_partials, d_o2, s);
     CK(cudaGetLastError());
     if (!lcpts.empty()) {
         CK(cudaMemcpyAsync(d_lcpts, lcpts.data(), sizeof(LcPointDev) * lcpts.size(), cudaMemcpyHostToDevice, s));

@@ -222,9 +222,9 @@ struct FinalizeArgs {
 // o2, m2, xsec, mean bin, and the badradar flag and log-factor of a model wider
 // than the overflow spectrum.
 constexpr int DOP_OVF_TERMS = 6;
-// sum obs^2 / var of each radar frame
-void launch_frame_o2(const FrameHost *fh, int nframes, const FrameGeom *geoms, const double *obs, const double *oov,
-                     double *o2, cudaStream_t s);
+// sum obs^2 / var of each radar frame (partials: as Chi2Args's, scratch here)
+void launch_frame_o2(const int2 *items, int nitems, const FrameHost *fh, int nframes, const FrameGeom *geoms,
+                     const double *obs, const double *oov, double *partials, double *o2, cudaStream_t s);
 
 struct LcSetDev {
     int npts, n;                // calc points, observed points

@@ -83,3 +83,19 @@ def test_bins_without_fit_add_nothing(cuda_device, form):
     assert not np.isfinite(b["o2"])
     for k in size:
         assert abs(b[k] - a[k]) <= tol * size[k], k
+
+
+# images of one share of the data's sum, of eight and of 256
+@pytest.mark.parametrize("side", [30, 200, 1024])
+def test_observed_sum(cuda_device, side):
+    """sum obs^2/var, formed once per dataset: a term of 2^54 before terms of 1,
+    each addition compensated, so the total is off by its own rounding (2)."""
+    m = synth.harmonic_model()
+    p = synth.eval_params()
+    ds = synth.batched_dataset(1, (151, 151), (side, side), (side, side), None, p, seed=3)
+    oov = np.ones(side * side)
+    oov[0] = 2.0 ** 54
+    e = _engine(m, p, ds, np.ones(side * side), oov)
+    e.evaluate(eng.FORM_BATCHED_FP64)
+    assert abs(e.results()[0]["o2"] - math.fsum(oov)) <= 2
+    e.close()
