@@ -102,7 +102,9 @@ static void spline_plan(const double *x, int n, double *out)
 // box. Images of up to 32768 bins: one per 2048 bins, at most 8, since a lit box
 // is a few per cent of such an image in a fit and each block costs a count
 // (core.cu, k_chi2_summary). Larger ones: one per 4096 bins, 16 bins a thread
-// where all are lit, while the frames' blocks fit the chip four to an SM. The
+// where all are lit, while the frames' blocks (and one more for a frame's
+// geometry) fit the chip four to an SM: 64 uneven frames take 17 us with 8
+// shares each and 19 with 9, a second wave. The
 // finalize stage with 8 blocks a frame and so, us, FP32: one frame of 512 x 512
 // bins 37.6 and 17.0, of 1024 x 1024 109 and 19, of 2048 x 2048 425 and 24, 16 of
 // 512 x 1024 93 and 44, 64 of 256 x 512 47.8 and 47.7; a share per 8192 or 16384
@@ -110,7 +112,7 @@ static void spline_plan(const double *x, int n, double *out)
 static int chi2_shares(long long bins, int nframes)
 {
     const long long small = std::min<long long>(8, (bins + 2047) / 2048);
-    const long long large = std::min<long long>(4 * 148 / nframes, (bins + 4095) / 4096);
+    const long long large = std::min<long long>(4 * 148 / nframes - 1, (bins + 4095) / 4096);
     return (int)std::max<long long>(1, std::max(small, large));
 }
 
