@@ -20,7 +20,7 @@
 // equals: no order is needed for it, and no sort. Only cos(e) of a limb pixel,
 // whose winner's smoothed normal faces away, depends on the order (it stays
 // that of the last earlier winner whose normal faced the viewer); such a
-// pixel walks its candidates in index order (pixel_history).
+// pixel steps back through its earlier winners (pixel_history).
 //
 // What bounds it: instruction issue and latency, not memory (the tile's data
 // come from L2). A facet of a 20000-pixel body spans about 4 pixels: the exact
@@ -780,40 +780,47 @@ __device__ inline bool entry_covers(const RasterArgs &a, const double4 *vt, cons
     return facet_st(q, x0, y0, s, t);
 }
 
-// cos(e)'s facet of a pixel whose final winner's smoothed normal faces away:
-// the last of the pixel's winners, walked in facet index order from depth z0
-// (has: the pixel was not blank), whose normal faces the viewer, by the sign of
-// its view-z component (facet, s and t; facet -1 when there is none).
+// cos(e)'s facet of a pixel whose final winner's smoothed normal faces away: the
+// last of the pixel's earlier winners whose normal faces the viewer, by the sign
+// of its view-z component (facet, s and t; facet -1 when there is none). Winners
+// are the facets deeper than z0 (has: the pixel was not blank) and than every
+// one of lower index, so the winner before facet f is the deepest facet below f:
+// the walk steps back from the final winner. Forwards, through every winner from
+// the first, 20 points of a 30 % rough body of 8192 facets took 348 us, 234
+// backwards; 16 frames of 511^2 pixels of 32768 facets with 3 % roughness 257 and
+// 240; 25 points of a smooth body the same.
 template <typename T, int NT>
 __device__ __noinline__ PixelHit pixel_history(const RasterArgs &a, const FrameGeom &g, const int2 *bin,
-                                               const TileShared<T, NT> &sh, bool staged, int p, bool has, double z0)
+                                               const TileShared<T, NT> &sh, bool staged, int p, int below, bool has,
+                                               double z0)
 {
     PixelHit h = {-1, -1, 0.0, 0.0, 0.0, 0.0, 0.0};
     const double4 *vt = static_cast<const double4 *>(a.vt) + g.vt_base;
     const double x0 = sh.xs[p / TILE_W], y0 = sh.ys[p % TILE_W];
     const int nc = candidates<T, NT>(sh, p);
-    int cur = -1;
     for (;;) {
-        int bf = INT_MAX;
+        int bf = -1;
         double bz = 0.0, bs = 0.0, bt = 0.0;
         for (int i = 0; i < nc; i++) {
             const int k = candidate<T, NT>(sh, p, i);
             if (k < 0) continue;
             const int f = bin[k].x;
-            if (f <= cur || f >= bf) continue;
+            if (f >= below) continue;
             FacetTerms q;
             double s, t;
             if (!entry_covers<T, NT>(a, vt, bin, sh, staged, k, x0, y0, q, s, t)) continue;
             const double z = facet_z(q, s, t);
-            if (!has || z > z0) { bf = f; bz = z; bs = s; bt = t; }
+            if (has && !(z > z0)) continue;
+            if (bf < 0 || z > bz || (z == bz && f < bf)) { bf = f; bz = z; bs = s; bt = t; }
         }
-        if (bf == INT_MAX) return h;
-        cur = bf;
-        z0 = bz;
-        has = true;
+        if (bf < 0) return h;
         double m[3];
         body_normal64(a, bf, bs, bt, true, m);
-        if (view_row64(g, 2, m) > 0.0) { h.gf = bf; h.gs = bs; h.gt = bt; }
+        if (view_row64(g, 2, m) > 0.0) {
+            h.gf = bf; h.gs = bs; h.gt = bt;
+            return h;
+        }
+        below = bf;
     }
 }
 
@@ -1208,7 +1215,7 @@ k_raster(const __grid_constant__ RasterArgs a)
                         faces = view_row64(g, 2, m) > 0.0;
                     }
                     if (!faces) {
-                        const PixelHit c = pixel_history<T, NT>(a, g, bin, sh, staged, p, had, had_z);
+                        const PixelHit c = pixel_history<T, NT>(a, g, bin, sh, staged, p, h.f, had, had_z);
                         h.gf = c.gf; h.gs = c.gs; h.gt = c.gt;
                         if (h.gf >= 0) normal();
                     }
