@@ -1050,12 +1050,15 @@ int EngineImpl::tune_bins()
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return part(x) < part(y); });
     std::vector<int4> sorted(work.size());
     for (int k = 0; k < 3; k++) work_n[k] = work_busy[k] = 0;
+    long long entries[3] = {0, 0, 0};
     for (size_t k = 0; k < work.size(); k++) {
         sorted[k] = work[order[k]];
         const int w = part(order[k]);
         work_n[w]++;
         work_busy[w] += counts[sorted[k].y] > 0;
+        entries[w] += counts[sorted[k].y];
     }
+    for (int k = 0; k < 3; k++) work_few[k] = raster_few(entries[k], work_busy[k]);
     if (!d_work_sorted) {
         int rc = mem.alloc(&d_work_sorted, work.size());
         if (rc) return rc;
@@ -1188,6 +1191,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
             rv.work = d_work + view_work0[v];
             rv.nwork = view_nwork[v];
             rv.mode = g.kind == VIEW_RADAR ? RASTER_RADAR : g.kind == VIEW_LC_SUN ? RASTER_SUN : RASTER_PHOTO;
+            rv.few = work_few[rv.mode];
             launch_raster_f64(rv, s);
             if (int rc_ = launched(g.kind == VIEW_RADAR ? "radar view chain" : "lightcurve view chain")) return rc_;
         }
@@ -1217,6 +1221,7 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
         for (int k = 0; k < 3; k++) {
             RasterArgs rk = ra;
             rk.mode = k;
+            rk.few = work_few[k];
             rk.work = d_work_sorted + w0;
             rk.nwork = work_n[k];
             w0 += work_n[k];

@@ -298,8 +298,9 @@ struct EngineImpl {
     int4 *d_work_sorted = nullptr;
     int tuned_max_count = 0, tuned_nonempty = 0;
     // the sorted work list holds radar, sun-view and observer-view tiles
-    // (RASTER_*): tiles of each part, and its first ones non-empty at tuning
-    int work_n[3] = {0, 0, 0}, work_busy[3] = {0, 0, 0};
+    // (RASTER_*): tiles of each part, its first ones non-empty at tuning, and
+    // whether those held few facets each (RasterArgs::few)
+    int work_n[3] = {0, 0, 0}, work_busy[3] = {0, 0, 0}, work_few[3] = {0, 0, 0};
     int fixed_cap = 0;            // > 0: bin capacity set by the caller, no autotuning
     int fp32_exact = 1;           // shape_engine_set_fp32_exact (part of the tuning key only)
     // Raster kernel per form (RasterArgs::variant) and grid (0: one CTA per

@@ -96,6 +96,7 @@ struct RasterArgs {
     int accumulate;
     unsigned char *won;
     int variant;               // 0: 256 threads per tile, 1: 128
+    int few;                   // 1: the kernel for views of few facets per tile (raster_few)
     int mode;                  // RASTER_*
     // RASTER_PHOTO: the views' points, the tiles' brightness sums and the
     // brightness images of sky frames (LcPointDev::b_base)
@@ -328,6 +329,11 @@ void launch_chi2_summary(const Chi2Args &ca, const FinalizeArgs &fa, const Summa
 // the totals alone (no radar frames)
 void launch_totals(const SummaryArgs &a, cudaStream_t s, bool pdl);
 
+// Whether tiles of this many bin entries in all are rastered by the kernels for
+// few facets per tile (raster_impl.cuh, FEW): where the tiles that have any hold
+// RASTER_FEW_MEAN on average.
+constexpr int RASTER_FEW_MEAN = 24;
+inline int raster_few(long long entries, long long tiles) { return tiles > 0 && entries <= RASTER_FEW_MEAN * tiles; }
 // raster_f64.cu / raster_f32.cu
 void launch_raster_f64(const RasterArgs &a, cudaStream_t s);
 void launch_raster_f32(const RasterArgs &a, cudaStream_t s);

@@ -230,6 +230,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     int *dcount = static_cast<int *>(c->bin_count.p);
     // bins sized from the previous call's fullest tile; a tile that still
     // overflows takes the raster's ordered full-scan path (same results)
+    long long entries = 0, busy = 0;
     for (int pass = 0; pass < 2; pass++) {
         if (int r2 = grow(c->bin_ids, sizeof(int2) * (size_t)ntiles * c->cap)) return r2;
         launch_reset_state(dst, 1, dcount, ntiles, s);
@@ -240,7 +241,12 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
         PV_CK(cudaMemcpyAsync(counts.data(), dcount, sizeof(int) * ntiles, cudaMemcpyDeviceToHost, s));
         PV_CK(cudaStreamSynchronize(s));
         int mx = 0;
-        for (int v : counts) mx = std::max(mx, v);
+        entries = busy = 0;
+        for (int v : counts) {
+            mx = std::max(mx, v);
+            entries += v;
+            busy += v > 0;
+        }
         if (mx <= c->cap || pass == 1) break;
         while (c->cap < mx && c->cap < 8192) c->cap *= 2;
     }
@@ -265,6 +271,7 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     ra.keep_pos = 1;
     ra.accumulate = 1;
     ra.mode = RASTER_POS;
+    ra.few = raster_few(entries, busy);
     ra.won = static_cast<unsigned char *>(c->won.p);
     launch_raster_f64(ra, s);
     PV_CK(cudaGetLastError());

@@ -639,6 +639,25 @@ struct PixelHit {
     double z, s, t, gs, gt;
 };
 
+// A facet's edges over a tile (facet_edges): t, s - t and 1 - s as linear functions
+// c0 + cx li + cy lj of the pixel, raised by what they may be off, and the rows
+// (bits 0-15) and columns (16-31) of its box.
+struct FacetEdges {
+    float c0[3], cx[3], cy[3];
+    unsigned box;
+};
+// A bin of few entries, most of many pixels: a coarse model in a large window. A
+// thread per facet that lists its pixels takes them one after the other while
+// its CTA waits, so in the kernels for such views (RasterArgs::few) phase A keeps
+// a bin's edges and boxes if it has at most FEW entries, and in phase B each
+// pixel tests all of them. Device time of an evaluation with lists and so, us,
+// FP32: one frame of 1001^2 pixels, 8000 facets, 142 and 109; 16 of 301^2, 128
+// facets, 123 and 98; 25 lightcurve points of up to 257^2, 512 facets, 110 and 78;
+// 4 frames of 511^2, 8192 facets, 131 and 118. With more entries the lists are as
+// fast (one frame of 801^2, 32768 facets, some 25 a tile: 146 with lists, 138
+// with FEW 24, 145 with 32).
+constexpr int FEW = 24;
+
 // Shared memory of a tile's CTA of NT threads. The exact terms of the bin's
 // facets are kept when the bin has at most NT of them (most tiles); otherwise a
 // pixel forms those of its own facets again.
@@ -647,7 +666,10 @@ struct TileShared {
     union {
         struct {
             double term[10][NT];                     // FacetTerms of bin entry k in column k
-            unsigned short cand[TILE_PIX][CAND];     // bin entries that may cover the pixel
+            union {
+                unsigned short cand[TILE_PIX][CAND]; // bin entries that may cover the pixel
+                FacetEdges edge[FEW];                // a bin of at most FEW entries: theirs
+            };
         };
         PixelHit hit[TILE_PIX];                      // tile_chunks: the outcome
         StageRow<T> stage[NT];                       // phase C: a row per thread
@@ -755,20 +777,27 @@ __device__ inline bool facet_entry(const RasterArgs &a, const FrameGeom &g, cons
     return true;
 }
 
-// The candidates of a pixel in turn: entry i (of cnt) of pixel p, or -1 where
-// the overflow list's slot i - CAND holds another pixel's.
+// The candidates of a pixel in turn: entry i (of candidates()) of pixel p, or -1
+// where the overflow list's slot i - CAND holds another pixel's. few: a bin of at
+// most FEW entries, the pixel's are the bits of sh.cnt; left: those to come.
 template <typename T, int NT>
-__device__ inline int candidate(const TileShared<T, NT> &sh, int p, int i)
+__device__ __forceinline__ int candidate(const TileShared<T, NT> &sh, bool few, int p, int i, unsigned &left)
 {
+    if (few) {
+        const int k = __ffs(left) - 1;
+        left &= left - 1;
+        return k;
+    }
     if (i < CAND) return sh.cand[p][i];
     const unsigned v = sh.more[i - CAND];
     return (int)(v >> 16) == p ? (int)(v & 0xffffu) : -1;
 }
 // How many to walk: the pixel's own, or all of the overflow list too.
 template <typename T, int NT>
-__device__ inline int candidates(const TileShared<T, NT> &sh, int p)
+__device__ __forceinline__ int candidates(const TileShared<T, NT> &sh, bool few, int p)
 {
     const int c = sh.cnt[p];
+    if (few) return __popc(c);
     return c <= CAND ? c : CAND + sh.n;
 }
 // Whether bin entry k covers the pixel centre (x0, y0): its terms, s and t.
@@ -789,20 +818,21 @@ __device__ inline bool entry_covers(const RasterArgs &a, const double4 *vt, cons
 // the first, 20 points of a 30 % rough body of 8192 facets took 348 us, 234
 // backwards; 16 frames of 511^2 pixels of 32768 facets with 3 % roughness 257 and
 // 240; 25 points of a smooth body the same.
-template <typename T, int NT>
-__device__ __noinline__ PixelHit pixel_history(const RasterArgs &a, const FrameGeom &g, const int2 *bin,
-                                               const TileShared<T, NT> &sh, bool staged, int p, int below, bool has,
-                                               double z0)
+template <typename T, int NT, bool FEW_VIEWS>
+__device__ __noinline__ PixelHit pixel_history(const RasterArgs &a, const FrameGeom &g, const int2 *bin, int count,
+                                               const TileShared<T, NT> &sh, int p, int below, bool has, double z0)
 {
+    const bool staged = count <= NT, few = FEW_VIEWS && count <= FEW;
     PixelHit h = {-1, -1, 0.0, 0.0, 0.0, 0.0, 0.0};
     const double4 *vt = static_cast<const double4 *>(a.vt) + g.vt_base;
     const double x0 = sh.xs[p / TILE_W], y0 = sh.ys[p % TILE_W];
-    const int nc = candidates<T, NT>(sh, p);
+    const int nc = candidates<T, NT>(sh, few, p);
     for (;;) {
+        unsigned left = sh.cnt[p];
         int bf = -1;
         double bz = 0.0, bs = 0.0, bt = 0.0;
         for (int i = 0; i < nc; i++) {
-            const int k = candidate<T, NT>(sh, p, i);
+            const int k = candidate<T, NT>(sh, few, p, i, left);
             if (k < 0) continue;
             const int f = bin[k].x;
             if (f >= below) continue;
@@ -824,29 +854,41 @@ __device__ __noinline__ PixelHit pixel_history(const RasterArgs &a, const FrameG
     }
 }
 
-// Phase A for one bin entry k of the tile whose first pixel centre is (x0, y0):
-// the pixels of each row of the facet's box that lie between its edges get the
-// entry as a candidate. In pixel units from the tile's corner, t, s - t and
-// 1 - s are linear functions c0 + cx li + cy lj; a pixel the exact test accepts
-// has them above -m, where m bounds the FP32 error of c0, cx and cy over the
-// box (one part in 10^6 of the coefficients times the offsets' magnitude,
-// several times the rounding of these few operations) and the exact test's own
-// 1e-10. Coefficients out of FP32's range bound nothing (the whole box). room:
-// entries that sh.more takes.
+// The edges of a facet of the tile whose first pixel centre is (x0, y0). In pixel
+// units from the tile's corner, t, s - t and 1 - s are linear functions
+// c0 + cx li + cy lj; a pixel the exact test accepts has them above -m, where m
+// bounds the FP32 error of c0, cx and cy over the box and the exact test's own
+// 1e-10. With u = 2^-24: A, den and kmpp rounded and multiplied give sx, sy, tx
+// and ty to 5u, X and Y are right to 3u, so s0 and t0 are off by at most
+// 10u mag (|X| + |Y|), their difference and the addition of m by 2u more, cx and
+// cy by 6u, and the sum at a pixel of the box adds 2u of its terms and 7u 30 mag
+// from cx and cy: in all 14u mag (|X| + |Y|) + 240u mag, 8.4e-7 and 1.5e-5 beside
+// m's 2e-6 and 6.4e-5. Coefficients out of FP32's range bound nothing (the whole
+// box).
+__device__ inline FacetEdges facet_edges(const FacetTerms &q, double x0, double y0, float ikm, double kmpp)
+{
+    const float d = (float)q.den * (float)kmpp;
+    const float sx = (float)q.A * d, sy = -(float)q.B * d, tx = -(float)q.D * d, ty = (float)q.C * d;
+    const float X = (float)(x0 - q.x) * ikm, Y = (float)(y0 - q.y) * ikm;
+    const float mag = fabsf(sx) + fabsf(sy) + fabsf(tx) + fabsf(ty);
+    const float m = 2e-6f * (1.0f + mag * (fabsf(X) + fabsf(Y) + 32.0f));
+    const float s0 = sx * X + sy * Y, t0 = tx * X + ty * Y;
+    FacetEdges e = {{t0 + m, s0 - t0 + m, 1.0f - s0 + m}, {tx, sx - tx, -sx}, {ty, sy - ty, -sy}, 0u};
+    if (!(m < 1e24f))
+        for (int k = 0; k < 3; k++) { e.c0[k] = 1.0f; e.cx[k] = e.cy[k] = 0.0f; }
+    return e;
+}
+
+// Phase A for bin entry k: the pixels of each row of the facet's box that lie
+// between its edges get the entry as a candidate. room: entries that sh.more
+// takes.
 template <typename T, int NT>
 __device__ inline void bound_facet(int k, const FacetTerms &q, int box, double x0, double y0, float ikm, double kmpp,
                                    int room, TileShared<T, NT> &sh)
 {
     const int ri1 = box & 15, ri2 = (box >> 4) & 15, rj1 = (box >> 8) & 15, rj2 = (box >> 12) & 15;
-    const float d = (float)q.den * (float)kmpp;
-    const float sx = (float)q.A * d, sy = -(float)q.B * d, tx = -(float)q.D * d, ty = (float)q.C * d;
-    const float X = (float)(x0 - q.x) * ikm, Y = (float)(y0 - q.y) * ikm;
-    const float mag = fabsf(sx) + fabsf(sy) + fabsf(tx) + fabsf(ty);
-    const float m = 1e-6f * (1.0f + mag * (fabsf(X) + fabsf(Y) + 32.0f));
-    const float s0 = sx * X + sy * Y, t0 = tx * X + ty * Y;
-    float c0[3] = {t0 + m, s0 - t0 + m, 1.0f - s0 + m}, cx[3] = {tx, sx - tx, -sx}, cy[3] = {ty, sy - ty, -sy};
-    if (!(m < 1e24f))
-        for (int e = 0; e < 3; e++) { c0[e] = 1.0f; cx[e] = cy[e] = 0.0f; }
+    const FacetEdges fe = facet_edges(q, x0, y0, ikm, kmpp);
+    const float *c0 = fe.c0, *cx = fe.cx, *cy = fe.cy;
     float inv[3];
 #pragma unroll
     for (int e = 0; e < 3; e++) inv[e] = -__fdividef(1.0f, fabsf(cy[e]));
@@ -872,6 +914,34 @@ __device__ inline void bound_facet(int k, const FacetTerms &q, int box, double x
             }
         }
     }
+}
+
+// Phase A for entry k of a bin of at most FEW: its edges and box, for the pixels to
+// test.
+template <typename T, int NT>
+__device__ inline void few_facet(int k, const FacetTerms &q, int box, double x0, double y0, float ikm, double kmpp,
+                                 TileShared<T, NT> &sh)
+{
+    FacetEdges e = facet_edges(q, x0, y0, ikm, kmpp);
+    // bits first .. last of a bound pair
+    auto span = [](int first, int last) { return (2u << last) - (1u << first); };
+    e.box = span(box & 15, (box >> 4) & 15) | span((box >> 8) & 15, (box >> 12) & 15) << 16;
+    sh.edge[k] = e;
+}
+// The entries (bits) of such a bin that may cover the tile's pixel (li, lj).
+template <typename T, int NT>
+__device__ inline unsigned few_candidates(const TileShared<T, NT> &sh, int count, int li, int lj)
+{
+    const float fi = (float)li, fj = (float)lj;
+    unsigned mask = 0;
+    for (int k = 0; k < count; k++) {
+        const FacetEdges &e = sh.edge[k];
+        bool in = (e.box >> li & e.box >> (16 + lj) & 1u) != 0;
+#pragma unroll
+        for (int j = 0; j < 3; j++) in = in && e.c0[j] + e.cx[j] * fi + e.cy[j] * fj >= 0.0f;
+        mask |= (unsigned)in << k;
+    }
+    return mask;
 }
 
 // A tile whose bin overflowed its capacity (then: all facets that meet the tile),
@@ -954,9 +1024,10 @@ __device__ __noinline__ void tile_chunks(const RasterArgs &a, const FrameGeom &g
             for (int r = 0; r < PP; r++) {
                 if (below[r] == 0) continue;
                 const int p = tid + r * NT, li = p / TILE_W, lj = p % TILE_W;
-                const int nc = all ? m : candidates<T, NT>(sh, p);
+                unsigned none = 0;
+                const int nc = all ? m : candidates<T, NT>(sh, false, p);
                 for (int i = 0; i < nc; i++) {
-                    const int k = all ? i : candidate<T, NT>(sh, p, i);
+                    const int k = all ? i : candidate<T, NT>(sh, false, p, i, none);
                     if (k < 0) continue;
                     const int2 e = sh.fl[k];
                     const int b = e.y;
@@ -1047,7 +1118,8 @@ template <typename T, int MODE> __host__ __device__ constexpr int raster_warps()
     return MODE == RASTER_SUN || MODE == RASTER_PHOTO ? RASTER_WARPS_MAPS
          : sizeof(T) == 4 ? RASTER_WARPS_F32 : RASTER_WARPS_F64;
 }
-template <typename T, int NT, int MODE>
+// FEW_VIEWS: bins of at most FEW entries are not listed.
+template <typename T, int NT, int MODE, bool FEW_VIEWS>
 __global__ void __launch_bounds__(NT, raster_warps<T, MODE>() * 32 / NT)
 k_raster(const __grid_constant__ RasterArgs a)
 {
@@ -1110,14 +1182,15 @@ k_raster(const __grid_constant__ RasterArgs a)
 
         // ---- A: facets to pixels
         bool slow = count > a.cap || count > 65536;      // a candidate is held in 16 bits
-        const bool staged = count <= NT;
+        const bool staged = count <= NT, few = FEW_VIEWS && count <= FEW;
         if (!slow) {
             const float ikm = (float)g.ikm;
             for (int k = tid; k < count; k += NT) {
                 const int2 e = bin[k];
                 const FacetTerms q = facet_terms(vt, a.fvi[e.x]);
                 if (staged) store_terms<T, NT>(sh, k, q);
-                bound_facet<T, NT>(k, q, e.y, x0, y0, ikm, g.kmpp, CAND_MORE, sh);
+                if (few) few_facet<T, NT>(k, q, e.y, x0, y0, ikm, g.kmpp, sh);
+                else bound_facet<T, NT>(k, q, e.y, x0, y0, ikm, g.kmpp, CAND_MORE, sh);
             }
             __syncthreads();
             slow = sh.n > CAND_MORE;
@@ -1144,9 +1217,11 @@ k_raster(const __grid_constant__ RasterArgs a)
                 h = sh.hit[p];
             } else {
                 const double xp = sh.xs[li], yp = sh.ys[lj];
-                const int nc = candidates<T, NT>(sh, p);
+                if (few) sh.cnt[p] = few_candidates<T, NT>(sh, count, li, lj);
+                const int nc = candidates<T, NT>(sh, few, p);
+                unsigned left = sh.cnt[p];
                 for (int i = 0; i < nc; i++) {
-                    const int k = candidate<T, NT>(sh, p, i);
+                    const int k = candidate<T, NT>(sh, few, p, i, left);
                     FacetTerms q;
                     double s, t;
                     if (k < 0 || !entry_covers<T, NT>(a, vt, bin, sh, staged, k, xp, yp, q, s, t)) continue;
@@ -1215,7 +1290,7 @@ k_raster(const __grid_constant__ RasterArgs a)
                         faces = view_row64(g, 2, m) > 0.0;
                     }
                     if (!faces) {
-                        const PixelHit c = pixel_history<T, NT>(a, g, bin, sh, staged, p, h.f, had, had_z);
+                        const PixelHit c = pixel_history<T, NT, FEW_VIEWS>(a, g, bin, count, sh, p, h.f, had, had_z);
                         h.gf = c.gf; h.gs = c.gs; h.gt = c.gt;
                         if (h.gf >= 0) normal();
                     }
@@ -1355,15 +1430,22 @@ k_raster(const __grid_constant__ RasterArgs a)
 // variant 0: 256 threads per tile; 1: 128 (two pixels a thread, smaller CTAs).
 // f(kernel, threads) for the kernel that a's mode and variant select (a single
 // POS view is one launch of a few tiles: 256 threads).
+template <typename T, int MODE, typename F>
+inline void with_raster_kernel_of(const RasterArgs &a, F f)
+{
+    if (a.variant == 1 && MODE != RASTER_POS)
+        return a.few ? f(k_raster<T, 128, MODE, true>, 128) : f(k_raster<T, 128, MODE, false>, 128);
+    return a.few ? f(k_raster<T, 256, MODE, true>, 256) : f(k_raster<T, 256, MODE, false>, 256);
+}
 template <typename T, typename F>
 inline void with_raster_kernel(const RasterArgs &a, F f)
 {
     if constexpr (sizeof(T) == 8) {
-        if (a.mode == RASTER_SUN) return a.variant == 1 ? f(k_raster<T, 128, RASTER_SUN>, 128) : f(k_raster<T, 256, RASTER_SUN>, 256);
-        if (a.mode == RASTER_POS) return f(k_raster<T, 256, RASTER_POS>, 256);
-        if (a.mode == RASTER_PHOTO) return a.variant == 1 ? f(k_raster<T, 128, RASTER_PHOTO>, 128) : f(k_raster<T, 256, RASTER_PHOTO>, 256);
+        if (a.mode == RASTER_SUN) return with_raster_kernel_of<T, RASTER_SUN>(a, f);
+        if (a.mode == RASTER_POS) return with_raster_kernel_of<T, RASTER_POS>(a, f);
+        if (a.mode == RASTER_PHOTO) return with_raster_kernel_of<T, RASTER_PHOTO>(a, f);
     }
-    return a.variant == 1 ? f(k_raster<T, 128, RASTER_RADAR>, 128) : f(k_raster<T, 256, RASTER_RADAR>, 256);
+    return with_raster_kernel_of<T, RASTER_RADAR>(a, f);
 }
 
 template <typename T>
@@ -1381,10 +1463,13 @@ inline cudaError_t configure_raster_t()
     cudaError_t e = cudaSuccess;
     RasterArgs a = {};
     for (a.mode = RASTER_RADAR; a.mode <= (sizeof(T) == 8 ? RASTER_POS : RASTER_RADAR); a.mode++)
-        for (a.variant = 0; a.variant < 2 && e == cudaSuccess; a.variant++)
+        for (int k = 0; k < 4 && e == cudaSuccess; k++) {
+            a.variant = k & 1;
+            a.few = k >> 1;
             with_raster_kernel<T>(a, [&](auto kern, int) {
                 e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, RASTER_SHARED_PCT);
             });
+        }
     return e;
 }
 

@@ -35,6 +35,7 @@ def _rough(levels, sigma, seed):
 
 # (octahedron levels, roughness, POS half width, smoothing)
 GRID = [
+    (2, 0.5, 45, 1),        # tiles of few facets
     (3, 0.4, 20, 1),
     (4, 0.45, 15, 0),
     (5, 0.6, 15, 1),        # pixels past their own candidate lists

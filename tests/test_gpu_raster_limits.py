@@ -1,6 +1,7 @@
 """Tiles past the raster's lists, rastered in chunks of facets: chunks whose own
 candidates overflow, scans of all facets that meet a tile whose bin is full,
-limb pixels whose cosine is several winners back. Maps equal the oracle's in
+limb pixels whose cosine is several winners back. And coarse bodies, whose tiles
+hold few facets of many pixels. Maps equal the oracle's in
 every form and kernel, cos(e) in the FP64 forms; lightcurve views' too."""
 import numpy as np
 import pytest
@@ -42,6 +43,13 @@ GRID = [
     (6, 0.95, 7, 1, 64),        # one tile of 15^2 pixels scanned out of 32768 facets
     (4, 0.45, 15, 0, 32),       # facet normals
     (2, 0.3, 40, 1, 1),         # few facets, each over several tiles
+    # coarse bodies: tiles of few entries, whose pixels test all of them
+    (0, 0.0, 33, 1, 0),         # 8 facets, edges through pixel centres
+    (1, 0.5, 60, 1, 0),
+    (2, 0.6, 50, 1, 0),         # limb pixels among them
+    (3, 0.5, 50, 1, 0),         # some tiles of more than FEW entries
+    (3, 0.5, 50, 0, 0),
+    (2, 0.6, 50, 1, 5),         # few entries, full bins
 ]
 
 
@@ -59,7 +67,7 @@ def test_radar(cuda_device, levels, sigma, n, smooth, cap):
                 assert np.array_equal(g[k], o["pos"][f][k]), (form, mode, f, k)
 
 
-@pytest.mark.parametrize("levels,sigma,pos,cap", [(6, 0.95, 31, 0), (4, 0.45, 41, 16)])
+@pytest.mark.parametrize("levels,sigma,pos,cap", [(6, 0.95, 31, 0), (4, 0.45, 41, 16), (2, 0.5, 101, 0)])
 def test_lightcurve(cuda_device, levels, sigma, pos, cap):
     m = _rough(levels, sigma)
     p = synth.eval_params(mask_tol=0.0)
