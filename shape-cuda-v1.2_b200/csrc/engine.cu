@@ -1433,12 +1433,15 @@ int EngineImpl::raster_grid(int form, int nonempty, const RasterArgs &a, bool f3
 namespace {
 // Raster choices by size class, shared by the engines of the process (the
 // server's clones of one dataset tune once).
+// busy: the non-empty tiles of the radar, sun and observer views, each part a
+// launch of kernels of its own; few: bit k where part k has the kernels for few
+// facets per tile.
 struct TuneKey {
-    int device, form, exact, nviews, nf, nonempty, maxcount;
+    int device, form, exact, nviews, nf, busy[3], few, maxcount;
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(device, form, exact, nviews, nf, nonempty, maxcount) <
-               std::tie(o.device, o.form, o.exact, o.nviews, o.nf, o.nonempty, o.maxcount);
+        return std::tie(device, form, exact, nviews, nf, busy[0], busy[1], busy[2], few, maxcount) <
+               std::tie(o.device, o.form, o.exact, o.nviews, o.nf, o.busy[0], o.busy[1], o.busy[2], o.few, o.maxcount);
     }
 };
 struct TuneChoice {
@@ -1451,8 +1454,10 @@ std::map<TuneKey, TuneChoice> tune_cache;
 // The tuning file (SHAPE_B200_TUNING_CACHE names it; none by default): one
 // JSON object per line and size class, keyed by the GPU's name and SM count
 // so that a file carried to another machine of the same kind is reused and
-// one of another kind is ignored. Read once per device, rewritten whenever
-// a new size class is tuned.
+// one of another kind is ignored, as is a line of other kernels (TUNE_KERNELS:
+// the choices that its numbers mean, raised when those change). Read once per
+// device, rewritten whenever a new size class is tuned.
+constexpr int TUNE_KERNELS = 2;
 std::string gpu_tag(int device)
 {
     cudaDeviceProp pr;
@@ -1476,14 +1481,15 @@ void tune_file_load(int device)
     while (fgets(line, sizeof line, fp)) {
         TuneKey k{};
         TuneChoice c{};
+        int kernels = 0;
         if (sscanf(line,
-                   "{\"gpu\": \"%255[^\"]\", \"form\": %d, \"exact\": %d, \"views\": %d, \"facets\": %d, "
-                   "\"nonempty\": %d, \"maxcount16\": %d, \"variant\": %d, \"persistent\": %d, "
-                   "\"ms\": [%lf, %lf, %lf, %lf]}",
-                   gpu, &k.form, &k.exact, &k.nviews, &k.nf, &k.nonempty, &k.maxcount, &c.variant, &c.persistent,
-                   &c.ms[0], &c.ms[1], &c.ms[2], &c.ms[3]) != 13)
+                   "{\"gpu\": \"%255[^\"]\", \"kernels\": %d, \"form\": %d, \"exact\": %d, \"views\": %d, "
+                   "\"facets\": %d, \"nonempty\": [%d, %d, %d], \"few\": %d, \"maxcount16\": %d, "
+                   "\"variant\": %d, \"persistent\": %d, \"ms\": [%lf, %lf, %lf, %lf]}",
+                   gpu, &kernels, &k.form, &k.exact, &k.nviews, &k.nf, &k.busy[0], &k.busy[1], &k.busy[2], &k.few,
+                   &k.maxcount, &c.variant, &c.persistent, &c.ms[0], &c.ms[1], &c.ms[2], &c.ms[3]) != 17)
             continue;
-        if (tag != gpu || c.variant < 0 || c.variant > 1 || c.persistent < 0 || c.persistent > 1) continue;
+        if (tag != gpu || kernels != TUNE_KERNELS || c.variant < 0 || c.variant > 1 || c.persistent < 0 || c.persistent > 1) continue;
         k.device = device;
         tune_cache.emplace(k, c);
     }
@@ -1503,11 +1509,11 @@ void tune_file_save()
         const TuneChoice &c = kv.second;
         if (!tags.count(k.device)) tags[k.device] = gpu_tag(k.device);
         fprintf(fp,
-                "{\"gpu\": \"%s\", \"form\": %d, \"exact\": %d, \"views\": %d, \"facets\": %d, "
-                "\"nonempty\": %d, \"maxcount16\": %d, \"variant\": %d, \"persistent\": %d, "
-                "\"ms\": [%.6g, %.6g, %.6g, %.6g]}\n",
-                tags[k.device].c_str(), k.form, k.exact, k.nviews, k.nf, k.nonempty, k.maxcount, c.variant,
-                c.persistent, c.ms[0], c.ms[1], c.ms[2], c.ms[3]);
+                "{\"gpu\": \"%s\", \"kernels\": %d, \"form\": %d, \"exact\": %d, \"views\": %d, "
+                "\"facets\": %d, \"nonempty\": [%d, %d, %d], \"few\": %d, \"maxcount16\": %d, "
+                "\"variant\": %d, \"persistent\": %d, \"ms\": [%.6g, %.6g, %.6g, %.6g]}\n",
+                tags[k.device].c_str(), TUNE_KERNELS, k.form, k.exact, k.nviews, k.nf, k.busy[0], k.busy[1],
+                k.busy[2], k.few, k.maxcount, c.variant, c.persistent, c.ms[0], c.ms[1], c.ms[2], c.ms[3]);
     }
     fclose(fp);
     rename(tmp.c_str(), path);
@@ -1520,7 +1526,8 @@ void tune_file_save()
 int EngineImpl::autotune(int form)
 {
     const TuneKey key{device, form, form == SHAPE_FORM_BATCHED_FP32 ? fp32_exact : 0, nviews, nf,
-                      tuned_nonempty, tuned_max_count / 16};
+                      {work_busy[0], work_busy[1], work_busy[2]},
+                      work_few[0] | work_few[1] << 1 | work_few[2] << 2, tuned_max_count / 16};
     {
         std::lock_guard<std::mutex> lk(tune_mu);
         tune_file_load(device);
