@@ -624,19 +624,6 @@ def main():
     kpe = E.kernels_per_eval(form)
     stages = E.stage_times(form if form != eng.FORM_PLAIN_FP64 else eng.FORM_BATCHED_FP64)
 
-    # the FP32 form with shape_engine_set_fp32_exact(0) (accepted, without
-    # effect: coverage is FP64 in every form), a short run beside the default
-    fast = None
-    if form == eng.FORM_BATCHED_FP32 and not lcs and not args.no_plain:
-        E.set_fp32_exact(False)
-        fx_ms, _ = run(form, max(20, min(args.steps, 100)), 3, False)
-        E.set_scale(0, trial(0))           # both forms at the same scale factors
-        c64 = E.evaluate(eng.FORM_BATCHED_FP64)["chi2"]
-        c32f = E.evaluate(form)["chi2"]
-        E.set_fp32_exact(True)
-        fast = {"frame_evals_per_s": nu / (statistics.mean(fx_ms) / 1e3), "ms_per_step": statistics.mean(fx_ms),
-                "dchi2_rel_fp32_vs_fp64": abs(c32f - c64) / abs(c64)}
-
     total_dev = sum(dev_ms)
     total_host = sum(host_ms)
     units_all = ws * nu
@@ -683,7 +670,6 @@ def main():
                    "dchi2_rel_per_frame_fp32_vs_fp64": dchi_frames,
                    "plain_fp64_frame_evals_per_s": plain_rate,
                    "batched_over_plain_fp64": value / ws / plain_rate,
-                   "fp32_fast_option": fast,
                    "p50_ms": statistics.median(dev_ms), "p99_ms": float(np.percentile(dev_ms, 99)),
                    "stage_ms": stages,
                    "step_algorithmic_bytes": step_bytes,

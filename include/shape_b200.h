@@ -193,9 +193,9 @@ int shape_engine_stage_times(shape_engine *e, int form, double *ms, int max);
 int shape_engine_set_bin_capacity(shape_engine *e, int cap);
 /* Batched FP32 form, radar views. Coverage and depth are evaluated in FP64 in
  * every form, so the FP32 form's facet and depth maps are the FP64 form's with
- * either value; the switch is kept for callers that set it (it used to admit
- * decisions in FP32, which were faster then). Takes effect at the next
- * evaluation. */
+ * either value and it changes nothing, the raster's tuning included; the switch
+ * is kept for callers that set it (it used to admit decisions in FP32, which
+ * were faster then). */
 int shape_engine_set_fp32_exact(shape_engine *e, int exact);
 /* vary_params (src/shape/vary_params.c:84-327): the four means the
  * reference computes for its joint adjustments of the 0th delay-correction

@@ -1437,11 +1437,11 @@ namespace {
 // launch of kernels of its own; few: bit k where part k has the kernels for few
 // facets per tile.
 struct TuneKey {
-    int device, form, exact, nviews, nf, busy[3], few, maxcount;
+    int device, form, nviews, nf, busy[3], few, maxcount;
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(device, form, exact, nviews, nf, busy[0], busy[1], busy[2], few, maxcount) <
-               std::tie(o.device, o.form, o.exact, o.nviews, o.nf, o.busy[0], o.busy[1], o.busy[2], o.few, o.maxcount);
+        return std::tie(device, form, nviews, nf, busy[0], busy[1], busy[2], few, maxcount) <
+               std::tie(o.device, o.form, o.nviews, o.nf, o.busy[0], o.busy[1], o.busy[2], o.few, o.maxcount);
     }
 };
 struct TuneChoice {
@@ -1483,11 +1483,11 @@ void tune_file_load(int device)
         TuneChoice c{};
         int kernels = 0;
         if (sscanf(line,
-                   "{\"gpu\": \"%255[^\"]\", \"kernels\": %d, \"form\": %d, \"exact\": %d, \"views\": %d, "
+                   "{\"gpu\": \"%255[^\"]\", \"kernels\": %d, \"form\": %d, \"views\": %d, "
                    "\"facets\": %d, \"nonempty\": [%d, %d, %d], \"few\": %d, \"maxcount16\": %d, "
                    "\"variant\": %d, \"persistent\": %d, \"ms\": [%lf, %lf, %lf, %lf]}",
-                   gpu, &kernels, &k.form, &k.exact, &k.nviews, &k.nf, &k.busy[0], &k.busy[1], &k.busy[2], &k.few,
-                   &k.maxcount, &c.variant, &c.persistent, &c.ms[0], &c.ms[1], &c.ms[2], &c.ms[3]) != 17)
+                   gpu, &kernels, &k.form, &k.nviews, &k.nf, &k.busy[0], &k.busy[1], &k.busy[2], &k.few,
+                   &k.maxcount, &c.variant, &c.persistent, &c.ms[0], &c.ms[1], &c.ms[2], &c.ms[3]) != 16)
             continue;
         if (tag != gpu || kernels != TUNE_KERNELS || c.variant < 0 || c.variant > 1 || c.persistent < 0 || c.persistent > 1) continue;
         k.device = device;
@@ -1509,10 +1509,10 @@ void tune_file_save()
         const TuneChoice &c = kv.second;
         if (!tags.count(k.device)) tags[k.device] = gpu_tag(k.device);
         fprintf(fp,
-                "{\"gpu\": \"%s\", \"kernels\": %d, \"form\": %d, \"exact\": %d, \"views\": %d, "
+                "{\"gpu\": \"%s\", \"kernels\": %d, \"form\": %d, \"views\": %d, "
                 "\"facets\": %d, \"nonempty\": [%d, %d, %d], \"few\": %d, \"maxcount16\": %d, "
                 "\"variant\": %d, \"persistent\": %d, \"ms\": [%.6g, %.6g, %.6g, %.6g]}\n",
-                tags[k.device].c_str(), TUNE_KERNELS, k.form, k.exact, k.nviews, k.nf, k.busy[0], k.busy[1],
+                tags[k.device].c_str(), TUNE_KERNELS, k.form, k.nviews, k.nf, k.busy[0], k.busy[1],
                 k.busy[2], k.few, k.maxcount, c.variant, c.persistent, c.ms[0], c.ms[1], c.ms[2], c.ms[3]);
     }
     fclose(fp);
@@ -1525,7 +1525,7 @@ void tune_file_save()
 // fastest. Runs before the form's first evaluation.
 int EngineImpl::autotune(int form)
 {
-    const TuneKey key{device, form, form == SHAPE_FORM_BATCHED_FP32 ? fp32_exact : 0, nviews, nf,
+    const TuneKey key{device, form, nviews, nf,
                       {work_busy[0], work_busy[1], work_busy[2]},
                       work_few[0] | work_few[1] << 1 | work_few[2] << 2, tuned_max_count / 16};
     {
@@ -2328,10 +2328,7 @@ int shape_engine_get_active(shape_engine *h, unsigned char *vertex_act, unsigned
 int shape_engine_set_fp32_exact(shape_engine *h, int exact)
 {
     if (!h || (exact != 0 && exact != 1)) return shape::set_err(SHAPE_E_ARG, "set_fp32_exact: 0 or 1");
-    shape::EngineImpl &E = h->impl;
-    if (E.fp32_exact != exact) E.tuned[SHAPE_FORM_BATCHED_FP32] = 0;
-    E.fp32_exact = exact;
-    return SHAPE_OK;
+    return SHAPE_OK;            // coverage is FP64 with either value
 }
 
 int shape_engine_set_spin_device(shape_engine *h, int on)

@@ -286,7 +286,6 @@ struct EngineImpl {
         dof = o.dof; dof_deldop = o.dof_deldop; dof_doppler = o.dof_doppler; dof_lghtcrv = o.dof_lghtcrv;
         frame_sdev = o.frame_sdev;
         fixed_cap = o.fixed_cap;
-        fp32_exact = o.fp32_exact;
         tune_mode = o.tune_mode;
         have_spin = o.have_spin; spin_st = o.spin_st;
         spin_angleoff = o.spin_angleoff; spin_omegaoff = o.spin_omegaoff;
@@ -302,7 +301,6 @@ struct EngineImpl {
     // whether those held few facets each (RasterArgs::few)
     int work_n[3] = {0, 0, 0}, work_busy[3] = {0, 0, 0}, work_few[3] = {0, 0, 0};
     int fixed_cap = 0;            // > 0: bin capacity set by the caller, no autotuning
-    int fp32_exact = 1;           // shape_engine_set_fp32_exact (part of the tuning key only)
     // Raster kernel per form (RasterArgs::variant) and grid (0: one CTA per
     // tile that was non-empty at bin tuning; 1: persistent, resident CTAs x
     // SMs striding over the tiles). tune_mode -1: the first batched

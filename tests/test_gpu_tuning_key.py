@@ -87,3 +87,17 @@ def test_lines_of_other_builds_are_not_taken(cuda_device, tmp_path, line):
     # a line of this build's is
     path.write_text(json.dumps(dict(rec, ms=planted)) + "\n")
     assert _run(path)["ms"] == planted
+
+
+def test_fp32_exact_keeps_the_choice(cuda_device):
+    """The switch changes no result, so it does not have the form timed again."""
+    m, p, ds = cases.c2(12)
+    e = eng.make_engine(m, p, deldops=[ds])
+    e.evaluate(eng.FORM_BATCHED_FP32)
+    a = e.raster_tuning(eng.FORM_BATCHED_FP32)
+    for exact in (False, True):
+        e.set_fp32_exact(exact)
+        assert e.raster_tuning(eng.FORM_BATCHED_FP32) == a and a["tuned"]
+        e.evaluate(eng.FORM_BATCHED_FP32)
+        assert e.raster_tuning(eng.FORM_BATCHED_FP32) == a
+    e.close()
