@@ -1310,6 +1310,12 @@ void launch_xform_f64(const FrameGeom *g, int nviews, const double4 *vx, int nv,
 void launch_bin_f64(const FrameGeom *g, int view0, int nviews, const ModelDev &m, const double4 *vt,
                     FrameState *st, int *bin_count, int2 *bin_ids, int cap, cudaStream_t s, bool pdl, bool vnormals)
 {
+    // the vertex normals' blocks are one more row of the grid; where the views
+    // take all that a grid may have (65535), a launch of their own
+    if (vnormals && nviews + 1 > 65535) {
+        launch_realize_vn(m, s);
+        vnormals = false;
+    }
     dim3 grid((m.nf + 255) / 256, nviews + (vnormals ? 1 : 0));
     const VnormalArgs vna = {vnormals ? m.nv : 0, m.af_ptr, m.af_idx, m.vn, m.vnf};
     launch_k(k_bin<double4>, grid, dim3(256), 0, s, pdl, g, view0, m.nf, (const int4 *)m.fvi, (const double4 *)m.fn,

@@ -1301,9 +1301,9 @@ int EngineImpl::enqueue(int form, cudaEvent_t *marks)
 // and copies excluded).
 int EngineImpl::kernels_per_eval(int form) const
 {
-    // front (and binning), or realize (vertices + facets, vertex normals) and the
-    // state reset
-    int n = form == SHAPE_FORM_PLAIN_FP64 ? 3 : front_bins() ? 1 : 2;
+    // front, binning and (launch_bin_f64) vertex normals, or realize (vertices +
+    // facets, vertex normals) and the state reset
+    int n = form == SHAPE_FORM_PLAIN_FP64 ? 3 : front_bins() ? 1 : nviews < 65535 ? 2 : 3;
     n += (spin_device && n_spin_src > 0) ? 1 : 0;   // view realization from the spin state
     if (form == SHAPE_FORM_PLAIN_FP64) {
         n += 3 * nviews;
