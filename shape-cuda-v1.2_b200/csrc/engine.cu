@@ -1575,40 +1575,80 @@ int EngineImpl::autotune(int form)
     return SHAPE_OK;
 }
 
-// Copies device ranges to the host, in one stream synchronization and through
-// the engine's pinned buffer (a pageable copy of its own per range took 14 us
-// for any small one and 110 for a 181^2 sky frame's three). Ranges larger than
-// the buffer may grow to are copied straight.
+// Floats to doubles, one by one: as vectors the compiler passes their upper halves
+// through the stack, and 262144 of them took 446 us instead of 150. They come
+// through a block that stays in the cache, as a wide copy reads the pinned
+// buffer faster than single loads do.
+#if defined(__GNUC__) && !defined(__clang__)
+__attribute__((optimize("no-tree-vectorize")))
+#endif
+static void widen(double *to, const unsigned char *from, size_t n)
+{
+    float block[2048];
+    for (size_t k0 = 0; k0 < n; k0 += 2048) {
+        const size_t m = std::min<size_t>(2048, n - k0);
+        memcpy(block, from + sizeof(float) * k0, sizeof(float) * m);
+        for (size_t k = 0; k < m; k++) to[k0 + k] = block[k];
+    }
+}
+
+// Copies device ranges to the host through the engine's pinned buffer (a pageable
+// copy of its own per range took 14 us for any small one and 110 for a 181^2 sky
+// frame's three): one stream synchronization where they fit READBACK_BUFFER, one
+// per buffer up to READBACK_MAX, beyond it straight copies. The buffer stays
+// small because its allocation is part of the first read: growing it to 2 MB took
+// 1.3 ms and more of that, to 4 MB 3 to 8, while 2.1 MB through 1 MB take 242 us
+// and through 2 MB 235.
 int EngineImpl::read_back(std::initializer_list<ReadBack> parts)
 {
     size_t total = 0;
-    for (const ReadBack &p : parts) total += (p.bytes + 15) & ~(size_t)15;
-    if (total > READBACK_MAX) {
+    bool floats = false;
+    for (const ReadBack &p : parts) {
+        total += (p.bytes + 15) & ~(size_t)15;
+        floats = floats || p.widen;
+    }
+    if (total > READBACK_MAX && !floats) {
         CK(cudaStreamSynchronize(stream));
         for (const ReadBack &p : parts)
             if (p.bytes) CK(cudaMemcpy(p.dst, p.src, p.bytes, cudaMemcpyDeviceToHost));
         return SHAPE_OK;
     }
     std::lock_guard<std::mutex> lk(read_mu);         // results may be read from several threads
-    if (total > h_read_bytes) {
+    if (total > h_read_bytes && h_read_bytes < READBACK_BUFFER) {
         size_t want = h_read_bytes ? h_read_bytes : (size_t)1 << 16;
-        while (want < total) want *= 2;
+        while (want < total && want < READBACK_BUFFER) want *= 2;
         if (h_read) { cudaFreeHost(h_read); h_read = nullptr; h_read_bytes = 0; }
         CK(cudaMallocHost((void **)&h_read, want));
         h_read_bytes = want;
     }
+    // the pieces of the parts that the buffer holds
+    struct Piece { unsigned char *dst; size_t off, bytes; bool widen; };
+    std::vector<Piece> pieces;
     size_t off = 0;
+    auto flush = [&]() -> int {
+        CK(cudaStreamSynchronize(stream));
+        for (const Piece &q : pieces) {
+            if (q.widen) widen(reinterpret_cast<double *>(q.dst), h_read + q.off, q.bytes / sizeof(float));
+            else memcpy(q.dst, h_read + q.off, q.bytes);
+        }
+        pieces.clear();
+        off = 0;
+        return SHAPE_OK;
+    };
     for (const ReadBack &p : parts) {
-        if (p.bytes) CK(cudaMemcpyAsync(h_read + off, p.src, p.bytes, cudaMemcpyDeviceToHost, stream));
-        off += (p.bytes + 15) & ~(size_t)15;
+        unsigned char *dst = static_cast<unsigned char *>(p.dst);
+        for (size_t done = 0; done < p.bytes;) {
+            if (off == h_read_bytes)
+                if (int rc = flush()) return rc;
+            const size_t n = std::min(p.bytes - done, h_read_bytes - off);
+            CK(cudaMemcpyAsync(h_read + off, static_cast<const unsigned char *>(p.src) + done, n,
+                               cudaMemcpyDeviceToHost, stream));
+            pieces.push_back(Piece{dst + done * (p.widen ? 2 : 1), off, n, p.widen});
+            off += (n + 15) & ~(size_t)15;
+            done += n;
+        }
     }
-    CK(cudaStreamSynchronize(stream));
-    off = 0;
-    for (const ReadBack &p : parts) {
-        if (p.bytes) memcpy(p.dst, h_read + off, p.bytes);
-        off += (p.bytes + 15) & ~(size_t)15;
-    }
-    return SHAPE_OK;
+    return flush();
 }
 
 // 1 when the last launch has completed on the device, 0 otherwise.
@@ -2065,17 +2105,8 @@ int shape_engine_get_fit(shape_engine *h, int frame, double *fit)
     size_t D = (size_t)E.frames[frame].ndel * E.frames[frame].ndop;
     long long off = E.frame_off[frame];
     cudaSetDevice(E.device);
-    if (E.last_form == SHAPE_FORM_BATCHED_FP32) {
-        // the floats land in the upper half of fit and spread upwards from there
-        float *tmp = reinterpret_cast<float *>(fit) + D;
-        if (int rc = E.read_back({{tmp, E.d_fit32 + off, sizeof(float) * D}})) return rc;
-        for (size_t k = 0; k < D; k++) {
-            float v;
-            memcpy(&v, tmp + k, sizeof v);
-            fit[k] = v;
-        }
-        return SHAPE_OK;
-    }
+    if (E.last_form == SHAPE_FORM_BATCHED_FP32)
+        return E.read_back({{fit, E.d_fit32 + off, sizeof(float) * D, true}});
     return E.read_back({{fit, E.d_fit64 + off, sizeof(double) * D}});
 }
 

@@ -259,9 +259,10 @@ struct EngineImpl {
     int enqueue(int form, cudaEvent_t *marks = nullptr);
     int launch(int form);
     // device ranges to copy out (bytes 0: skipped), and the pinned buffer they
-    // pass through: grown on demand, at most READBACK_MAX bytes
-    struct ReadBack { void *dst; const void *src; size_t bytes; };
-    static constexpr size_t READBACK_MAX = (size_t)4 << 20;
+    // pass through: grown on demand, at most READBACK_BUFFER bytes
+    // (widen: bytes of floats, to doubles)
+    struct ReadBack { void *dst; const void *src; size_t bytes; bool widen = false; };
+    static constexpr size_t READBACK_BUFFER = (size_t)1 << 20, READBACK_MAX = (size_t)4 << 20;
     unsigned char *h_read = nullptr;
     size_t h_read_bytes = 0;
     std::mutex read_mu;
