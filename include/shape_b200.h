@@ -179,17 +179,17 @@ int shape_engine_get_realized(shape_engine *e, double *x, double *vn, double *fn
 /* Runs one evaluation of a batched form stage by stage, with CUDA events
  * between the stages, and writes the stage times in ms: [0] realize, [1] state
  * reset and image clears, [2] view transforms, [3] facet binning,
- * [4] tile raster + delay-Doppler synthesis, [5] chi-square partials,
- * [6] lightcurve shadowing + photometry, [7] finalize + summary. Datasets
- * whose chi-square partials, frame results and totals run as one kernel
- * (every radar frame's chunk list fits its staging) time that kernel in [7]
- * and leave [5] empty. Returns the number of stages written. */
+ * [4] tile raster with delay-Doppler synthesis, shadowing and photometry,
+ * [5] and [6] empty (kept for callers that index the stages), [7] sky frames,
+ * lightcurves, chi-square, results and totals. [0] to [3] are launches of their
+ * own here; an evaluation does this work in its first one or two. Returns the
+ * number of stages written. */
 int shape_engine_stage_times(shape_engine *e, int form, double *ms, int max);
 
 /* Facet-bin capacity per 16x16 POS tile. 0 (default) lets finalize size it
  * from a dry-run binning of the model (next power of two above 1.25x the
- * fullest tile); tiles whose bin overflows are rasterized by scans of all
- * facets, which are exact but slow. Takes effect at the next finalize. */
+ * fullest tile); a tile whose bin overflows is rasterized from a scan of all
+ * facets, which is exact but slower. Takes effect at the next finalize. */
 int shape_engine_set_bin_capacity(shape_engine *e, int cap);
 /* Batched FP32 form, radar views. Coverage and depth are evaluated in FP64 in
  * every form, so the FP32 form's facet and depth maps are the FP64 form's with
@@ -244,7 +244,7 @@ int shape_engine_get_raster_tuning(shape_engine *e, int form, int *variant, int 
  * the engine's stream, so the next evaluation of every form sees them and
  * nothing is rebuilt; the results equal those of an engine built
  * with the new view. Bin capacities keep their tuning (a tile that now
- * overflows takes the ordered full-scan path). Before finalize the frame's
+ * overflows is rasterized from a scan of all facets). Before finalize the frame's
  * descriptor is updated. Workloads a server already took from this engine
  * keep their views. */
 int shape_engine_set_frame_view(shape_engine *e, int global_frame, const double ae[9], const double oe[9],

@@ -1,6 +1,7 @@
 // FP64 core kernels of the SHAPE B200 engine: model realization, view
-// transforms, facet binning, chi-square reductions, lightcurve photometry
-// and the evaluation summary.
+// transforms, facet binning, chi-square reductions, lightcurve splines, sky
+// frames and the evaluation summary. (Shading, shadows and photometry of a
+// pixel belong to the raster, raster_impl.cuh.)
 //
 // This translation unit is compiled with -fmad=false: the realization, the
 // view transforms and the facet bounding boxes must reproduce the reference
@@ -194,7 +195,7 @@ __global__ void k_xform(const FrameGeom *__restrict__ geoms, const double4 *__re
 
 // Facet culling, bounding box, outbnd flag and POSrect bookkeeping of
 // posvis (src/shape/posvis.c:142-199, 322-364), then one bin entry per
-// overlapped 16x16 tile. Bin order is arbitrary; the raster kernel sorts.
+// overlapped 16x16 tile. Bin order is arbitrary; the raster needs none.
 __device__ inline bool faces_viewer(const FrameGeom &g, const double4 &nb)
 {
     double nz = 0.0;
@@ -318,7 +319,6 @@ __device__ inline FrameState blank_state()
     s.idellim[1] = s.idoplim[1] = INT_MIN;
     s.dellim[0] = s.doplim[0] = dkey(HUGENUMBER);
     s.dellim[1] = s.doplim[1] = dkey(-HUGENUMBER);
-    s.any_lit = 0;
     s.any_overflow = 0;
     return s;
 }
@@ -871,8 +871,8 @@ __global__ void __launch_bounds__(256) k_poset_frames(PosetArgs a)
 // coefficient w = h[i-1]/span, diagonal 2, upper 1 - w): forward elimination
 // keeps each row's multiplier of y2[i+1] in y2[i] and its eliminated right-hand
 // side, back substitution forms y2[i] = mult[i] y2[i+1] + r[i]. The reference
-// solves the span-scaled rows in this order, so the FP64 fits are bit-identical
-// to its. Multipliers and pivots depend on the epochs only and come from the
+// solves the span-scaled rows in this order, so equal brightnesses give its fits
+// to the bit (they are sums over tiles here, in another order than its). Multipliers and pivots depend on the epochs only and come from the
 // host (spline_plan); what remains serial is r[i] = (rhs[i] - w r[i-1]) / piv
 // and the back substitution. The quotient is Markstein's: q = RN(a RN(1/b)),
 // then q + RN(1/b) (a - q b) with the residual exact in a fused multiply-add,
@@ -901,8 +901,8 @@ __device__ double splint_dev(const double *x, const double *y, const double *y2,
 // (src/shape/calc_fits.c:1651-1679, 1947).
 //
 // The recurrences (spline elimination and back substitution, the chi-square
-// sums, the log-factor sum) stay serial in the reference's order, so results
-// are bit-identical to it; everything else, their operands included, is formed
+// sums, the log-factor sum) stay serial in the reference's order, so equal
+// brightnesses give its results to the bit; everything else, their operands included, is formed
 // by the whole block first (in shared memory when a.smem_per_set > 0, else in
 // the set's scratch). What bounds it is their latency: with each step's slopes,
 // pivot and division inside the recurrence, the finalize and summary stage of

@@ -1008,7 +1008,7 @@ double EngineImpl::penalty_sum(const double *ms)
 
 // Bin autotuning from a dry-run binning of the model as loaded: the bin
 // capacity becomes the next power of two above 1.25x the fullest tile (so a
-// fit's small model changes do not overflow into the full-scan path), and
+// fit's small model changes do not leave facets to be scanned for), and
 // the batched raster visits tiles in decreasing facet count, so the heavy
 // tiles start first instead of forming a tail.
 int EngineImpl::tune_bins()
@@ -1068,10 +1068,6 @@ int EngineImpl::tune_bins()
     return SHAPE_OK;
 }
 
-// Enqueue one evaluation (without the H2D of parameters / D2H of the summary).
-// marks (optional, batched forms only): events recorded after each stage
-// 0 realize, 1 reset, 2 transform, 3 bin, 4 raster, 5 chi2, 6 lightcurve
-// photometry, 7 finalize + summary.
 // Facets x views up to which a batched evaluation bins in its first launch
 // (k_front), which then realizes each facet once per view instead of reading
 // the realized normal and corners, but saves a launch and the wait for it. On
@@ -1081,6 +1077,11 @@ int EngineImpl::tune_bins()
 constexpr long long FRONT_BINS = 131072;
 bool EngineImpl::front_bins() const { return (long long)nviews * nf <= FRONT_BINS; }
 
+// Enqueue one evaluation (the plain form's and stage timing's parameters are
+// uploaded before). marks (optional, batched forms only): events recorded after
+// each stage, 0 realize, 1 reset, 2 transform, 3 bin, 4 raster, 5 and 6 nothing,
+// 7 sky frames, lightcurves, chi-square and totals; the stages before the raster
+// are then launches of their own, which an evaluation does not have.
 int EngineImpl::enqueue(int form, cudaEvent_t *marks)
 {
     cudaStream_t s = stream;

@@ -21,8 +21,6 @@ namespace shape {
 
 constexpr int TILE_W = 16;          // POS tile: 16 x 16 pixels, one CTA
 constexpr int TILE_PIX = TILE_W * TILE_W;
-constexpr int RASTER_THREADS = TILE_PIX;
-constexpr int STAGE_FACETS = 128;   // facets staged in shared memory per pass
 constexpr int CHI2_THREADS = 256;
 constexpr int FIT32_PAD = 16;       // FP32 fit arena padding (vector reductions, k_raster)
 constexpr int DOP_MAXOVERFLOW = 2000;   // Doppler overflow spectrum bins (MAXOVERFLOW, src/shape/const.h:181)
@@ -91,7 +89,6 @@ struct FrameState {
     unsigned long long ofr_ov[4];    // ordered keys: imin, imax, jmin, jmax (doubles)
     int idellim[2], idoplim[2];
     unsigned long long dellim[2], doplim[2];  // ordered keys of min / max
-    int any_lit;
     int any_overflow;                // Doppler frame: a footprint left the spectrum
 };
 

@@ -1,5 +1,6 @@
 // posmask's per-pixel arithmetic (src/shape/posmask.c:58-174), shared by
-// the lightcurve kernel (core.cu) and the one-view posmask (posview.cu).
+// the observer views' raster (raster_impl.cuh) and the one-view posmask
+// (posview.cu).
 #pragma once
 
 #include "shape_types.h"

@@ -228,8 +228,8 @@ static int posvis_impl(int device, const shape_pos_view *view, shape_pos_images 
     const FrameGeom *dgeom = static_cast<const FrameGeom *>(c->geom.p);
     FrameState *dst = static_cast<FrameState *>(c->state.p);
     int *dcount = static_cast<int *>(c->bin_count.p);
-    // bins sized from the previous call's fullest tile; a tile that still
-    // overflows takes the raster's ordered full-scan path (same results)
+    // bins sized from the previous call's fullest tile; for a tile that still
+    // overflows the raster scans all facets (same results)
     long long entries = 0, busy = 0;
     for (int pass = 0; pass < 2; pass++) {
         if (int r2 = grow(c->bin_ids, sizeof(int2) * (size_t)ntiles * c->cap)) return r2;
@@ -353,7 +353,6 @@ __global__ void k_pos2deldop(P2dArgs a)
     atomicMax(&S.dellim[1], dkey(pp.del));
     atomicMin(&S.doplim[0], dkey(pp.dop));
     atomicMax(&S.doplim[1], dkey(pp.dop));
-    S.any_lit = 1;
     if (d.ok) pixel_dd_scatter<double, double>(a.ra, g, cose, d, a.fit);
 }
 

@@ -1,5 +1,6 @@
-// FP32 instantiation of the tile rasterizer (batched FP32 form: FMA
-// contraction allowed; vertex transforms arrive already rounded from FP64).
+// FP32 instantiation of the tile rasterizer (radar views of the batched FP32
+// form: FP64 vertices, coverage and depths, FP32 shading and synthesis; FMA
+// contraction allowed).
 #include "raster_impl.cuh"
 
 namespace shape {
