@@ -25,7 +25,9 @@
 // What bounds it: instruction issue and latency, not memory (the tile's data
 // come from L2). A facet of a 20000-pixel body spans about 4 pixels: the exact
 // test runs once per (facet, covered pixel) instead of once per pixel of every
-// facet that meets a warp's block, and nothing is sorted.
+// facet that meets a warp's block, and nothing is sorted. Facets of hundreds of
+// pixels are tested by all pixels instead (FEW); bodies of many layers go through
+// the phases in chunks of facets (tile_chunks).
 #pragma once
 
 #include <algorithm>
@@ -628,7 +630,8 @@ __device__ inline unsigned long long warp_kmax(unsigned long long k)
 }
 // Candidate facets a pixel holds, and those a tile holds beyond them. A convex
 // body has one layer of facets (a few pixels on shared edges two), a 3 % rough
-// 32768-facet body up to 14 at its limb; a tile with more takes the slow path.
+// 32768-facet body up to 14 at its limb; a tile with more is rastered in chunks
+// (tile_chunks).
 constexpr int CAND = 8;
 constexpr int CAND_MORE = 512;
 
