@@ -866,18 +866,18 @@ __device__ __noinline__ PixelHit pixel_history(const RasterArgs &a, const FrameG
 // 10u mag (|X| + |Y|), their difference and the addition of m by 2u more, cx and
 // cy by 6u, and the sum at a pixel of the box adds 2u of its terms and 7u 30 mag
 // from cx and cy: in all 14u mag (|X| + |Y|) + 240u mag, 8.4e-7 and 1.5e-5 beside
-// m's 2e-6 and 6.4e-5. Coefficients out of FP32's range bound nothing (the whole
-// box).
+// m's 2e-6 and 6.4e-5. Coefficients out of FP32's range, and a den below its normal
+// numbers (facets of 1e19 length units), bound nothing (the whole box).
 __device__ inline FacetEdges facet_edges(const FacetTerms &q, double x0, double y0, float ikm, double kmpp)
 {
-    const float d = (float)q.den * (float)kmpp;
+    const float den = (float)q.den, d = den * (float)kmpp;
     const float sx = (float)q.A * d, sy = -(float)q.B * d, tx = -(float)q.D * d, ty = (float)q.C * d;
     const float X = (float)(x0 - q.x) * ikm, Y = (float)(y0 - q.y) * ikm;
     const float mag = fabsf(sx) + fabsf(sy) + fabsf(tx) + fabsf(ty);
     const float m = 2e-6f * (1.0f + mag * (fabsf(X) + fabsf(Y) + 32.0f));
     const float s0 = sx * X + sy * Y, t0 = tx * X + ty * Y;
     FacetEdges e = {{t0 + m, s0 - t0 + m, 1.0f - s0 + m}, {tx, sx - tx, -sx}, {ty, sy - ty, -sy}, 0u};
-    if (!(m < 1e24f))
+    if (!(m < 1e24f) || fabsf(den) < 1.2e-38f)
         for (int k = 0; k < 3; k++) { e.c0[k] = 1.0f; e.cx[k] = e.cy[k] = 0.0f; }
     return e;
 }
